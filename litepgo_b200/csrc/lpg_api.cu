@@ -113,6 +113,7 @@ void upload_plan(lpg_fem& hh, int V, int T) {
         m.tc_loc = upload(h->b_tc[10], p.tc_loc);
         m.tc_items = reinterpret_cast<uint4*>(upload(h->b_tc[11], p.tc_items));
         m.tc_ents = upload(h->b_tc[12], p.tc_ents);
+        m.tc_dent = upload(h->b_tc[13], p.tc_dent);
         m.tc_max_els = m.tc_max_verts = m.tc_max_vals = 0;
         for (int c = 0; c < m.tc_ncl; ++c) {
             m.tc_max_els = std::max(m.tc_max_els, p.tc_el_ptr[c + 1] - p.tc_el_ptr[c]);
@@ -209,16 +210,25 @@ struct BusyGuard {
 lpg_fem::~lpg_fem() {
     if (pcg_graph) cudaGraphExecDestroy(pcg_graph);
     if (batch_graph) cudaGraphExecDestroy(batch_graph);
+    if (host_result) cudaFreeHost(host_result);
     if (own_stream) cudaStreamDestroy(own_stream);
+}
+
+void lpg_fem::create_result() {
+    LPG_CUDA(cudaMemset(d_result.as<EvalResult>(1), 0, sizeof(EvalResult)));
+    LPG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host_result), sizeof(EvalResult), cudaHostAllocDefault));
 }
 
 void lpg_fem::sync() { LPG_CUDA(cudaStreamSynchronize(stream)); }
 
 unsigned lpg_fem::take_status() {
-    unsigned st = 0;
-    LPG_CUDA(cudaMemcpyAsync(&st, d_status.ptr, sizeof st, cudaMemcpyDeviceToHost, stream));
-    LPG_CUDA(cudaMemsetAsync(d_status.ptr, 0, sizeof(unsigned), stream));
+    LPG_CUDA(cudaMemcpyAsync(host_result, d_result.ptr, sizeof(EvalResult), cudaMemcpyDeviceToHost, stream));
     sync();
+    const unsigned st = host_result->status;
+    if (st != 0) { // only a failed call has bits to clear
+        LPG_CUDA(cudaMemsetAsync(status_word(), 0, sizeof(unsigned), stream));
+        sync();
+    }
     return st;
 }
 
@@ -246,14 +256,18 @@ void lpg_fem::eval_async(const double* du, double* dgrad, int hessian, int preci
     a.hess = hessian != LPG_HESSIAN_NONE ? dhess : nullptr;
     a.layout = layout;
     // Per-cluster energies, then partial sums.
-    a.cluster_energy = d_cluster_energy.as<double>(static_cast<size_t>(std::max(dm.ncl, dm.tc_ncl)) + 256);
-    a.energy = d_energy.as<double>(1);
+    a.cluster_energy = d_cluster_energy.as<double>(
+        static_cast<size_t>(std::max({dm.ncl, dm.tc_ncl, tet_energy_blocks(dm)})) + 256);
+    a.energy = energy_word();
+    a.done = done_word();
     a.elem_energy = delem;
-    a.status = d_status.as<unsigned>(1);
+    a.status = status_word();
     a.ev_begin = ev_begin;
     a.ev_end = ev_end;
     const int pi = precision == LPG_PRECISION_F64 ? 0 : 1;
     a.cl_variant = tune.cl[pi];
+    a.emesh = emesh;
+    a.mstate = mesh_exact;
     a.tc_skip = tc_skip;
     a.cl_skip = cl_skip;
     if (dm.K == 64) {
@@ -422,7 +436,7 @@ int lpg_fem_create(int V, const double* X, int T, const int32_t* tets, const dou
             m.fpinv64 = upload(h->b_fpinv64, fpinv);
             m.fpinv32 = upload(h->b_fpinv32, f32);
         }
-        LPG_CUDA(cudaMemset(h->d_status.as<unsigned>(1), 0, sizeof(unsigned)));
+        h->create_result();
         LPG_CUDA(cudaDeviceSynchronize());
         // Launch variants tuned on this mesh unless LPG_AUTOTUNE=0 (then the defaults stay).
         const char* at = std::getenv("LPG_AUTOTUNE");
@@ -519,7 +533,7 @@ int lpg_fem_create_hex_hermite(int V, const double* X, int T, const int32_t* cel
         m.hex_theta = upload(h->b_hex[2], th);
         m.herm_q = upload(h->b_hex[3], qt);
         m.herm_h = upload(h->b_herm, hb);
-        LPG_CUDA(cudaMemset(h->d_status.as<unsigned>(1), 0, sizeof(unsigned)));
+        h->create_result();
         LPG_CUDA(cudaDeviceSynchronize());
         *out = h.release();
     });
@@ -588,7 +602,7 @@ int lpg_fem_create_hex(int V, const double* X, int T, const int32_t* cells, cons
         m.hex_cells = upload(h->b_hex[1], std::vector<int32_t>(cells, cells + 8 * static_cast<size_t>(T)));
         m.hex_theta = upload(h->b_hex[2], th);
         m.hex_q = upload(h->b_hex[3], qt);
-        LPG_CUDA(cudaMemset(h->d_status.as<unsigned>(1), 0, sizeof(unsigned)));
+        h->create_result();
         LPG_CUDA(cudaDeviceSynchronize());
         *out = h.release();
     });
@@ -680,13 +694,12 @@ int lpg_fem_eval(lpg_fem_t h, const double* u, int io_mem, double* energy, doubl
             dhess = hess_mem == LPG_MEM_DEVICE ? hess : h->d_hess.ensure(hbytes);
         }
         h->eval_async(du, dgrad, hessian, precision, layout, dhess, nullptr);
-        double e = 0;
-        LPG_CUDA(cudaMemcpyAsync(&e, h->d_energy.ptr, sizeof e, cudaMemcpyDeviceToHost, h->stream));
         if (grad && io_mem == LPG_MEM_HOST)
             LPG_CUDA(cudaMemcpyAsync(grad, dgrad, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         if (dhess && hess_mem == LPG_MEM_HOST)
             LPG_CUDA(cudaMemcpyAsync(hess, dhess, hbytes, cudaMemcpyDeviceToHost, h->stream));
         raise_status(h->take_status());
+        const double e = h->host_result->energy;
         if (!std::isfinite(e)) fail(LPG_EDOMAIN, "MeshEnergy: non-finite energy sum");
         if (energy) *energy = e;
     });
@@ -705,9 +718,9 @@ int lpg_fem_deformation_gradients(lpg_fem_t h, const double* u, int io_mem, doub
         const double* du = h->stage_in(u, io_mem, h->d_u, n);
         double* dF = io_mem == LPG_MEM_DEVICE ? F : h->d_vjp.as<double>(std::max<size_t>(9 * rows, 1));
         if (hex)
-            launch_hex_deformation_gradients(h->dm, du, dF, h->d_status.as<unsigned>(1), h->stream);
+            launch_hex_deformation_gradients(h->dm, du, dF, h->status_word(), h->stream);
         else
-            launch_deformation_gradients(h->dm, du, dF, h->d_status.as<unsigned>(1), h->stream);
+            launch_deformation_gradients(h->dm, du, dF, h->status_word(), h->stream);
         if (io_mem == LPG_MEM_HOST && rows > 0)
             LPG_CUDA(cudaMemcpyAsync(F, dF, 9 * rows * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         raise_status(h->take_status());
@@ -751,8 +764,9 @@ int lpg_fem_eval_material(lpg_fem_t h, const double* W, const double* P, const d
         a.hess = hessian != LPG_HESSIAN_NONE ? (out_mem == LPG_MEM_DEVICE ? hess : h->d_hess.ensure(hbytes)) : nullptr;
         a.layout = layout;
         a.cluster_energy = h->d_cluster_energy.as<double>(static_cast<size_t>(std::max(h->dm.ncl, h->dm.tc_ncl)) + 256);
-        a.energy = h->d_energy.as<double>(1);
-        a.status = h->d_status.as<unsigned>(1);
+        a.energy = h->energy_word();
+        a.done = h->done_word();
+        a.status = h->status_word();
         const int pi = precision == LPG_PRECISION_F64 ? 0 : 1;
         const size_t nel = std::max<size_t>(static_cast<size_t>(h->dm.T), 1);
         if (hex) {
@@ -767,12 +781,11 @@ int lpg_fem_eval_material(lpg_fem_t h, const double* W, const double* P, const d
                                  h->d_vjp.as<double>(12 * nel), proj, h->d_plist.as<int>(nel),
                                  h->d_pcount.as<unsigned>(1), h->tune.clamp[pi], a, s);
         }
-        double e = 0;
-        LPG_CUDA(cudaMemcpyAsync(&e, a.energy, sizeof e, cudaMemcpyDeviceToHost, s));
         if (grad && out_mem == LPG_MEM_HOST && n > 0)
             LPG_CUDA(cudaMemcpyAsync(grad, a.grad, n * sizeof(double), cudaMemcpyDeviceToHost, s));
         if (a.hess && out_mem == LPG_MEM_HOST) LPG_CUDA(cudaMemcpyAsync(hess, a.hess, hbytes, cudaMemcpyDeviceToHost, s));
         raise_status(h->take_status());
+        const double e = h->host_result->energy;
         if (!std::isfinite(e)) fail(LPG_EDOMAIN, "MeshEnergy: non-finite energy sum");
         if (energy) *energy = e;
     });
@@ -837,7 +850,7 @@ int lpg_fem_feasible_step(lpg_fem_t h, const double* u, const double* du, int io
         const int nb = feasible_blocks(h->dm);
         double* bm = h->d_block.as<double>(std::max(nb, 1));
         double* al = h->d_alpha.as<double>(1);
-        launch_feasible(h->dm, d_u, d_du, bm, nb, al, h->d_status.as<unsigned>(1), h->stream);
+        launch_feasible(h->dm, d_u, d_du, bm, nb, al, h->status_word(), h->stream);
         double v = 1;
         LPG_CUDA(cudaMemcpyAsync(&v, al, sizeof v, cudaMemcpyDeviceToHost, h->stream));
         const unsigned st = h->take_status();
@@ -859,7 +872,7 @@ int lpg_fem_force_vjp_theta(lpg_fem_t h, const double* u, const double* w, int i
         const double* d_w = h->stage_in(w, io_mem, h->d_u2, n);
         const size_t T = static_cast<size_t>(h->dm.T);
         double* pe = (per_element && io_mem == LPG_MEM_DEVICE) ? out : h->d_vjp.as<double>(std::max<size_t>(2 * T, 2));
-        launch_force_vjp(h->dm, d_u, d_w, pe, h->d_status.as<unsigned>(1), h->stream);
+        launch_force_vjp(h->dm, d_u, d_w, pe, h->status_word(), h->stream);
         if (per_element) {
             if (io_mem == LPG_MEM_HOST && T > 0)
                 LPG_CUDA(cudaMemcpyAsync(out, pe, 2 * T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -980,7 +993,7 @@ int lpg_fem_force_vjp_fp(lpg_fem_t h, const double* u, const double* w, int io_m
         const double* d_w = h->stage_in(w, io_mem, h->d_u2, n);
         const size_t T = static_cast<size_t>(h->dm.T);
         double* pe = (per_element && io_mem == LPG_MEM_DEVICE) ? out : h->d_vjp.as<double>(std::max<size_t>(9 * T, 9));
-        launch_fp_vjp(h->dm, d_u, d_w, pe, h->d_status.as<unsigned>(1), h->stream);
+        launch_fp_vjp(h->dm, d_u, d_w, pe, h->status_word(), h->stream);
         if (per_element) {
             if (io_mem == LPG_MEM_HOST && T > 0)
                 LPG_CUDA(cudaMemcpyAsync(out, pe, 9 * T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -1127,7 +1140,7 @@ int lpg_fem_force_vjp_rest(lpg_fem_t h, const double* u, const double* w, int io
         const double* d_w = h->stage_in(w, io_mem, h->d_u2, n);
         double* d_out = io_mem == LPG_MEM_DEVICE ? out : h->d_grad.as<double>(std::max<size_t>(n, 1));
         double* pe = h->d_vjp.as<double>(std::max<size_t>(12 * static_cast<size_t>(h->dm.T), 1));
-        launch_rest_vjp(h->dm, d_u, d_w, pe, 1.0, d_out, h->d_status.as<unsigned>(1), h->stream);
+        launch_rest_vjp(h->dm, d_u, d_w, pe, 1.0, d_out, h->status_word(), h->stream);
         if (io_mem == LPG_MEM_HOST && n > 0)
             LPG_CUDA(cudaMemcpyAsync(out, d_out, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         raise_status(h->take_status());

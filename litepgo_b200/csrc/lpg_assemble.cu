@@ -245,10 +245,55 @@ __global__ void zero_rows_kernel(double* __restrict__ grad, const int* __restric
     }
 }
 
-// Deterministic sum of n doubles: kSumBlocks blocks sum fixed contiguous chunks (fixed thread ->
-// index map and tree), then one block sums the partials in order.
-constexpr int kSumBlocks = 256;
-__global__ void __launch_bounds__(256) sum_partial_kernel(const double* __restrict__ x, int n, double* part) {
+// The energy of a launch of 256-thread blocks from its n per-unit energies: the block that finishes
+// last sums them in a fixed order (thread t: units t, t + 256, ... in 16 chains; a fixed tree). Called
+// by every thread at the kernel's end, after thread 0 wrote the block's units. This takes the place of
+// a two-launch sum: an evaluation of 64^3 cubes sums 13,473 units in about 3 us here, against 4.1 us of
+// kernels and two more launches (a small evaluation is all launches: 180 tets took 57 us, 17.5 us of
+// them on the GPU).
+__device__ __forceinline__ void finish_energy(const double* x, int n, double* energy, unsigned* done) {
+    __shared__ double s_fin[8];
+    __shared__ bool s_last;
+    if (threadIdx.x == 0) {
+        __threadfence(); // this thread wrote the block's units
+        s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    constexpr int C = 16; // chains: loads in flight per thread
+    double v[C];
+#pragma unroll
+    for (int k = 0; k < C; ++k) v[k] = 0;
+    for (int i = threadIdx.x; i < n; i += 256 * C) {
+        double ld[C];
+#pragma unroll
+        for (int k = 0; k < C; ++k) ld[k] = i + 256 * k < n ? __ldcg(x + i + 256 * k) : 0.0;
+#pragma unroll
+        for (int k = 0; k < C; ++k) v[k] += ld[k];
+    }
+#pragma unroll
+    for (int w = C / 2; w > 0; w >>= 1)
+#pragma unroll
+        for (int k = 0; k < w; ++k) v[k] += v[k + w];
+    double t = v[0];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    if ((threadIdx.x & 31) == 0) s_fin[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double e = 0;
+        for (int w = 0; w < 8; ++w) e += s_fin[w];
+        *energy = e;
+        *done = 0;
+    }
+}
+
+// Deterministic sum of n doubles: fixed contiguous chunks per block (fixed thread -> index map and
+// tree), then finish_energy over the partials.
+constexpr int kSumBlocks = 64;
+__global__ void __launch_bounds__(256) sum_kernel(const double* __restrict__ x, int n, double* part, double* out,
+                                                  unsigned* done) {
     __shared__ double s[8];
     const int chunk = (n + gridDim.x - 1) / gridDim.x;
     const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
@@ -263,19 +308,12 @@ __global__ void __launch_bounds__(256) sum_partial_kernel(const double* __restri
         for (int w = 0; w < (blockDim.x >> 5); ++w) t += s[w];
         part[blockIdx.x] = t;
     }
+    finish_energy(part, gridDim.x, out, done);
 }
-__global__ void __launch_bounds__(256) sum_final_kernel(const double* __restrict__ part, int nb, double* out) {
-    __shared__ double s[8];
-    double v = threadIdx.x < nb ? part[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0;
-        for (int w = 0; w < (blockDim.x >> 5); ++w) t += s[w];
-        *out = t;
-    }
+// The sum of the n per-element energies into a.energy (a.cluster_energy is scratch).
+void launch_sum(const double* x, int n, const EvalArgs& a, cudaStream_t s) {
+    sum_kernel<<<std::max(1, std::min(kSumBlocks, (n + 255) / 256)), 256, 0, s>>>(x, n, a.cluster_energy, a.energy,
+                                                                                a.done);
 }
 
 // ---------------------------------------------------------------------------
@@ -1241,7 +1279,8 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 struct TcBounds {
     int e0 = 0, ne = 0, v0 = 0, nv = 0, i0 = 0, ni = 0, nd = 0, n0 = 0, nn = 0, r0 = 0, nr = 0;
 };
-constexpr int kTcFields = 12; // the bounds, then the cluster's skip flag (batched solves)
+// The bounds, the cluster's skip flag (batched solves), its diagonal items' contributors.
+constexpr int kTcFields = 13;
 // Field q of cluster cl as the words it is made of: {first, end} of a count field (the count is
 // end - first), {value, 0} otherwise. The lanes reading the fields of one cluster take no
 // divergent path (the array is selected, the second word's load predicated), and nothing here
@@ -1255,8 +1294,9 @@ __device__ __forceinline__ int2 tc_field_words(const DevMesh& m, const unsigned 
                        : q < 6 ? m.tc_item_ptr
                        : q == 6 ? m.tc_ndiag
                        : q < 9 ? m.tc_ent_ptr
+                       : q == 12 ? m.tc_dent
                        : m.tc_row_ptr;
-    if (q < 11) w.x = __ldg(ptr + cl);
+    if (q != 11) w.x = __ldg(ptr + cl);
     if (tc_count_field(q)) w.y = __ldg(ptr + cl + 1);
     if (q == 11 && skip != nullptr) w.x = __ldg(skip + cl) != 0;
     return w;
@@ -1265,12 +1305,14 @@ __device__ __forceinline__ int tc_field_value(int2 w, int q) { return tc_count_f
 __device__ __forceinline__ int tc_field(const DevMesh& m, const unsigned char* skip, int cl, int q) {
     return tc_field_value(tc_field_words(m, skip, cl, q), q);
 }
-// A skipped cluster has empty bounds: nothing is staged, evaluated or written.
-__device__ __forceinline__ TcBounds tc_bounds(const int* f) {
+// A skipped cluster has empty bounds: nothing is staged, evaluated or written. DIAG: the items and
+// contributors of the diagonal blocks only (the gradient's).
+template <bool DIAG = false> __device__ __forceinline__ TcBounds tc_bounds(const int* f) {
     TcBounds b;
     if (f[11]) return b;
     b.e0 = f[0], b.ne = f[1], b.v0 = f[2], b.nv = f[3], b.i0 = f[4], b.ni = f[5];
     b.nd = f[6], b.n0 = f[7], b.nn = f[8], b.r0 = f[9], b.nr = f[10];
+    if (DIAG) b.ni = b.nd, b.nn = f[12];
     return b;
 }
 
@@ -1294,22 +1336,19 @@ __device__ __forceinline__ void tc_load_idx(const DevMesh& m, const TcBounds& b,
 // Issues thread t's part of a cluster's stage: its element's record into registers, its
 // vertex's displacement and its share of the item table and contributor lists into shared memory
 // (cp.async, one group), and its owned row's words into registers.
-template <typename R, bool ITEMS>
+template <typename R>
 __device__ __forceinline__ void tc_issue(const DevMesh& m, const double* __restrict__ u, const TcBounds& b,
                                          const TcIdx& x, int t, bool sell, double* su, uint4* sitems, uint16_t* sents,
                                          R (&r12)[12], int (&rowv)[kTcRowRaw]) {
-    // Without items (energy only) an element the cluster does not own contributes nothing.
-    if (t < b.ne && (ITEMS || (x.ew >> 31))) load_rec<R>(rec_ptr<R>(m), static_cast<int>(x.ew & 0x7fffffffu), r12);
+    if (t < b.ne) load_rec<R>(rec_ptr<R>(m), static_cast<int>(x.ew & 0x7fffffffu), r12);
     if (t < b.nv) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) cp_async8(su + 3 * t + i, u + 3 * static_cast<size_t>(x.vert) + i);
     }
-    if (ITEMS) {
-        for (int k = t; k < b.ni; k += kTcThreads) cp_async16(sitems + k, m.tc_items + b.i0 + k);
-        for (int k = t; k < (b.nn >> 3); k += kTcThreads) cp_async16(sents + 8 * k, m.tc_ents + b.n0 + 8 * k);
-    }
+    for (int k = t; k < b.ni; k += kTcThreads) cp_async16(sitems + k, m.tc_items + b.i0 + k);
+    for (int k = t; k < (b.nn >> 3); k += kTcThreads) cp_async16(sents + 8 * k, m.tc_ents + b.n0 + 8 * k);
     cp_async_commit();
-    if (ITEMS && t < b.nr) {
+    if (t < b.nr) {
         rowv[0] = x.row;
         rowv[1] = x.so;
         rowv[2] = __ldg(m.row_ptr + x.row);
@@ -1323,12 +1362,11 @@ __device__ __forceinline__ void tc_issue(const DevMesh& m, const double* __restr
     }
 }
 
-template <typename R, bool WG, bool WH, int MINB, int UNR>
+template <typename R, bool WG, int MINB, int UNR>
 __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const DevMesh m, const EvalArgs a) {
     using X = M<R>;
     using HT = typename HOut<R>::T;
     constexpr int E = kTcElems;
-    constexpr bool ITEMS = WG || WH;
     constexpr int nw = kTcThreads / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* red = reinterpret_cast<double*>(smem_raw);
@@ -1358,12 +1396,12 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
     tc_load_idx(m, b, tid, x);
     R r12[12];
     int rowv[kTcRowRaw] = {0, 0, 0, 0, 0, 0};
-    tc_issue<R, ITEMS>(m, a.u, b, x, tid, sell, su, sitems, sents, r12, rowv);
+    tc_issue<R>(m, a.u, b, x, tid, sell, su, sitems, sents, r12, rowv);
     int2 ahead = tid < kTcFields ? tc_field_words(m, a.tc_skip, cl + grid, tid) : make_int2(0, 0);
-    int ne = b.ne, ni = WH ? b.ni : b.nd, nr = b.nr, ndc = b.nd;
+    int ne = b.ne, ni = b.ni, nr = b.nr, ndc = b.nd;
     for (int buf = 0; cl < m.tc_ncl; cl += grid, buf ^= 1) {
         int* rows = srow + buf * kTcRows * kTcRowInts;
-        if (ITEMS && tid < nr) {
+        if (tid < nr) {
 #pragma unroll
             for (int q = 0; q < 3; ++q) rows[kTcRowInts * tid + q] = rowv[q];
             rows[kTcRowInts * tid + 3] = (rowv[3] - rowv[2]) | (sell ? (rowv[5] - rowv[2]) << 8 : 0);
@@ -1376,7 +1414,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
         const uint32_t ew = x.ew;
         R Ds[3][3];
         bool in_ok = true;
-        if (tid < ne && (ITEMS || (ew >> 31))) {
+        if (tid < ne) {
             double uu[4][3];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -1388,7 +1426,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
         }
         __syncthreads(); // the displacements are read; their memory holds element data from here
         double eacc = 0;
-        if (tid < ne && (ITEMS || (ew >> 31))) {
+        if (tid < ne) {
             const int el = tid;
             const int e = static_cast<int>(ew & 0x7fffffffu);
             Kin<R> k;
@@ -1399,7 +1437,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
                 if (a.elem_energy) a.elem_energy[e] = static_cast<double>(Ee);
             }
             const R p = X::fma(k.lam, k.logJ, -k.mu);
-            tc_element_data<R, WG, WH>(k, p, ed, el);
+            tc_element_data<R, WG, true>(k, p, ed, el);
         }
         // Energy of the cluster's own elements: fixed thread order, fixed tree.
 #pragma unroll
@@ -1416,7 +1454,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
         // runs.
         tc_load_idx(m, tc_bounds(s_hdr[buf]), tid, x);
         if (tid < kTcFields) ahead = tc_field_words(m, a.tc_skip, cl + 2 * grid, tid);
-        if (ITEMS) {
+        {
             // Item pass. The nd diagonal items (the first nd) are summed by groups of S lanes
             // (tc_diag_split), each lane over a contiguous part of the contributor list in
             // ascending order, the parts added by shuffles; they fill whole warps (S nd lanes
@@ -1444,7 +1482,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
 #pragma unroll
                             for (int i = 0; i < 3; ++i) gs[i] = X::add(gs[i], ed[(kTcG + 3 * la + i) * E + el]);
                         }
-                        if (WH) {
+                        {
                             const R hh[3] = {ed[(kTcH + 3 * la) * E + el], ed[(kTcH + 3 * la + 1) * E + el],
                                              ed[(kTcH + 3 * la + 2) * E + el]};
                             const R dv = X::add(ed[kTcL * E + el], -ed[kTcP * E + el]), mg = ed[(kTcCC + pr) * E + el];
@@ -1458,7 +1496,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
 #pragma unroll
                         for (int i = 0; i < 3; ++i) gs[i] = X::add(gs[i], __shfl_xor_sync(0xffffffffu, gs[i], off));
                     }
-                    if (WH) {
+                    {
 #pragma unroll
                         for (int u6 = 0; u6 < 6; ++u6)
                             acc[u6] = X::add(acc[u6], __shfl_xor_sync(0xffffffffu, acc[u6], off));
@@ -1473,7 +1511,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
                             a.grad[3 * static_cast<size_t>(v) + i] = static_cast<double>(gs[i]);
                         }
                     }
-                    if (WH) {
+                    {
                         constexpr int sym3[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
 #pragma unroll
                         for (int i = 0; i < 3; ++i)
@@ -1481,7 +1519,7 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
                             for (int c = 0; c < 3; ++c) stage[tc_stage(it.x, csc, i, c)] = acc[sym3[3 * i + c]];
                     }
                 }
-            } else if (WH) {
+            } else {
                 for (int kk = nd + tid - dpad; kk < ni; kk += kTcThreads - dpad) {
                     const uint4 it = sitems[kk];
                     // The solver layout keeps only blocks right of the diagonal: an edge to a
@@ -1530,13 +1568,13 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
         const int nrc = nr;
         {
             const TcBounds bn = tc_bounds(s_hdr[buf]);
-            tc_issue<R, ITEMS>(m, a.u, bn, x, tid, sell, su, sitems, sents, r12, rowv);
+            tc_issue<R>(m, a.u, bn, x, tid, sell, su, sitems, sents, r12, rowv);
             ne = bn.ne;
-            ni = WH ? bn.ni : bn.nd;
+            ni = bn.ni;
             nr = bn.nr;
             ndc = bn.nd;
         }
-        if (WH) {
+        {
             // Copy pass: one warp per owned row.
             for (int j = warp; j < nrc; j += nw) {
                 const int* rw = rows + kTcRowInts * j;
@@ -1565,16 +1603,189 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
     cp_async_wait_all();
     st = __reduce_or_sync(0xffffffffu, st);
     if (lane == 0 && st) atomicOr(a.status, st);
+    finish_energy(a.cluster_energy, m.tc_ncl, a.energy, a.done);
 }
 
-template <typename R, bool WG, bool WH, int MINB = tc_minb<R>(0), int UNR = tc_unroll(0)>
-void launch_tet_cluster(const DevMesh& m, const EvalArgs& a, cudaStream_t s) {
-    const size_t sm = tc_smem_bytes<R>();
-    thread_local LaunchCache cache;
-    const int resident = resident_grid(tet_cluster_kernel<R, WG, WH, MINB, UNR>, kTcThreads, sm, cache);
-    const int blocks = std::min(resident, m.tc_ncl);
+// Energy and gradient alone (a line search's or an explicit step's residual) over the same clusters: the
+// element pass keeps only g_a (12 values, 24 KB in FP64), so three FP64 blocks fit an SM instead of two,
+// and only the diagonal items' contributors are staged. The displacements have memory of their own and
+// the items, contributors and rows two buffers, so the next cluster's stage is issued before the item
+// pass and a cluster takes two block barriers instead of four. Item pass: one lane per row, component
+// and part of the row's contributors, the parts split and added as in tet_cluster_kernel (the gradient is
+// bitwise that of the Hessian pass).
+constexpr int kTgEnts = 4 * kTcElems; // at most four contributors of diagonal items per element
+template <typename R> constexpr int tg_minb() { return sizeof(R) == 8 ? 3 : 4; }
+template <typename R> constexpr size_t tg_smem_bytes() {
+    return (32 + 3 * kTcVerts) * sizeof(double) + 12 * static_cast<size_t>(kTcElems) * sizeof(R) +
+           2 * (kTcRows * sizeof(uint4) + kTgEnts * sizeof(uint16_t) + kTcRows * sizeof(int));
+}
+template <typename R>
+__global__ void __launch_bounds__(kTcThreads, tg_minb<R>()) tet_gradient_kernel(const DevMesh m, const EvalArgs a) {
+    using X = M<R>;
+    constexpr int E = kTcElems;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* red = reinterpret_cast<double*>(smem_raw);
+    double* su = red + 32; // [nv][3]
+    R* ed = reinterpret_cast<R*>(su + 3 * kTcVerts);
+    uint4* sitems = reinterpret_cast<uint4*>(ed + 12 * E);
+    uint16_t* sents = reinterpret_cast<uint16_t*>(sitems + 2 * kTcRows);
+    int* srow = reinterpret_cast<int*>(sents + 2 * kTgEnts);
+    __shared__ int s_hdr[2][kTcFields];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int grid = static_cast<int>(gridDim.x);
+    unsigned st = 0;
+    int cl = blockIdx.x;
+    TcBounds b;
+    {
+        int f[kTcFields];
+#pragma unroll
+        for (int q = 0; q < kTcFields; ++q) f[q] = tc_field(m, a.tc_skip, cl, q);
+        b = tc_bounds<true>(f);
+    }
+    TcIdx x;
+    tc_load_idx(m, b, tid, x);
+    R r12[12];
+    auto issue = [&](const TcBounds& c, int bufn) {
+        if (tid < c.ne) load_rec<R>(rec_ptr<R>(m), static_cast<int>(x.ew & 0x7fffffffu), r12);
+        if (tid < c.nv) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) cp_async8(su + 3 * tid + i, a.u + 3 * static_cast<size_t>(x.vert) + i);
+        }
+        if (tid < c.ni) cp_async16(sitems + bufn * kTcRows + tid, m.tc_items + c.i0 + tid);
+        for (int k = tid; k < (c.nn >> 3); k += kTcThreads)
+            cp_async16(sents + bufn * kTgEnts + 8 * k, m.tc_ents + c.n0 + 8 * k);
+        cp_async_commit();
+    };
+    issue(b, 0);
+    int2 ahead = tid < kTcFields ? tc_field_words(m, a.tc_skip, cl + grid, tid) : make_int2(0, 0);
+    for (int buf = 0; cl < m.tc_ncl; cl += grid, buf ^= 1) {
+        const int ne = b.ne, nd = b.nd;
+        const uint32_t ew = x.ew, loc = x.loc;
+        if (tid < b.nr) srow[buf * kTcRows + tid] = x.row;
+        if (tid < kTcFields) s_hdr[buf][tid] = tc_field_value(ahead, tid);
+        cp_async_wait_all();
+        __syncthreads(); // the cluster's stage is complete, and the previous item pass
+        b = tc_bounds<true>(s_hdr[buf]);
+        tc_load_idx(m, b, tid, x); // the next cluster's
+        if (tid < kTcFields) ahead = tc_field_words(m, a.tc_skip, cl + 2 * grid, tid);
+        double eacc = 0;
+        if (tid < ne) {
+            double uu[4][3];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int lv = static_cast<int>((loc >> (8 * c)) & 0xffu);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) uu[c][i] = su[3 * lv + i];
+            }
+            const int e = static_cast<int>(ew & 0x7fffffffu);
+            Kin<R> k;
+            st |= kinematics_of<R>(m, e, r12, uu, k);
+            if (ew >> 31) {
+                const R Ee = k.vol * k.psi;
+                eacc = static_cast<double>(Ee);
+                if (a.elem_energy) a.elem_energy[e] = eacc;
+            }
+            tc_element_data<R, true, false>(k, X::fma(k.lam, k.logJ, -k.mu), ed - kTcG * E, tid);
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) eacc += __shfl_xor_sync(0xffffffffu, eacc, off);
+        if (lane == 0) red[warp] = eacc;
+        __syncthreads(); // element data complete; the displacements are read
+        if (tid == 0) {
+            double t = 0;
+            for (int w = 0; w < kTcThreads / 32; ++w) t += red[w];
+            a.cluster_energy[cl] = t;
+            if (!isfinite(t)) st |= ST_NONFINITE_OUT;
+        }
+        issue(b, buf ^ 1); // in flight during the item pass
+        const int sd = tc_diag_split(nd), lsd = sd == 4 ? 2 : 1, total = 3 * nd * sd;
+        for (int base = 0; base < total; base += kTcThreads) {
+            const int l = base + tid, part = l & (sd - 1), ri = (l >> lsd) / 3, i = (l >> lsd) - 3 * ri;
+            const bool active = l < total;
+            R g = 0;
+            uint4 it = make_uint4(0u, 0u, 0u, 0u);
+            if (active) {
+                it = sitems[buf * kTcRows + ri];
+                const uint16_t* en = sents + buf * kTgEnts + (it.z & 0xfffffu);
+                const int cnt = static_cast<int>(it.z >> 20);
+                const int c0 = (cnt * part + sd - 1) >> lsd, c1 = (cnt * (part + 1) + sd - 1) >> lsd;
+                for (int c = c0; c < c1; ++c) {
+                    const int w = en[c];
+                    g = X::add(g, ed[(3 * ((w >> 2) & 3) + i) * E + (w >> 8)]);
+                }
+            }
+            for (int off = 1; off < sd; off <<= 1) g = X::add(g, __shfl_xor_sync(0xffffffffu, g, off));
+            if (active && part == 0) {
+                if (!X::finite(g)) st |= ST_NONFINITE_OUT;
+                a.grad[3 * static_cast<size_t>(srow[buf * kTcRows + (it.w & 0xffu)]) + i] = static_cast<double>(g);
+            }
+        }
+    }
+    cp_async_wait_all();
+    st = __reduce_or_sync(0xffffffffu, st);
+    if (lane == 0 && st) atomicOr(a.status, st);
+    finish_energy(a.cluster_energy, m.tc_ncl, a.energy, a.done);
+}
+
+// Energy alone (a line search's trial points): one thread per element, the block's sum in thread order
+// and a fixed tree. In batched solves the elements of a finished mesh (state 2) are skipped. It reads a
+// record and an index per element once; the cluster pass evaluated the owned elements only, on 44 % of
+// its threads.
+template <typename R> __global__ void __launch_bounds__(256) tet_energy_kernel(const DevMesh m, const EvalArgs a) {
+    __shared__ double s[8];
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    unsigned st = 0;
+    double E = 0;
+    if (e < m.T && !(a.emesh != nullptr && a.mstate[a.emesh[e]] == 2)) {
+        Kin<R> k;
+        st |= kinematics<R>(m, e, __ldg(m.tets + e), a.u, k);
+        const R Ee = k.vol * k.psi;
+        E = static_cast<double>(Ee);
+        if (a.elem_energy) a.elem_energy[e] = E;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) E += __shfl_xor_sync(0xffffffffu, E, off);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = E;
+    st = __reduce_or_sync(0xffffffffu, st);
+    if ((threadIdx.x & 31) == 0 && st) atomicOr(a.status, st);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int w = 0; w < 8; ++w) t += s[w];
+        a.cluster_energy[blockIdx.x] = t;
+        if (!isfinite(t)) atomicOr(a.status, static_cast<unsigned>(ST_NONFINITE_OUT));
+    }
+    finish_energy(a.cluster_energy, gridDim.x, a.energy, a.done);
+}
+
+// A launch over the tet clusters with events around it; without clusters the energy is zero.
+template <class Kern>
+void launch_clusters(Kern kernel, size_t sm, LaunchCache& cache, const DevMesh& m, const EvalArgs& a, cudaStream_t s) {
+    const int blocks = std::min(resident_grid(kernel, kTcThreads, sm, cache), m.tc_ncl);
     if (a.ev_begin) LPG_CUDA(cudaEventRecord(a.ev_begin, s));
-    if (blocks > 0) tet_cluster_kernel<R, WG, WH, MINB, UNR><<<blocks, kTcThreads, sm, s>>>(m, a);
+    if (blocks > 0)
+        kernel<<<blocks, kTcThreads, sm, s>>>(m, a);
+    else
+        LPG_CUDA(cudaMemsetAsync(a.energy, 0, sizeof(double), s));
+    if (a.ev_end) LPG_CUDA(cudaEventRecord(a.ev_end, s));
+    LPG_CUDA(cudaGetLastError());
+}
+template <typename R, bool WG, int MINB = tc_minb<R>(0), int UNR = tc_unroll(0)>
+void launch_tet_cluster(const DevMesh& m, const EvalArgs& a, cudaStream_t s) {
+    thread_local LaunchCache cache;
+    launch_clusters(tet_cluster_kernel<R, WG, MINB, UNR>, tc_smem_bytes<R>(), cache, m, a, s);
+}
+template <typename R> void launch_tet_gradient(const DevMesh& m, const EvalArgs& a, cudaStream_t s) {
+    thread_local LaunchCache cache;
+    launch_clusters(tet_gradient_kernel<R>, tg_smem_bytes<R>(), cache, m, a, s);
+}
+template <typename R> void launch_tet_energy(const DevMesh& m, const EvalArgs& a, cudaStream_t s) {
+    const int blocks = tet_energy_blocks(m);
+    if (a.ev_begin) LPG_CUDA(cudaEventRecord(a.ev_begin, s));
+    if (blocks > 0)
+        tet_energy_kernel<R><<<blocks, 256, 0, s>>>(m, a);
+    else
+        LPG_CUDA(cudaMemsetAsync(a.energy, 0, sizeof(double), s));
     if (a.ev_end) LPG_CUDA(cudaEventRecord(a.ev_end, s));
     LPG_CUDA(cudaGetLastError());
 }
@@ -3094,43 +3305,36 @@ __global__ void set_theta_kernel(double* rec64, float* rec32, const double* __re
 // The Hessian-writing tet cluster kernel in the launch variant a.cl_variant.
 template <typename R, bool WG> void launch_tet_variant(const DevMesh& m, const EvalArgs& a, cudaStream_t s) {
     switch (a.cl_variant) {
-    case 1: launch_tet_cluster<R, WG, true, tc_minb<R>(1), tc_unroll(1)>(m, a, s); break;
-    case 2: launch_tet_cluster<R, WG, true, tc_minb<R>(2), tc_unroll(2)>(m, a, s); break;
-    default: launch_tet_cluster<R, WG, true>(m, a, s); break;
+    case 1: launch_tet_cluster<R, WG, tc_minb<R>(1), tc_unroll(1)>(m, a, s); break;
+    case 2: launch_tet_cluster<R, WG, tc_minb<R>(2), tc_unroll(2)>(m, a, s); break;
+    default: launch_tet_cluster<R, WG>(m, a, s); break;
     }
 }
 
-// Launches the element pass; returns the number of per-unit energies it wrote to cluster_energy.
-// Energy, gradient and the Exact Hessian come from the tet cluster kernel; the projected Hessian
-// is gathered from the per-element clamped blocks by the block gather.
-template <typename R> int launch_eval_t(const DevMesh& m, int hessian, const EvalArgs& a, cudaStream_t s) {
+// Launches the element pass. Energy, gradient and the Exact Hessian come from the tet cluster kernel, the
+// energy with or without the gradient from kernels of their own; the projected Hessian is gathered from
+// the per-element clamped blocks by the block gather (the optional events bracket both kernels).
+template <typename R> void launch_eval_t(const DevMesh& m, int hessian, const EvalArgs& a, cudaStream_t s) {
     const bool wg = a.grad != nullptr;
-    const int wh = a.hess == nullptr ? 0 : (hessian == LPG_HESSIAN_EXACT ? 1 : 2);
-    const int units = m.tc_ncl;
-    if (wh == 2) {
-        // Projected: energy (and gradient) from the element pass, the Hessian gathered from the
-        // per-element clamped blocks; the optional events bracket both kernels.
-        EvalArgs ea = a;
-        ea.ev_end = nullptr;
-        ea.hess = nullptr;
+    if (a.hess != nullptr && hessian == LPG_HESSIAN_EXACT) {
         if (wg)
-            launch_tet_cluster<R, true, false>(m, ea, s);
+            launch_tet_variant<R, true>(m, a, s);
         else
-            launch_tet_cluster<R, false, false>(m, ea, s);
-        launch_block_gather<R>(m, a, s);
-        if (a.ev_end) LPG_CUDA(cudaEventRecord(a.ev_end, s));
-    } else if (wg && wh == 1) {
-        launch_tet_variant<R, true>(m, a, s);
-    } else if (!wg && wh == 1) {
-        launch_tet_variant<R, false>(m, a, s);
-    } else if (wg) {
-        launch_tet_cluster<R, true, false>(m, a, s);
+            launch_tet_variant<R, false>(m, a, s);
     } else {
-        launch_tet_cluster<R, false, false>(m, a, s);
+        EvalArgs ea = a;
+        if (a.hess) ea.ev_end = nullptr;
+        if (wg)
+            launch_tet_gradient<R>(m, ea, s);
+        else
+            launch_tet_energy<R>(m, ea, s);
+        if (a.hess) {
+            launch_block_gather<R>(m, a, s);
+            if (a.ev_end) LPG_CUDA(cudaEventRecord(a.ev_end, s));
+        }
     }
     if (wg && m.num_unused > 0)
         zero_rows_kernel<<<(m.num_unused + 255) / 256, 256, 0, s>>>(a.grad, m.unused_rows, m.num_unused);
-    return units;
 }
 
 } // namespace
@@ -3138,15 +3342,16 @@ template <typename R> int launch_eval_t(const DevMesh& m, int hessian, const Eva
 size_t assembly_smem_bytes(const DevMesh& m) {
     const size_t gather = block_gather_bytes(m);
     if (m.K != 4) return gather;
-    return std::max(gather, std::max(tc_smem_bytes<double>(), tc_smem_bytes<float>()));
+    return std::max(gather, std::max(tc_smem_bytes<double>(), tc_smem_bytes<float>())); // the gradient pass needs less
 }
 
+int tet_energy_blocks(const DevMesh& m) { return (m.T + 255) / 256; }
+
 void launch_eval(const DevMesh& m, int precision, int hessian, const EvalArgs& a, cudaStream_t s) {
-    const int units = precision == LPG_PRECISION_F64 ? launch_eval_t<double>(m, hessian, a, s)
-                                                      : launch_eval_t<float>(m, hessian, a, s);
-    // Per-unit energies -> partials (stored after the units) -> total.
-    sum_partial_kernel<<<kSumBlocks, 256, 0, s>>>(a.cluster_energy, units, a.cluster_energy + units);
-    sum_final_kernel<<<1, 256, 0, s>>>(a.cluster_energy + units, kSumBlocks, a.energy);
+    if (precision == LPG_PRECISION_F64)
+        launch_eval_t<double>(m, hessian, a, s);
+    else
+        launch_eval_t<float>(m, hessian, a, s);
     LPG_CUDA(cudaGetLastError());
 }
 
@@ -3301,8 +3506,7 @@ void launch_material_eval(const DevMesh& m, int precision, int hessian, const do
     if (a.grad && m.num_unused > 0)
         zero_rows_kernel<<<(m.num_unused + 255) / 256, 256, 0, s>>>(a.grad, m.unused_rows, m.num_unused);
     // Energy: the per-element energies summed in a fixed order.
-    sum_partial_kernel<<<kSumBlocks, 256, 0, s>>>(elemE, m.T, a.cluster_energy);
-    sum_final_kernel<<<1, 256, 0, s>>>(a.cluster_energy, kSumBlocks, a.energy);
+    launch_sum(elemE, m.T, a, s);
     if (a.hess && m.T > 0) {
         const MatTangent src{A, hessian == LPG_HESSIAN_EXACT};
         EvalArgs ga = a;
@@ -3367,8 +3571,7 @@ void launch_hex_material_eval(const DevMesh& m, int precision, int hessian, cons
     }
     if (a.grad && m.num_unused > 0)
         zero_rows_kernel<<<(m.num_unused + 255) / 256, 256, 0, s>>>(a.grad, m.unused_rows, m.num_unused);
-    sum_partial_kernel<<<kSumBlocks, 256, 0, s>>>(elemE, m.T, a.cluster_energy);
-    sum_final_kernel<<<1, 256, 0, s>>>(a.cluster_energy, kSumBlocks, a.energy);
+    launch_sum(elemE, m.T, a, s);
     LPG_CUDA(cudaGetLastError());
 }
 
@@ -3429,8 +3632,7 @@ void launch_hermite_eval(const DevMesh& m, int precision, bool projected, const 
     }
     if (a.grad && m.num_unused > 0)
         zero_rows_kernel<<<(m.num_unused + 255) / 256, 256, 0, s>>>(a.grad, m.unused_rows, m.num_unused);
-    sum_partial_kernel<<<kSumBlocks, 256, 0, s>>>(elemE, m.T, a.cluster_energy);
-    sum_final_kernel<<<1, 256, 0, s>>>(a.cluster_energy, kSumBlocks, a.energy);
+    launch_sum(elemE, m.T, a, s);
     LPG_CUDA(cudaGetLastError());
 }
 
@@ -3482,8 +3684,7 @@ void launch_hex_eval(const DevMesh& m, int precision, bool projected, const doub
     }
     if (a.grad && m.num_unused > 0)
         zero_rows_kernel<<<(m.num_unused + 255) / 256, 256, 0, s>>>(a.grad, m.unused_rows, m.num_unused);
-    sum_partial_kernel<<<kSumBlocks, 256, 0, s>>>(elemE, m.T, a.cluster_energy);
-    sum_final_kernel<<<1, 256, 0, s>>>(a.cluster_energy, kSumBlocks, a.energy);
+    launch_sum(elemE, m.T, a, s);
     LPG_CUDA(cudaGetLastError());
 }
 

@@ -91,7 +91,9 @@ struct HostPlan {
     // higher-numbered vertex (a = b for a diagonal block), ascending by element (the
     // reference's per-column order).
     std::vector<int32_t> tc_row_ptr, tc_rows, tc_row_so;
-    std::vector<int32_t> tc_el_ptr, tc_vert_ptr, tc_verts, tc_item_ptr, tc_ndiag, tc_ent_ptr;
+    // tc_dent: a cluster's contributors of its diagonal items (the first of its list), rounded up
+    // to a multiple of 8: what the gradient-only pass stages.
+    std::vector<int32_t> tc_el_ptr, tc_vert_ptr, tc_verts, tc_item_ptr, tc_ndiag, tc_ent_ptr, tc_dent;
     std::vector<uint32_t> tc_els, tc_loc, tc_items;
     std::vector<uint16_t> tc_ents;
     // Value count of the solver layout: 9 per own slot, then the 9 x 32 zero block.
@@ -187,7 +189,7 @@ struct DevMesh {
     int tc_ncl = 0, tc_max_els = 0, tc_max_verts = 0, tc_max_vals = 0;
     int32_t *tc_row_ptr = nullptr, *tc_rows = nullptr, *tc_row_so = nullptr, *tc_el_ptr = nullptr,
             *tc_vert_ptr = nullptr, *tc_verts = nullptr, *tc_item_ptr = nullptr, *tc_ndiag = nullptr,
-            *tc_ent_ptr = nullptr;
+            *tc_ent_ptr = nullptr, *tc_dent = nullptr;
     uint32_t *tc_els = nullptr, *tc_loc = nullptr;
     uint4* tc_items = nullptr;
     uint16_t* tc_ents = nullptr;
@@ -226,6 +228,7 @@ struct EvalArgs {
     int layout = LPG_LAYOUT_BSR;
     double* cluster_energy = nullptr; // device, one per cluster (always written)
     double* energy = nullptr;      // device scalar (always written)
+    unsigned* done = nullptr;      // device counter of finished blocks, zero between launches
     double* elem_energy = nullptr; // device, T, or null
     const void* proj = nullptr;    // projected per-element 9x9 tangents (hessian PROJECTED*), or null
     unsigned* status = nullptr;    // device status word
@@ -235,6 +238,9 @@ struct EvalArgs {
     // mesh has finished; such a cluster writes nothing. Null: every cluster runs.
     const unsigned char* tc_skip = nullptr;
     const unsigned char* cl_skip = nullptr;
+    // The same per element for the energy-only pass: element -> mesh and per-mesh state (2 finished).
+    const int* emesh = nullptr;
+    const int* mstate = nullptr;
 };
 
 // Autotuned launch variants (register budgets and unroll depths; every variant of a kernel
@@ -251,6 +257,8 @@ struct Tuning {
     bool tuned = false;
 };
 void launch_eval(const DevMesh& m, int precision, int hessian, const EvalArgs& a, cudaStream_t s);
+// Blocks (and partial energies) of the tet energy-only pass.
+int tet_energy_blocks(const DevMesh& m);
 // Largest dynamic shared memory any assembly kernel of this mesh's cell type needs for its
 // largest cluster (the same formulas the launches use).
 size_t assembly_smem_bytes(const DevMesh& m);

@@ -748,7 +748,7 @@ void eval_elastic_async(lpg_fem& h, const lpg_newton_terms* t, const double* x, 
     double* W = h.d_mat[0].as<double>(std::max<size_t>(rows, 1));
     double* P = h.d_mat[1].as<double>(std::max<size_t>(9 * rows, 1));
     double* A = hk != LPG_HESSIAN_NONE ? h.d_mat[2].as<double>(std::max<size_t>(81 * rows, 1)) : nullptr;
-    unsigned* status = h.d_status.as<unsigned>(1);
+    unsigned* status = h.status_word();
     if (hex)
         launch_hex_deformation_gradients(m, x, F, status, s);
     else
@@ -762,7 +762,8 @@ void eval_elastic_async(lpg_fem& h, const lpg_newton_terms* t, const double* x, 
     a.hess = hk != LPG_HESSIAN_NONE ? K : nullptr;
     a.layout = layout;
     a.cluster_energy = h.d_cluster_energy.as<double>(static_cast<size_t>(std::max(m.ncl, m.tc_ncl)) + 256);
-    a.energy = h.d_energy.as<double>(1);
+    a.energy = h.energy_word();
+    a.done = h.done_word();
     a.status = status;
     const int pi = prec == LPG_PRECISION_F64 ? 0 : 1;
     if (hex) {
@@ -810,7 +811,7 @@ struct Solver {
         eval_elastic_async(h, P ? P->t : nullptr, x, g, LPG_HESSIAN_NONE, LPG_PRECISION_F64, LPG_LAYOUT_BSR, nullptr);
         return compose(x, f, g);
     }
-    // The potential from the elastic evaluation just enqueued (energy in h.d_energy, gradient
+    // The potential from the elastic evaluation just enqueued (energy in h.result(), gradient
     // in g if given): weight, quadratic term, load and constant.
     double compose(const double* x, const double* f, double* g) {
         double aq = 0;
@@ -822,9 +823,8 @@ struct Solver {
             LPG_CUDA(cudaGetLastError());
         }
         if (g && f) load_gradient<<<grid(n), kThreads, 0, s>>>(g, f, n);
-        double e = 0;
-        LPG_CUDA(cudaMemcpyAsync(&e, h.d_energy.ptr, sizeof e, cudaMemcpyDeviceToHost, s));
         raise_status(h.take_status());
+        double e = h.host_result->energy;
         if (P && P->n > 0) aq = 0.5 * stats<double, double>(x, P->Ax, nullptr)[0];
         if (P) e = P->w * e + aq + P->c;
         return e - energy_dot_f(x, f);
@@ -1281,7 +1281,7 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
             const size_t rows = static_cast<size_t>(h.dm.T) * (hex ? h.dm.nq : 1);
             double* Fx = h.d_mat[4].as<double>(std::max<size_t>(9 * rows, 1));
             double* Gd = h.d_mat[5].as<double>(std::max<size_t>(9 * rows, 1));
-            unsigned* stw = h.d_status.as<unsigned>(1);
+            unsigned* stw = h.status_word();
             if (hex) {
                 launch_hex_deformation_gradients(h.dm, x, Fx, stw, s);
                 launch_hex_deformation_gradients(h.dm, d, Gd, stw, s);
@@ -1295,7 +1295,7 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
             if (!(alpha >= 0.0 && alpha <= 1.0))
                 fail(LPG_ELOGIC, "Energy::max_feasible_step: the energy returned a value outside [0, 1]");
         } else {
-            launch_feasible(h.dm, x, d, bm, nb, al, h.d_status.as<unsigned>(1), s);
+            launch_feasible(h.dm, x, d, bm, nb, al, h.status_word(), s);
             LPG_CUDA(cudaMemcpyAsync(&alpha, al, sizeof alpha, cudaMemcpyDeviceToHost, s));
             raise_status(h.take_status());
         }
@@ -1411,7 +1411,7 @@ void adjoint_theta(lpg_fem& h, const double* u_star, const double* dLdu, const i
     const size_t T = static_cast<size_t>(h.dm.T);
     // dtheta = -(dg/dtheta)^T lambda.
     double* pe = h.d_vjp.as<double>(std::max<size_t>(2 * T, 2));
-    launch_force_vjp(h.dm, u, lam, pe, h.d_status.as<unsigned>(1), s);
+    launch_force_vjp(h.dm, u, lam, pe, h.status_word(), s);
     std::vector<double> host;
     if (per_element) {
         host.resize(2 * T);
@@ -1444,7 +1444,7 @@ void adjoint_fp(lpg_fem& h, const double* u_star, const double* dLdu, const int3
     const size_t T = static_cast<size_t>(h.dm.T);
     // dFp = -(dg/dFp)^T lambda.
     double* pe = h.d_vjp.as<double>(std::max<size_t>(9 * T, 9));
-    launch_fp_vjp(h.dm, u, lam, pe, h.d_status.as<unsigned>(1), s);
+    launch_fp_vjp(h.dm, u, lam, pe, h.status_word(), s);
     std::vector<double> host;
     if (per_element) {
         host.resize(9 * T);
@@ -1478,7 +1478,7 @@ void adjoint_rest(lpg_fem& h, const double* u_star, const double* dLdu, const in
     // dX = -(dg/dX)^T lambda.
     double* out = io_mem == LPG_MEM_DEVICE ? dX : h.d_grad.as<double>(std::max<size_t>(n, 1));
     double* pe = h.d_vjp.as<double>(std::max<size_t>(12 * static_cast<size_t>(h.dm.T), 1));
-    launch_rest_vjp(h.dm, u, lam, pe, -1.0, out, h.d_status.as<unsigned>(1), s);
+    launch_rest_vjp(h.dm, u, lam, pe, -1.0, out, h.status_word(), s);
     raise_status(h.take_status());
     if (io_mem == LPG_MEM_HOST && n > 0) LPG_CUDA(cudaMemcpyAsync(dX, out, n * sizeof(double), cudaMemcpyDeviceToHost, s));
     copy_lambda(h, lam, io_mem, lambda_out);
@@ -2201,7 +2201,7 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
         }
         for (int m = 0; m < M; ++m) gd[m] = gds[4 * m];
         // Line search per mesh from its feasible step.
-        launch_feasible(h.dm, x, dir, bm, nfeas, al, h.d_status.as<unsigned>(1), s, d.elem, d.emesh, d.exact);
+        launch_feasible(h.dm, x, dir, bm, nfeas, al, h.status_word(), s, d.elem, d.emesh, d.exact);
         seg_elem<<<M, 256, 0, s>>>(d.elem, d.eoff, 1, d.amin);
         raise_status(h.take_status());
         std::vector<double> amin;

@@ -39,13 +39,13 @@ struct lpg_fem {
     lpg::DeviceBuffer b_herm;   // Hermite hex meshes: box edge lengths per element
     lpg::DeviceBuffer d_herm_q; // Hermite projected Hessian: eigenvector scratch, 192^2 doubles per CTA
     lpg::DeviceBuffer b_cl[11]; // assembly clusters
-    lpg::DeviceBuffer b_tc[13]; // tet assembly clusters
+    lpg::DeviceBuffer b_tc[14]; // tet assembly clusters
     lpg::DeviceBuffer b_sell[6]; // sliced-ELL pattern of the solvers
     lpg::DeviceBuffer bt_int[8], bt_dbl[4], bt_skip[2]; // batched Newton (bt_skip: per-cluster skip flags)
     // Scratch of the evaluation entry points.
     lpg::DeviceBuffer d_plist, d_pcount; // elements listed for the projection's eigenvalue clamp
     lpg::DeviceBuffer d_mat[6];          // material outputs (W, P, A), per-element energies, F and G
-    lpg::DeviceBuffer d_status, d_cluster_energy, d_energy, d_block, d_alpha, d_u, d_u2, d_grad, d_hess, d_proj, d_vjp;
+    lpg::DeviceBuffer d_result, d_cluster_energy, d_block, d_alpha, d_u, d_u2, d_grad, d_hess, d_proj, d_vjp;
     // Solver state (Newton / PCG / adjoint).
     lpg::DeviceBuffer s_x, s_g, s_f, s_d, s_trial, s_mask, s_hess, s_hess64, s_dinv, s_r, s_z, s_p, s_ap, s_xcg, s_r64,
         s_b64, s_scal, s_part, s_flag, d_flush, s_p2, s_mask4;
@@ -57,8 +57,23 @@ struct lpg_fem {
     const void* pcg_graph_key[12] = {};
     cudaGraphExec_t batch_graph = nullptr; // the batched (per-mesh) PCG iterations
     const void* batch_graph_key[12] = {};
+    // What an evaluation leaves for the host, one 16-byte record on the device (d_result) and its
+    // copy in pinned host memory (host_result): take_status() moves it in one transfer.
+    struct EvalResult {
+        double energy;   // the last evaluation's energy
+        unsigned status; // status bits since the last take_status()
+        unsigned done;   // block counter of the energy sum (zero between launches)
+    };
+    EvalResult* host_result = nullptr;
+    EvalResult* result() { return static_cast<EvalResult*>(d_result.ptr); }
+    double* energy_word() { return &result()->energy; }
+    unsigned* status_word() { return &result()->status; }
+    unsigned* done_word() { return &result()->done; }
+    void create_result(); // allocates and clears both records
     ~lpg_fem();
     void sync();
+    // Waits for the stream and returns (and clears) the status bits; host_result->energy is then
+    // the last evaluation's energy.
     unsigned take_status();
     const double* stage_in(const double* p, int mem, lpg::DeviceBuffer& buf, size_t n);
     // Enqueues one evaluation on the handle's stream (no synchronisation).
