@@ -275,12 +275,9 @@ void lpg_fem::eval_async(const double* du, double* dgrad, int hessian, int preci
         const size_t T = static_cast<size_t>(dm.T);
         double* elemE = delem ? delem : d_mat[3].as<double>(std::max<size_t>(T, 1));
         void* blocks = a.hess ? d_proj.ensure(hermite_blocks_bytes(dm, precision, projected)) : nullptr;
-        int* flags = projected && a.hess ? d_plist.as<int>(std::max<size_t>(T, 1)) : nullptr;
-        double* qbuf = projected && a.hess && T > 0
-                           ? d_herm_q.as<double>(static_cast<size_t>(hermite_psd_grid(dm)) * 192 * 192)
-                           : nullptr;
+        double* scratch = projected && a.hess && T > 0 ? d_herm_q.as<double>(hermite_scratch_doubles(dm)) : nullptr;
         launch_hermite_eval(dm, precision, projected, du, elemE, d_vjp.as<double>(std::max<size_t>(192 * T, 1)), blocks,
-                            flags, qbuf, a, stream);
+                            scratch, a, stream);
         return;
     }
     if (dm.K == 8) {
@@ -289,9 +286,8 @@ void lpg_fem::eval_async(const double* du, double* dgrad, int hessian, int preci
         double* elemE = delem ? delem : d_mat[3].as<double>(std::max<size_t>(T, 1));
         void* blocks = a.hess ? d_proj.ensure(hex_blocks_bytes(dm, precision, projected)) : nullptr;
         a.cluster_energy = d_cluster_energy.as<double>(static_cast<size_t>(std::max(dm.ncl, dm.tc_ncl)) + 256);
-        int* flags = projected && a.hess ? d_plist.as<int>(std::max<size_t>(T, 1)) : nullptr;
         launch_hex_eval(dm, precision, projected, du, elemE, d_vjp.as<double>(std::max<size_t>(24 * T, 1)), blocks,
-                        flags, a, stream);
+                        a, stream);
         return;
     }
     if (a.hess && hessian == LPG_HESSIAN_PROJECTED) {
@@ -773,8 +769,7 @@ int lpg_fem_eval_material(lpg_fem_t h, const double* W, const double* P, const d
             const bool projected = hessian == LPG_HESSIAN_PROJECTED;
             void* blocks = a.hess ? h->d_proj.ensure(hex_blocks_bytes(h->dm, precision, projected)) : nullptr;
             launch_hex_material_eval(h->dm, precision, hessian, dW, dP, dA, h->d_mat[3].as<double>(nel),
-                                     h->d_vjp.as<double>(24 * nel), blocks,
-                                     projected && a.hess ? h->d_plist.as<int>(nel) : nullptr, a, s);
+                                     h->d_vjp.as<double>(24 * nel), blocks, a, s);
         } else {
             void* proj = a.hess ? h->d_proj.ensure(project_bytes(h->dm, precision)) : nullptr;
             launch_material_eval(h->dm, precision, hessian, dW, dP, dA, h->d_mat[3].as<double>(nel),

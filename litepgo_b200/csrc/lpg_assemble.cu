@@ -27,6 +27,7 @@
 
 #include "lpg_internal.h"
 #include "lpg_clamp9.h"
+#include "lpg_eig.cuh"
 #include "lpg_psd.h"
 
 namespace lpg {
@@ -2102,13 +2103,15 @@ __global__ void __launch_bounds__(256) material_pieces_kernel(const DevMesh m, c
 
 // ---------------------------------------------------------------------------
 // Hex Q1 neo-Hookean element pass (VolumetricFemEnergy<NeoHookean, HexQ1Basis, GaussLegendre3D<n>>,
-// volumetric_fem_energy.hpp:78-123 with hex_q1_basis.hpp and gauss_legendre_3d.hpp). One thread
-// per (element, vertex pair a <= b): at every quadrature point it forms J = sum_c X_c dN_c^T,
-// w = weight det J, grad N = J^-T dN, F = I + (sum_c u_c dN_c^T) J^-1, and accumulates
-// H_ab += w [mu (grad N_a . grad N_b) I + lambda h_a h_b^T - p h_b h_a^T], h = F^-T grad N; the
-// pair (a, a) threads also accumulate g_a = sum w P grad N_a and the (0, 0) thread the energy.
-// FP64 throughout; the blocks are stored in the precision's type. The kinematics are recomputed
-// by each of an element's 36 threads (cheap next to reading a per-point cache).
+// volumetric_fem_energy.hpp:78-123 with hex_q1_basis.hpp and gauss_legendre_3d.hpp), seven elements per
+// block. Per quadrature point a thread forms J = sum_c X_c dN_c^T, w = weight det J, grad N = J^-T dN,
+// F = I + (sum_c u_c dN_c^T) J^-1 and h = F^-T grad N once, into shared memory (eight points of the seven
+// elements at a time); then one thread per (element, vertex pair a <= b) accumulates
+// H_ab += w [mu (grad N_a . grad N_b) I + lambda h_a h_b^T - p h_b h_a^T], the pairs (a, a) also
+// g_a = sum w P grad N_a and the pair (0, 0) the energy. FP64 throughout; the blocks are stored in the
+// precision's type. FP64-bound: each of an element's 36 threads used to form the point's kinematics itself.
+// 7,480 hexes at 8 points: 105 -> 33 us (two 256-thread blocks per SM; eight elements in 288 threads left
+// one block per SM and took 44 us).
 // ---------------------------------------------------------------------------
 // The rest geometry at one quadrature point of a hex (dq: the point's table row): J = sum_c X_c
 // dN_c^T (corners in order, fma per entry), its determinant and its inverse by cofactors.
@@ -2147,104 +2150,138 @@ __device__ __forceinline__ void hex_pair(int pr, int& a, int& b) {
     b = a + (pr - base);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(128) hex_element_kernel(const DevMesh m, const double* __restrict__ u,
-                                                          double* __restrict__ elemE, double* __restrict__ per_elem,
-                                                          R* __restrict__ blocks, unsigned* status) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// What the pairs read of one quadrature point: per node grad N and h = F^-T grad N (6 values), then
+// w lambda, w p, w mu, w P (9, row-major) and w psi.
+constexpr int kHexPoint = 61, kHexL = 48, kHexPp = 49, kHexMu = 50, kHexP = 51, kHexPsi = 60;
+constexpr int kHexEl = 7;                    // elements per block
+constexpr int kHexThreads = 256;             // one thread per (element, pair), four idle
+static_assert(36 * kHexEl <= kHexThreads, "one thread per (element, pair)");
+constexpr int kHexChunk = 8;                 // points kept at a time
+
+// One quadrature point of a hex into rec (kHexPoint values); a point with a bad F contributes zeros.
+__device__ __forceinline__ unsigned hex_point(const DevMesh& m, int e, int q, const double* __restrict__ u, double* rec) {
     unsigned st = 0;
-    const int e = t / 36, pr = t - 36 * (t / 36);
-    if (e < m.T) {
-        int a, b;
-        hex_pair(pr, a, b);
-        const int32_t* cell = m.hex_cells + 8 * static_cast<size_t>(e);
-        const double lam = m.hex_theta[2 * static_cast<size_t>(e)], mu = m.hex_theta[2 * static_cast<size_t>(e) + 1];
-        if (!(lam >= 0 && mu > 0 && isfinite(lam) && isfinite(mu))) st |= ST_BAD_THETA;
-        double Hb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, ga[3] = {0, 0, 0}, E = 0;
-        for (int q = 0; q < m.nq; ++q) {
-            const double* dq = m.hex_q + 25 * static_cast<size_t>(q);
-            // J^-1 (det J > 0 was checked when the mesh was built) and grad u in reference coordinates.
-            double Ji[9], dJ;
-            hex_point_geometry(m, cell, dq, Ji, dJ);
-            double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            bool ok = true;
-            for (int c = 0; c < 8; ++c) {
-                const int v = __ldg(cell + c);
+    const int32_t* cell = m.hex_cells + 8 * static_cast<size_t>(e);
+    const double lam = m.hex_theta[2 * static_cast<size_t>(e)], mu = m.hex_theta[2 * static_cast<size_t>(e) + 1];
+    if (!(lam >= 0 && mu > 0 && isfinite(lam) && isfinite(mu))) st |= ST_BAD_THETA;
+    const double* dq = m.hex_q + 25 * static_cast<size_t>(q);
+    // J^-1 (det J > 0 was checked when the mesh was built) and grad u in reference coordinates.
+    double Ji[9], dJ;
+    hex_point_geometry(m, cell, dq, Ji, dJ);
+    double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    bool ok = true;
+    for (int c = 0; c < 8; ++c) {
+        const int v = __ldg(cell + c);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double uu = __ldg(u + 3 * static_cast<size_t>(v) + i);
+            ok = ok && isfinite(uu);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) G[3 * i + d] = fma(uu, __ldg(dq + 3 * c + d), G[3 * i + d]);
+        }
+    }
+    if (!ok) st |= ST_BAD_INPUT;
+    const double w = __ldg(dq + 24) * dJ;
+    double F[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            F[3 * i + j] = (i == j ? 1.0 : 0.0) + G[3 * i] * Ji[j] + G[3 * i + 1] * Ji[3 + j] + G[3 * i + 2] * Ji[6 + j];
+    double C[9]; // cofactors: F^-T = C / det F
+    C[0] = F[4] * F[8] - F[5] * F[7];
+    C[1] = F[5] * F[6] - F[3] * F[8];
+    C[2] = F[3] * F[7] - F[4] * F[6];
+    C[3] = F[2] * F[7] - F[1] * F[8];
+    C[4] = F[0] * F[8] - F[2] * F[6];
+    C[5] = F[1] * F[6] - F[0] * F[7];
+    C[6] = F[1] * F[5] - F[2] * F[4];
+    C[7] = F[2] * F[3] - F[0] * F[5];
+    C[8] = F[0] * F[4] - F[1] * F[3];
+    const double detF = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
+    if (!(detF > 0) || !isfinite(detF)) {
+        st |= isfinite(detF) ? ST_BAD_DET : ST_NONFINITE_F;
+        for (int t = 0; t < kHexPoint; ++t) rec[t] = 0.0;
+        return st;
+    }
+    const double L = log(detF), p = lam * L - mu, iF = 1.0 / detF;
+    double FiT[9], ff = 0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        FiT[k] = C[k] * iF;
+        ff += F[k] * F[k];
+        rec[kHexP + k] = w * (mu * F[k] + p * FiT[k]);
+    }
+    rec[kHexL] = w * lam;
+    rec[kHexPp] = w * p;
+    rec[kHexMu] = w * mu;
+    rec[kHexPsi] = w * (0.5 * mu * (ff - 3.0) - mu * L + 0.5 * lam * L * L);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        double n[3]; // rows of dN J^-1
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            n[j] = __ldg(dq + 3 * c) * Ji[j] + __ldg(dq + 3 * c + 1) * Ji[3 + j] + __ldg(dq + 3 * c + 2) * Ji[6 + j];
+            rec[6 * c + j] = n[j];
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) rec[6 * c + 3 + i] = FiT[3 * i] * n[0] + FiT[3 * i + 1] * n[1] + FiT[3 * i + 2] * n[2];
+    }
+    return st;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kHexThreads, 2) hex_element_kernel(const DevMesh m, const double* __restrict__ u,
+                                                                  double* __restrict__ elemE,
+                                                                  double* __restrict__ per_elem,
+                                                                  R* __restrict__ blocks, unsigned* status) {
+    __shared__ double sp[kHexEl * kHexChunk * kHexPoint];
+    const int tid = threadIdx.x, el = tid / 36, pr = tid - 36 * el;
+    const int e0 = blockIdx.x * kHexEl, e = e0 + el;
+    unsigned st = 0;
+    const bool on = el < kHexEl && e < m.T;
+    int a, b;
+    hex_pair(pr, a, b);
+    double Hb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, ga[3] = {0, 0, 0}, E = 0;
+    for (int q0 = 0; q0 < m.nq; q0 += kHexChunk) {
+        const int nq = min(kHexChunk, m.nq - q0);
+        __syncthreads(); // the previous points are read
+        for (int t = tid; t < kHexEl * nq; t += kHexThreads) {
+            const int te = e0 + t / nq, tq = t - nq * (t / nq);
+            if (te < m.T) st |= hex_point(m, te, q0 + tq, u, sp + kHexPoint * ((t / nq) * kHexChunk + tq));
+        }
+        __syncthreads();
+        if (!on) continue;
+        for (int q = 0; q < nq; ++q) {
+            const double* rec = sp + kHexPoint * (el * kHexChunk + q);
+            const double* ra = rec + 6 * a;
+            const double* rb = rec + 6 * b;
+            if (blocks) {
+                const double wl = rec[kHexL], wp = rec[kHexPp];
+                const double dn = rec[kHexMu] * (ra[0] * rb[0] + ra[1] * rb[1] + ra[2] * rb[2]);
+                const double hb[3] = {rb[3], rb[4], rb[5]};
+                double la[3], pa[3];
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    const double uu = __ldg(u + 3 * static_cast<size_t>(v) + i);
-                    ok = ok && isfinite(uu);
+                    la[i] = wl * ra[3 + i];
+                    pa[i] = -wp * ra[3 + i];
+                }
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) G[3 * i + d] = fma(uu, __ldg(dq + 3 * c + d), G[3 * i + d]);
+                for (int i = 0; i < 3; ++i) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) Hb[3 * i + k] = fma(la[i], hb[k], fma(hb[i], pa[k], Hb[3 * i + k]));
+                    Hb[4 * i] += dn;
                 }
             }
-            if (!ok) st |= ST_BAD_INPUT;
-            const double w = __ldg(dq + 24) * dJ;
-            double F[9];
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j)
-                    F[3 * i + j] = (i == j ? 1.0 : 0.0) + G[3 * i] * Ji[j] + G[3 * i + 1] * Ji[3 + j] + G[3 * i + 2] * Ji[6 + j];
-            double C[9]; // cofactors: F^-T = C / det F
-            C[0] = F[4] * F[8] - F[5] * F[7];
-            C[1] = F[5] * F[6] - F[3] * F[8];
-            C[2] = F[3] * F[7] - F[4] * F[6];
-            C[3] = F[2] * F[7] - F[1] * F[8];
-            C[4] = F[0] * F[8] - F[2] * F[6];
-            C[5] = F[1] * F[6] - F[0] * F[7];
-            C[6] = F[1] * F[5] - F[2] * F[4];
-            C[7] = F[2] * F[3] - F[0] * F[5];
-            C[8] = F[0] * F[4] - F[1] * F[3];
-            const double detF = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
-            if (!(detF > 0) || !isfinite(detF)) {
-                st |= isfinite(detF) ? ST_BAD_DET : ST_NONFINITE_F;
-                continue;
-            }
-            const double L = log(detF), p = lam * L - mu;
-            double FiT[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) FiT[k] = C[k] / detF;
-            // grad N of a and b: rows of dN J^-1.
-            double na[3], nb[3];
-            const double* dA = dq + 3 * a;
-            const double* dB = dq + 3 * b;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                na[j] = __ldg(dA) * Ji[j] + __ldg(dA + 1) * Ji[3 + j] + __ldg(dA + 2) * Ji[6 + j];
-                nb[j] = __ldg(dB) * Ji[j] + __ldg(dB + 1) * Ji[3 + j] + __ldg(dB + 2) * Ji[6 + j];
-            }
-            double ha[3], hb[3];
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                ha[i] = FiT[3 * i] * na[0] + FiT[3 * i + 1] * na[1] + FiT[3 * i + 2] * na[2];
-                hb[i] = FiT[3 * i] * nb[0] + FiT[3 * i + 1] * nb[1] + FiT[3 * i + 2] * nb[2];
-            }
-            const double dn = na[0] * nb[0] + na[1] * nb[1] + na[2] * nb[2];
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    double v = lam * ha[i] * hb[k] - p * hb[i] * ha[k];
-                    if (i == k) v += mu * dn;
-                    Hb[3 * i + k] = fma(w, v, Hb[3 * i + k]);
-                }
             if (a == b) {
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    double s = 0;
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) s += (mu * F[3 * i + j] + p * FiT[3 * i + j]) * na[j];
-                    ga[i] = fma(w, s, ga[i]);
-                }
-                if (a == 0) {
-                    double ff = 0;
-#pragma unroll
-                    for (int k = 0; k < 9; ++k) ff += F[k] * F[k];
-                    E = fma(w, 0.5 * mu * (ff - 3.0) - mu * L + 0.5 * lam * L * L, E);
-                }
+                for (int i = 0; i < 3; ++i)
+                    ga[i] += rec[kHexP + 3 * i] * ra[0] + rec[kHexP + 3 * i + 1] * ra[1] + rec[kHexP + 3 * i + 2] * ra[2];
+                if (a == 0) E += rec[kHexPsi];
             }
         }
+    }
+    if (on) {
         if (a == b) { // a diagonal block: mirror the upper triangle so the matrix is bitwise symmetric
             Hb[3] = Hb[1];
             Hb[6] = Hb[2];
@@ -2271,7 +2308,7 @@ __global__ void __launch_bounds__(128) hex_element_kernel(const DevMesh m, const
         }
     }
     st = __reduce_or_sync(0xffffffffu, st);
-    if ((threadIdx.x & 31) == 0 && st) atomicOr(status, st);
+    if ((tid & 31) == 0 && st) atomicOr(status, st);
 }
 
 // Force-response parameter VJP of hex meshes (the tet pass's force_vjp_kernel at every
@@ -2470,102 +2507,16 @@ __global__ void __launch_bounds__(128) hex_material_kernel(const DevMesh m, cons
     if ((threadIdx.x & 31) == 0 && st) atomicOr(status, st);
 }
 
-// The projection pre-test on a material's own tangents: one thread per (element, point), the
-// symmetrised As = (A + A^T) / 2 through the LDL^T test; an element with a point that fails is
-// marked in flags (zeroed before).
-__global__ void __launch_bounds__(128) hex_material_tangent_test_kernel(const DevMesh m, const double* __restrict__ A,
-                                                                        int* __restrict__ flags) {
-    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= static_cast<size_t>(m.T) * m.nq) return;
-    const int e = static_cast<int>(t / m.nq);
-    const double* Aq = A + 81 * t;
-    double V[81];
-    double scale = 0;
-    for (int r = 0; r < 9; ++r)
-        for (int c = 0; c < 9; ++c) {
-            const double v = 0.5 * (__ldg(Aq + 9 * r + c) + __ldg(Aq + 9 * c + r));
-            V[9 * r + c] = v;
-            if (r == c) scale = fmax(scale, fabs(v));
-        }
-    if (!(scale < INFINITY) || !semidefinite_ldlt<9>(V, 64 * Eps<double>::v * scale)) flags[e] = 1;
-}
-
-// Pre-test of the hex projection: H = sum_q w_q B_q^T A_q B_q (w_q > 0) is semi-definite when
-// every quadrature point's tangent A_q = dP/dF is, and then H is its own projection. One thread
-// per (element, point) forms
-//   A(3 i + j, 3 k + l) = mu d_ik d_jl + lambda G_ij G_kl - p G_il G_kj,  G = F^-T, p = lambda log J - mu
-// (bitwise symmetric: each product is formed from the same two factors both ways) and runs the
-// LDL^T test with the tet pass's round-off allowance; an element with a point that fails is
-// marked in flags (zeroed before) for the eigen-projection. A failed point (det F <= 0 or
-// non-finite) marks its element too; the element pass reports it.
-__global__ void __launch_bounds__(128) hex_tangent_test_kernel(const DevMesh m, const double* __restrict__ u,
-                                                               int* __restrict__ flags) {
-    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= static_cast<size_t>(m.T) * m.nq) return;
-    const int e = static_cast<int>(t / m.nq), q = static_cast<int>(t - static_cast<size_t>(m.nq) * e);
-    const int32_t* cell = m.hex_cells + 8 * static_cast<size_t>(e);
-    const double lam = m.hex_theta[2 * static_cast<size_t>(e)], mu = m.hex_theta[2 * static_cast<size_t>(e) + 1];
-    const double* dq = m.hex_q + 25 * static_cast<size_t>(q);
-    double Ji[9], dJ;
-    hex_point_geometry(m, cell, dq, Ji, dJ);
-    double G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int c = 0; c < 8; ++c) {
-        const int v = __ldg(cell + c);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double uu = __ldg(u + 3 * static_cast<size_t>(v) + i);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) G[3 * i + d] = fma(uu, __ldg(dq + 3 * c + d), G[3 * i + d]);
-        }
-    }
-    double F[9];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            F[3 * i + j] = (i == j ? 1.0 : 0.0) + G[3 * i] * Ji[j] + G[3 * i + 1] * Ji[3 + j] + G[3 * i + 2] * Ji[6 + j];
-    double C[9];
-    C[0] = F[4] * F[8] - F[5] * F[7];
-    C[1] = F[5] * F[6] - F[3] * F[8];
-    C[2] = F[3] * F[7] - F[4] * F[6];
-    C[3] = F[2] * F[7] - F[1] * F[8];
-    C[4] = F[0] * F[8] - F[2] * F[6];
-    C[5] = F[1] * F[6] - F[0] * F[7];
-    C[6] = F[1] * F[5] - F[2] * F[4];
-    C[7] = F[2] * F[3] - F[0] * F[5];
-    C[8] = F[0] * F[4] - F[1] * F[3];
-    const double detF = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
-    if (!(detF > 0) || !isfinite(detF)) {
-        flags[e] = 1;
-        return;
-    }
-    double Gt[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Gt[k] = C[k] / detF;
-    const double p = lam * log(detF) - mu;
-    double A[81];
-    double scale = 0;
-#pragma unroll
-    for (int r = 0; r < 9; ++r)
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            const int i = r / 3, j = r % 3, k = c / 3, l = c % 3;
-            double v = lam * (Gt[r] * Gt[c]) - p * (Gt[3 * i + l] * Gt[3 * k + j]);
-            if (r == c) {
-                v += mu;
-                scale = fmax(scale, fabs(v));
-            }
-            A[9 * r + c] = v;
-        }
-    if (!(scale < INFINITY) || !semidefinite_ldlt<9>(A, 64 * Eps<double>::v * scale)) flags[e] = 1;
-}
-
-// Projected Hessian of hex meshes (HessianKind::Projected, mesh_energy.cpp:16-27): one warp per
-// element loads its record of 36 FP64 blocks (hex_element_kernel) as the 24x24 element Hessian
-// into shared memory, runs the parallel-ordered Jacobi iteration (lpg_psd.h) and writes
-// V max(L, 0) V^T back as 36 blocks in the precision's type: in place for FP64 (a warp reads its
-// whole record before it writes), into a separate FP32 record array for mixed precision. Each
-// entry is formed once from the upper triangle, so the diagonal blocks stay bitwise symmetric.
+// Projected Hessian of hex meshes (HessianKind::Projected, mesh_energy.cpp:16-27): one warp per element
+// loads its record of 36 FP64 blocks (hex_element_kernel) as the 24 x 24 element Hessian, projects it
+// (WarpEig) and writes the result as 36 blocks in the precision's type: in place for FP64 (a lane writes
+// the entries it read), into a separate FP32 record array for mixed precision. Each entry is formed from
+// its upper-triangle position, so the diagonal blocks stay bitwise symmetric. An element without an
+// eigenvalue below -8 eps |H| is kept as it is.
+// Bound by the FP64 pipe (about 8,500 warp instructions per element) and by the latency of its chains at 16
+// warps per SM.
+// 7,480 hexes, every one indefinite: 214 us (a cyclic Jacobi iteration in shared memory took 1,664 us, and a
+// per-point semi-definiteness test before it 53 us).
 struct WarpTeam {
     int l;
     __device__ int lane() const { return l; }
@@ -2579,50 +2530,98 @@ struct WarpTeam {
 };
 
 constexpr int kHexPsdWarps = 4;
+using HexEig = WarpEig<24>;
 
 template <typename R>
-__global__ void __launch_bounds__(32 * kHexPsdWarps) hex_psd_kernel(int T, const double* in, R* out,
-                                                                   const int* __restrict__ flags, unsigned* status) {
-    using J = PsdJacobi<24>;
-    __shared__ double sA[kHexPsdWarps][24 * J::S], sV[kHexPsdWarps][24 * J::S];
-    __shared__ double sCS[kHexPsdWarps][J::kCs], sL[kHexPsdWarps][24];
-    __shared__ int sPQ[kHexPsdWarps][24];
+__global__ void __launch_bounds__(32 * kHexPsdWarps, 4) hex_psd_kernel(int T, const double* in, R* out,
+                                                                      unsigned* status) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ unsigned short s_at[kHexRecord]; // record entry -> row << 8 | column of its upper entry
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    HexEig& W = reinterpret_cast<HexEig*>(smem_raw)[w];
+    for (int t = threadIdx.x; t < kHexRecord; t += blockDim.x) {
+        int a, b;
+        hex_pair(t / 9, a, b);
+        const int i = 3 * a + (t % 9) / 3, k = 3 * b + t % 3;
+        s_at[t] = static_cast<unsigned short>(min(i, k) << 8 | max(i, k));
+    }
+    __syncthreads();
     const int e = blockIdx.x * kHexPsdWarps + w; // uniform over the warp: a warp leaves whole
     if (e >= T) return;
     const double* rec = in + kHexRecord * static_cast<size_t>(e);
     R* o = out + kHexRecord * static_cast<size_t>(e);
-    if (flags[e] == 0) { // semi-definite (hex_tangent_test_kernel): the Hessian as it is
-        if (static_cast<const void*>(rec) != static_cast<const void*>(o))
-            for (int t = lane; t < kHexRecord; t += 32) o[t] = static_cast<R>(rec[t]);
-        return;
+    constexpr int S = HexEig::S;
+    constexpr int kPer = (kHexRecord + 31) / 32;
+    double h[kPer], amax = 0;
+    bool finite = true;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int t = lane + 32 * q;
+        h[q] = t < kHexRecord ? rec[t] : 0.0;
+        amax = fmax(amax, fabs(h[q]));
+        finite = finite && isfinite(h[q]);
     }
-    double* A = sA[w];
-    for (int t = lane; t < kHexRecord; t += 32) {
-        int a, b;
-        hex_pair(t / 9, a, b);
-        const int i = 3 * a + (t % 9) / 3, k = 3 * b + t % 3;
-        const double v = rec[t];
-        A[i * J::S + k] = v;
-        if (a != b) A[k * J::S + i] = v;
-    }
-    J::eigen(WarpTeam{lane}, A, sV[w], sCS[w], sPQ[w], sL[w]);
-    unsigned st = 0;
-    for (int t = lane; t < kHexRecord; t += 32) {
-        int a, b;
-        hex_pair(t / 9, a, b);
-        int i = 3 * a + (t % 9) / 3, k = 3 * b + t % 3;
-        if (i > k) {
-            const int x = i;
-            i = k;
-            k = x;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    finite = __all_sync(0xffffffffu, finite);
+    int kind = 0;
+    double up = 1.0;
+    if (finite && amax > 0.0) {
+        // Exact power-of-two scaling to max |entry| in [0.5, 1).
+        int ex;
+        frexp(amax, &ex);
+        const double down = ldexp(1.0, -ex);
+        up = ldexp(1.0, ex);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int t = lane + 32 * q;
+            if (t < kHexRecord) {
+                const int i = s_at[t] >> 8, k = s_at[t] & 0xff;
+                W.M[i * S + k] = W.M[k * S + i] = down * h[q];
+            }
         }
-        const double v = J::entry(sV[w], sL[w], i, k);
-        if (!isfinite(v)) st |= ST_NONFINITE_OUT;
-        o[t] = static_cast<R>(v);
+        __syncwarp();
+        kind = W.project(lane);
+        if (kind < 0) {
+            using J = PsdJacobi<24>;
+            static_assert(J::S == S, "one row stride");
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) {
+                const int t = lane + 32 * q;
+                if (t < kHexRecord) {
+                    const int i = s_at[t] >> 8, k = s_at[t] & 0xff;
+                    W.M[i * S + k] = W.M[k * S + i] = down * rec[t];
+                }
+            }
+            J::eigen(WarpTeam{lane}, W.M, W.V, W.d, reinterpret_cast<int*>(W.e), W.e2);
+            for (int t = lane; t < kHexRecord; t += 32) {
+                const int i = s_at[t] >> 8, k = s_at[t] & 0xff;
+                W.M[i * S + k] = J::entry(W.V, W.e2, i, k);
+            }
+            __syncwarp();
+            kind = 2;
+        }
+    }
+    unsigned st = finite ? 0u : static_cast<unsigned>(ST_NONFINITE_OUT);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int t = lane + 32 * q;
+        if (t < kHexRecord) {
+            const double p = kind == 0 ? 0.0 : up * W.M[(s_at[t] >> 8) * S + (s_at[t] & 0xff)];
+            const double v = kind == 2 ? p : rec[t] + p;
+            if (!isfinite(v)) st |= ST_NONFINITE_OUT;
+            o[t] = static_cast<R>(v);
+        }
     }
     st = __reduce_or_sync(0xffffffffu, st);
     if (lane == 0 && st) atomicOr(status, st);
+}
+// Each element's FP64 record projected into out's records (which may be the same memory).
+template <typename R> void launch_hex_psd(const DevMesh& m, const double* in, R* out, unsigned* status, cudaStream_t s) {
+    const size_t sm = kHexPsdWarps * sizeof(HexEig);
+    thread_local LaunchCache cache;
+    resident_grid(hex_psd_kernel<R>, 32 * kHexPsdWarps, sm, cache);
+    hex_psd_kernel<R><<<(m.T + kHexPsdWarps - 1) / kHexPsdWarps, 32 * kHexPsdWarps, sm, s>>>(m.T, in, out, status);
 }
 
 // Feasible step of a hex mesh: at every quadrature point F and dF (the increment's gradient),
@@ -2716,132 +2715,122 @@ __device__ __forceinline__ void hermite_G(const double* tq, int b, const double 
     for (int d = 0; d < 3; ++d) G[d] = sb * __ldg(tq + 3 * b + d) / h[d];
 }
 
-__device__ __forceinline__ void hermite_pair(int pr, int& a, int& b) {
-    a = 0;
-    int base = 0;
-    while (pr >= base + (64 - a)) {
-        base += 64 - a;
-        ++a;
-    }
-    b = a + (pr - base);
+// Three blocks per element (thirds of the block pairs), 192 threads. Per block: the element's 192 DOFs, and
+// each point's w lambda, w p, w mu, F^-T and w P in shared memory (four threads per point); then, eight
+// points at a time, every node's G and h = F^-T G, and one thread per pair of node pairs (2 x 2 blocks
+// H_ab, a <= b, in registers) accumulates them; diagonal blocks are mirrored so the matrix is bitwise
+// symmetric. The first block also writes the energy (points in order) and the gradient. FP64-bound
+// (28 operations per block and point; a thread's four nodes serve four blocks).
+// 80 elements at 64 points: 1,056 us (one 128-thread block per element, the nodes' gradients and
+// kinematics formed per block pair) -> 114 us.
+constexpr int kHermTiles = 32 * 33 / 2;          // 2 x 2 tiles of node pairs
+constexpr int kHermParts = 3;                    // blocks per element
+constexpr int kHermThreads = 192;
+constexpr int kHermChunk = 8;                    // points kept at a time
+constexpr int kHermPoint = 22;                   // w lambda, w p, w mu, w psi, F^-T (9), w P (9)
+static_assert(kHermThreads * kHermParts >= kHermTiles, "one thread per tile");
+
+// Tile t of the 32 x 32 upper triangle of node pairs: row tr, column tc >= tr.
+__device__ __forceinline__ void herm_tile(int t, int& tr, int& tc) {
+    tr = static_cast<int>((65.0f - sqrtf(65.0f * 65.0f - 8.0f * static_cast<float>(t))) * 0.5f);
+    while (tr > 0 && t < tr * 32 - tr * (tr - 1) / 2) --tr;
+    while (t >= (tr + 1) * 32 - (tr + 1) * tr / 2) ++tr;
+    tc = tr + t - (tr * 32 - tr * (tr - 1) / 2);
 }
 
-// One CTA per element: the element's 192 DOFs and each point's w, p, F^-T and P in shared
-// memory (points by thread), then the energy (thread 0, points in order), the gradient (a thread
-// per node) and the 2080 blocks H_ab, a <= b (strided over the CTA; diagonal blocks mirrored so
-// the matrix is bitwise symmetric).
-constexpr int kHermiteThreads = 128;
-
-// With flags (projected Hessian), flags[e] is set when the tangent d2W/dF2 of some point is not
-// positive semi-definite (the element's Hessian then needs the eigenvalue clamp), and cleared
-// otherwise: a sum of w B^T A B with semi-definite A is semi-definite.
 template <typename R>
-__global__ void __launch_bounds__(kHermiteThreads) hermite_element_kernel(const DevMesh m, const double* __restrict__ u,
+__global__ void __launch_bounds__(kHermThreads, 2) hermite_element_kernel(const DevMesh m, const double* __restrict__ u,
                                                                           double* __restrict__ elemE,
                                                                           double* __restrict__ per_elem,
-                                                                          R* __restrict__ blocks, unsigned* status,
-                                                                          int* __restrict__ flags = nullptr) {
-    __shared__ int sFlag;
+                                                                          R* __restrict__ blocks, unsigned* status) {
     __shared__ double sD[192];
-    __shared__ double sK[64 * 20]; // per point: w, p, F^-T (9), P (9)
-    __shared__ double sE[64];
-    __shared__ int sOk[64];
-    const int e = blockIdx.x, tid = threadIdx.x;
+    __shared__ double sK[64 * kHermPoint];
+    __shared__ double sN[kHermChunk * 64 * 6]; // G, h per node
+    const int e = blockIdx.x / kHermParts, third = blockIdx.x - kHermParts * e, tid = threadIdx.x;
     unsigned st = 0;
     const int32_t* cell = m.hex_cells + 8 * static_cast<size_t>(e);
     const double lam = m.hex_theta[2 * static_cast<size_t>(e)], mu = m.hex_theta[2 * static_cast<size_t>(e) + 1];
     if (!(lam >= 0 && mu > 0 && isfinite(lam) && isfinite(mu))) st |= ST_BAD_THETA;
     const double h[3] = {m.herm_h[3 * static_cast<size_t>(e)], m.herm_h[3 * static_cast<size_t>(e) + 1],
                          m.herm_h[3 * static_cast<size_t>(e) + 2]};
-    for (int t = tid; t < 192; t += blockDim.x) {
+    for (int t = tid; t < 192; t += kHermThreads) {
         const double d = __ldg(u + 24 * static_cast<size_t>(__ldg(cell + t / 24)) + t % 24);
         if (!isfinite(d)) st |= ST_BAD_INPUT;
         sD[t] = d;
     }
-    if (tid == 0) sFlag = 0;
     __syncthreads();
-    for (int q = tid; q < m.nq; q += blockDim.x) {
-        const double* tq = m.herm_q + kHermiteTable * static_cast<size_t>(q);
+    for (int t4 = tid; t4 < 4 * 64; t4 += kHermThreads) { // whole warps; four neighbouring lanes per point
+        const int q = t4 >> 2, part = t4 & 3;
         double Gu[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        for (int b = 0; b < 64; ++b) {
-            double G[3];
-            hermite_G(tq, b, h, G);
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int d = 0; d < 3; ++d) Gu[3 * i + d] = fma(sD[3 * b + i], G[d], Gu[3 * i + d]);
-        }
-        double F[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) F[k] = Gu[k] + (k % 4 == 0 ? 1.0 : 0.0);
-        double C[9];
-        C[0] = F[4] * F[8] - F[5] * F[7];
-        C[1] = F[5] * F[6] - F[3] * F[8];
-        C[2] = F[3] * F[7] - F[4] * F[6];
-        C[3] = F[2] * F[7] - F[1] * F[8];
-        C[4] = F[0] * F[8] - F[2] * F[6];
-        C[5] = F[1] * F[6] - F[0] * F[7];
-        C[6] = F[1] * F[5] - F[2] * F[4];
-        C[7] = F[2] * F[3] - F[0] * F[5];
-        C[8] = F[0] * F[4] - F[1] * F[3];
-        const double detF = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
-        double* k = sK + 20 * q;
-        if (!(detF > 0) || !isfinite(detF)) {
-            st |= isfinite(detF) ? ST_BAD_DET : ST_NONFINITE_F;
-            sOk[q] = 0;
-            sE[q] = 0;
-            continue;
-        }
-        sOk[q] = 1;
-        const double L = log(detF), p = lam * L - mu, w = __ldg(tq + 192) * h[0] * h[1] * h[2];
-        k[0] = w;
-        k[1] = p;
-        if (flags) {
-            // The point's tangent A[(3i+j)(3k+l)] = mu d_ik d_jl + lambda H_ij H_kl - p H_il H_kj (H = F^-T).
-            double Gt[9], A[81], scale = 0;
-#pragma unroll
-            for (int t = 0; t < 9; ++t) Gt[t] = C[t] / detF;
-            for (int r = 0; r < 9; ++r)
-                for (int c = 0; c < 9; ++c) {
-                    const int i = r / 3, j = r % 3, kk = c / 3, l = c % 3;
-                    double v = lam * (Gt[r] * Gt[c]) - p * (Gt[3 * i + l] * Gt[3 * kk + j]);
-                    if (r == c) {
-                        v += mu;
-                        scale = fmax(scale, fabs(v));
-                    }
-                    A[9 * r + c] = v;
-                }
-            if (!(scale < INFINITY) || !semidefinite_ldlt<9>(A, 64 * Eps<double>::v * scale)) sFlag = 1;
-        }
-        double ff = 0;
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            const double fit = C[t] / detF;
-            k[2 + t] = fit;
-            k[11 + t] = mu * F[t] + p * fit;
-            ff += F[t] * F[t];
-        }
-        sE[q] = w * (0.5 * mu * (ff - 3.0) - mu * L + 0.5 * lam * L * L);
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double E = 0;
-        for (int q = 0; q < m.nq; ++q) E += sE[q];
-        if (!isfinite(E)) st |= ST_NONFINITE_OUT;
-        elemE[e] = E;
-        if (flags) flags[e] = sFlag;
-    }
-    if (per_elem) {
-        for (int b = tid; b < 64; b += blockDim.x) {
-            double ga[3] = {0, 0, 0};
-            for (int q = 0; q < m.nq; ++q) {
-                if (!sOk[q]) continue;
+        const double* tq = m.herm_q + kHermiteTable * static_cast<size_t>(min(q, m.nq - 1));
+        if (q < m.nq)
+#pragma unroll 4
+            for (int b = part; b < 64; b += 4) {
                 double G[3];
-                hermite_G(m.herm_q + kHermiteTable * static_cast<size_t>(q), b, h, G);
-                const double* k = sK + 20 * q;
+                hermite_G(tq, b, h, G);
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
-                    ga[i] = fma(k[0], k[11 + 3 * i] * G[0] + k[12 + 3 * i] * G[1] + k[13 + 3 * i] * G[2], ga[i]);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) Gu[3 * i + d] = fma(sD[3 * b + i], G[d], Gu[3 * i + d]);
+            }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            Gu[k] += __shfl_xor_sync(0xffffffffu, Gu[k], 1);
+            Gu[k] += __shfl_xor_sync(0xffffffffu, Gu[k], 2);
+        }
+        if (q < m.nq && part == 0) {
+            double F[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) F[k] = Gu[k] + (k % 4 == 0 ? 1.0 : 0.0);
+            double C[9];
+            C[0] = F[4] * F[8] - F[5] * F[7];
+            C[1] = F[5] * F[6] - F[3] * F[8];
+            C[2] = F[3] * F[7] - F[4] * F[6];
+            C[3] = F[2] * F[7] - F[1] * F[8];
+            C[4] = F[0] * F[8] - F[2] * F[6];
+            C[5] = F[1] * F[6] - F[0] * F[7];
+            C[6] = F[1] * F[5] - F[2] * F[4];
+            C[7] = F[2] * F[3] - F[0] * F[5];
+            C[8] = F[0] * F[4] - F[1] * F[3];
+            const double detF = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
+            double* k = sK + kHermPoint * q;
+            if (!(detF > 0) || !isfinite(detF)) {
+                st |= isfinite(detF) ? ST_BAD_DET : ST_NONFINITE_F;
+                for (int t = 0; t < kHermPoint; ++t) k[t] = 0.0; // contributes nothing
+            } else {
+                const double L = log(detF), p = lam * L - mu, w = __ldg(tq + 192) * h[0] * h[1] * h[2];
+                double ff = 0;
+#pragma unroll
+                for (int t = 0; t < 9; ++t) {
+                    const double fit = C[t] / detF;
+                    k[4 + t] = fit;
+                    k[13 + t] = w * (mu * F[t] + p * fit);
+                    ff += F[t] * F[t];
+                }
+                k[0] = w * lam;
+                k[1] = w * p;
+                k[2] = w * mu;
+                k[3] = w * (0.5 * mu * (ff - 3.0) - mu * L + 0.5 * lam * L * L);
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && third == 0) {
+        double E = 0;
+        for (int q = 0; q < m.nq; ++q) E += sK[kHermPoint * q + 3];
+        if (!isfinite(E)) st |= ST_NONFINITE_OUT;
+        elemE[e] = E;
+    }
+    if (per_elem && third == 0) {
+        for (int b = tid; b < 64; b += kHermThreads) {
+            double ga[3] = {0, 0, 0};
+#pragma unroll 4
+            for (int q = 0; q < m.nq; ++q) {
+                double G[3];
+                hermite_G(m.herm_q + kHermiteTable * static_cast<size_t>(q), b, h, G);
+                const double* k = sK + kHermPoint * q + 13;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) ga[i] += k[3 * i] * G[0] + k[3 * i + 1] * G[1] + k[3 * i + 2] * G[2];
             }
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -2851,328 +2840,191 @@ __global__ void __launch_bounds__(kHermiteThreads) hermite_element_kernel(const 
         }
     }
     if (blocks) {
-        for (int pr = tid; pr < 2080; pr += blockDim.x) {
-            int a, b;
-            hermite_pair(pr, a, b);
-            double Hb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            for (int q = 0; q < m.nq; ++q) {
-                if (!sOk[q]) continue;
-                const double* tq = m.herm_q + kHermiteTable * static_cast<size_t>(q);
-                double Ga[3], Gb[3];
-                hermite_G(tq, a, h, Ga);
-                hermite_G(tq, b, h, Gb);
-                const double* k = sK + 20 * q;
-                const double w = k[0], p = k[1];
-                double ha[3], hb[3];
+        const int tile = third * kHermThreads + tid;
+        int tr = 0, tc = 0;
+        if (tile < kHermTiles) herm_tile(tile, tr, tc);
+        double acc[2][2][9];
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                for (int t = 0; t < 9; ++t) acc[x][y][t] = 0;
+        for (int q0 = 0; q0 < m.nq; q0 += kHermChunk) {
+            const int nq = min(kHermChunk, m.nq - q0);
+            __syncthreads(); // the previous points' nodes are read
+            for (int t = tid; t < 64 * nq; t += kHermThreads) {
+                const int q = t >> 6, b = t & 63;
+                double G[3];
+                hermite_G(m.herm_q + kHermiteTable * static_cast<size_t>(q0 + q), b, h, G);
+                const double* k = sK + kHermPoint * (q0 + q) + 4;
+                double* o = sN + 6 * t;
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    ha[i] = k[2 + 3 * i] * Ga[0] + k[3 + 3 * i] * Ga[1] + k[4 + 3 * i] * Ga[2];
-                    hb[i] = k[2 + 3 * i] * Gb[0] + k[3 + 3 * i] * Gb[1] + k[4 + 3 * i] * Gb[2];
-                }
-                const double dn = Ga[0] * Gb[0] + Ga[1] * Gb[1] + Ga[2] * Gb[2];
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        double v = lam * ha[i] * hb[c] - p * hb[i] * ha[c];
-                        if (i == c) v += mu * dn;
-                        Hb[3 * i + c] = fma(w, v, Hb[3 * i + c]);
-                    }
-            }
-            if (a == b) {
-                Hb[3] = Hb[1];
-                Hb[6] = Hb[2];
-                Hb[7] = Hb[5];
-            }
-            R* o = blocks + kHermiteRecord * static_cast<size_t>(e) + 9 * pr;
-#pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                if (!isfinite(Hb[t])) st |= ST_NONFINITE_OUT;
-                o[t] = static_cast<R>(Hb[t]);
-            }
-        }
-    }
-    st = __reduce_or_sync(0xffffffffu, st);
-    if ((tid & 31) == 0 && st) atomicOr(status, st);
-}
-
-
-// ---------------------------------------------------------------------------
-// Projected Hessian of tricubic Hermite hexes: V max(L, 0) V^T of each flagged element's 192 x 192
-// Hessian (mesh_energy.cpp:16-27, there Eigen's SelfAdjointEigenSolver). One CTA per element:
-// the lower triangle, packed, in shared memory is reduced to tridiagonal form by Householder
-// reflections (Golub & Van Loan, Matrix Computations, 8.3.1), the reflections are accumulated
-// into Q (column-major, in the CTA's global scratch), and the implicit QL iteration with
-// Wilkinson shifts (Golub & Van Loan 8.3.3, in the form of the EISPACK tql2 routine) diagonalises
-// the tridiagonal matrix, one thread generating each sweep's plane rotations and every thread
-// applying them to its row of Q. The projection is then H - sum_{L_m < 0} L_m v_m v_m^T (or the
-// sum over the positive eigenpairs when they are fewer), written back as the element's blocks.
-// ---------------------------------------------------------------------------
-constexpr int kHermN = 192;
-constexpr int kHermPacked = kHermN * (kHermN + 1) / 2;
-constexpr int kHermPsdThreads = 256;
-constexpr int kHermQlSweeps = 60; // per eigenvalue, far above the few the iteration takes
-constexpr size_t kHermPsdSmem = sizeof(double) * (kHermPacked + 6 * kHermN + 32);
-
-__device__ __forceinline__ int hpk(int r, int c) { return r * (r + 1) / 2 + c; } // r >= c
-__device__ __forceinline__ double hsym(const double* Ap, int r, int c) { return r >= c ? Ap[hpk(r, c)] : Ap[hpk(c, r)]; }
-
-// Block-wide sum (every thread receives it); red holds 32 doubles.
-__device__ __forceinline__ double herm_sum(double v, double* red) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = 0;
-    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += red[w];
-    __syncthreads();
-    return t;
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kHermPsdThreads) hermite_psd_kernel(int T, double* in, R* out,
-                                                                      const int* __restrict__ flags,
-                                                                      double* __restrict__ qbuf, unsigned* status) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* Ap = reinterpret_cast<double*>(smem_raw); // packed lower triangle
-    double* d = Ap + kHermPacked;                     // diagonal, then eigenvalues
-    double* ev = d + kHermN;                          // off-diagonal
-    double* beta = ev + kHermN;                       // reflector coefficients
-    double* vp = beta + kHermN;                       // p, then w, of the current reflection
-    double* rc = vp + kHermN;                         // a sweep's rotations: c, s (2 per index)
-    double* red = rc + 2 * kHermN;
-    __shared__ int s_hi, s_count, s_bad;
-    const int tid = threadIdx.x, bd = blockDim.x;
-    constexpr int n = kHermN;
-    double* Q = qbuf + static_cast<size_t>(blockIdx.x) * n * n; // Q(r, c) at c n + r
-    unsigned st = 0;
-    for (int e = blockIdx.x; e < T; e += gridDim.x) {
-        const double* rec = in + kHermiteRecord * static_cast<size_t>(e);
-        R* o = out + kHermiteRecord * static_cast<size_t>(e);
-        if (!flags[e]) { // semi-definite at every point: its own projection
-            if (static_cast<const void*>(o) != static_cast<const void*>(rec))
-                for (int t = tid; t < kHermiteRecord; t += bd) o[t] = static_cast<R>(rec[t]);
-            continue;
-        }
-        // The element matrix: block (a, b), a <= b, entry (i, c) is H(3a + i, 3b + c).
-        for (int t = tid; t < kHermiteRecord; t += bd) {
-            const int pr = t / 9, ic = t - 9 * (t / 9);
-            int a, b;
-            hermite_pair(pr, a, b);
-            const int r = 3 * a + ic / 3, c = 3 * b + ic % 3;
-            if (r >= c) Ap[hpk(r, c)] = rec[t];
-            else if (a != b) Ap[hpk(c, r)] = rec[t];
-        }
-        __syncthreads();
-        // Householder tridiagonalisation: column k's reflection P = I - beta v v^T maps
-        // A[k+1:, k] to (alpha, 0, ...); v is kept in place of the column below the subdiagonal.
-        for (int k = 0; k < n - 2; ++k) {
-            const int m = n - k - 1;
-            double x2 = 0;
-            for (int j = tid + 1; j < m; j += bd) {
-                const double x = Ap[hpk(k + 1 + j, k)];
-                x2 = fma(x, x, x2);
-            }
-            x2 = herm_sum(x2, red);
-            const double x0 = Ap[hpk(k + 1, k)];
-            if (x2 == 0.0) { // already tridiagonal in this column
-                if (tid == 0) {
-                    beta[k] = 0.0;
-                    ev[k] = x0;
-                }
-                __syncthreads();
-                continue;
-            }
-            const double alpha = -copysign(sqrt(fma(x0, x0, x2)), x0);
-            const double v0 = x0 - alpha, bk = 1.0 / (alpha * (alpha - x0)); // 2 / v^T v
-            __syncthreads();
-            if (tid == 0) {
-                Ap[hpk(k + 1, k)] = v0;
-                beta[k] = bk;
-                ev[k] = alpha;
-            }
-            __syncthreads();
-            // p = beta A22 v (row i of the trailing block), then K = beta / 2 p^T v, w = p - K v.
-            double pv = 0;
-            for (int i = tid; i < m; i += bd) {
-                double acc = 0;
-                for (int j = 0; j < m; ++j) acc = fma(hsym(Ap, k + 1 + i, k + 1 + j), Ap[hpk(k + 1 + j, k)], acc);
-                const double p = bk * acc;
-                vp[i] = p;
-                pv = fma(p, Ap[hpk(k + 1 + i, k)], pv);
-            }
-            const double K = 0.5 * bk * herm_sum(pv, red);
-            for (int i = tid; i < m; i += bd) vp[i] = fma(-K, Ap[hpk(k + 1 + i, k)], vp[i]);
-            __syncthreads();
-            // A22 -= v w^T + w v^T on the lower triangle (rows paired for balance).
-            for (int t = tid; t < m; t += bd) {
-                const int i = t;
-                const double vi = Ap[hpk(k + 1 + i, k)], wi = vp[i];
-                for (int j = 0; j <= i; ++j) {
-                    const double vj = Ap[hpk(k + 1 + j, k)], wj = vp[j];
-                    Ap[hpk(k + 1 + i, k + 1 + j)] -= fma(vi, wj, wi * vj);
+                    o[i] = G[i];
+                    o[3 + i] = k[3 * i] * G[0] + k[3 * i + 1] * G[1] + k[3 * i + 2] * G[2];
                 }
             }
             __syncthreads();
-        }
-        for (int i = tid; i < n; i += bd) d[i] = Ap[hpk(i, i)];
-        if (tid == 0) {
-            ev[n - 2] = Ap[hpk(n - 1, n - 2)];
-            beta[n - 2] = 0.0;
-            ev[n - 1] = 0.0;
-        }
-        // Q = P_0 P_1 ... P_{n-3}, accumulated from the last reflection (Q = I to begin with).
-        for (int t = tid; t < n * n; t += bd) Q[t] = (t % n == t / n) ? 1.0 : 0.0;
-        __syncthreads();
-        for (int k = n - 3; k >= 0; --k) {
-            const double bk = beta[k];
-            if (bk == 0.0) continue;
-            const int m = n - k - 1;
-            // Columns c of Q with c > k: Q[k+1:, c] -= bk v (v^T Q[k+1:, c]); a warp per column.
-            const int warp = tid >> 5, lane = tid & 31;
-            for (int c = k + 1 + warp; c < n; c += bd >> 5) {
-                double* qc = Q + static_cast<size_t>(c) * n + k + 1;
-                double acc = 0;
-                for (int j = lane; j < m; j += 32) acc = fma(Ap[hpk(k + 1 + j, k)], qc[j], acc);
+            if (tile < kHermTiles)
+#pragma unroll 1
+                for (int q = 0; q < nq; ++q) {
+                    const double* k = sK + kHermPoint * (q0 + q);
+                    const double wl = k[0], wp = k[1], wm = k[2];
+                    const double* na = sN + 6 * (64 * q + 2 * tr);
+                    const double* nb = sN + 6 * (64 * q + 2 * tc);
+                    double Gb[2][3], hb[2][3];
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-                const double f = bk * acc;
-                for (int j = lane; j < m; j += 32) qc[j] = fma(-f, Ap[hpk(k + 1 + j, k)], qc[j]);
-            }
-            __syncthreads();
-        }
-        // Implicit QL with Wilkinson shifts on (d, ev); rotations applied to the rows of Q. An
-        // off-diagonal entry is negligible below eps times the tridiagonal matrix's norm bound
-        // max |d_i| + |e_i| (as tql2 tests): the element's rigid-body modes are exact zero
-        // eigenvalues, next to which a test relative to the neighbouring diagonal entries alone
-        // never deflates.
-        if (tid == 0) s_bad = 0;
-        __syncthreads();
-        double tnorm = 0.0;
-        if (tid == 0)
-            for (int i = 0; i < n; ++i) tnorm = fmax(tnorm, fabs(d[i]) + fabs(ev[i]));
-        for (int l = 0; l < n; ++l) {
-            for (int iter = 0;; ++iter) {
-                if (tid == 0) {
-                    int m = l;
-                    for (; m < n - 1; ++m)
-                        if (fabs(ev[m]) <= 2.220446049250313e-16 * tnorm) break;
-                    s_hi = m;
-                    s_count = 0;
-                    if (m != l) {
-                        if (iter >= kHermQlSweeps) {
-                            s_bad = 1;
-                            s_hi = l;
-                        } else {
-                            double g = (d[l + 1] - d[l]) / (2.0 * ev[l]);
-                            double r = hypot(g, 1.0);
-                            g = d[m] - d[l] + ev[l] / (g + copysign(r, g));
-                            double sn = 1.0, cs = 1.0, p = 0.0;
-                            int i = m - 1;
-                            bool split = false;
-                            for (; i >= l; --i) {
-                                const double f = sn * ev[i], b = cs * ev[i];
-                                r = hypot(f, g);
-                                ev[i + 1] = r;
-                                if (r == 0.0) {
-                                    d[i + 1] -= p;
-                                    ev[m] = 0.0;
-                                    split = true;
-                                    break;
-                                }
-                                sn = f / r;
-                                cs = g / r;
-                                g = d[i + 1] - p;
-                                r = (d[i] - g) * sn + 2.0 * cs * b;
-                                p = sn * r;
-                                d[i + 1] = g + p;
-                                g = cs * r - b;
-                                rc[2 * i] = cs;
-                                rc[2 * i + 1] = sn;
-                                ++s_count;
-                            }
-                            if (!split) {
-                                d[l] -= p;
-                                ev[l] = g;
-                                ev[m] = 0.0;
+                    for (int y = 0; y < 2; ++y)
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) Gb[y][i] = nb[6 * y + i], hb[y][i] = nb[6 * y + 3 + i];
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        double la[3], pa[3], ga[3];
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            ga[i] = wm * na[6 * x + i];
+                            la[i] = wl * na[6 * x + 3 + i];
+                            pa[i] = -wp * na[6 * x + 3 + i];
+                        }
+#pragma unroll
+                        for (int y = 0; y < 2; ++y) {
+                            const double dn = ga[0] * Gb[y][0] + ga[1] * Gb[y][1] + ga[2] * Gb[y][2];
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) {
+#pragma unroll
+                                for (int c = 0; c < 3; ++c)
+                                    acc[x][y][3 * i + c] = fma(la[i], hb[y][c], fma(hb[y][i], pa[c], acc[x][y][3 * i + c]));
+                                acc[x][y][4 * i] += dn;
                             }
                         }
                     }
                 }
-                __syncthreads();
-                const int m = s_hi, cnt = s_count;
-                // Every thread holds the sweep's bounds before thread 0 may write the next ones
-                // (after a converged l it goes straight on to l + 1).
-                __syncthreads();
-                if (m == l) break;
-                // Apply rotations i = m-1 .. m-cnt to row r of Q: columns i and i+1.
-                for (int r = tid; r < n; r += bd) {
-                    double hi = Q[static_cast<size_t>(m) * n + r];
-                    for (int i = m - 1; i >= m - cnt; --i) {
-                        const double cs = rc[2 * i], sn = rc[2 * i + 1];
-                        const double lo = Q[static_cast<size_t>(i) * n + r];
-                        Q[static_cast<size_t>(i + 1) * n + r] = fma(sn, lo, cs * hi);
-                        hi = fma(cs, lo, -sn * hi);
+        }
+        if (tile < kHermTiles) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    const int a = 2 * tr + x, b = 2 * tc + y;
+                    if (b < a) continue;
+                    double(&H)[9] = acc[x][y];
+                    if (a == b) {
+                        H[3] = H[1];
+                        H[6] = H[2];
+                        H[7] = H[5];
                     }
-                    Q[static_cast<size_t>(m - cnt) * n + r] = hi;
+                    R* o = blocks + kHermiteRecord * static_cast<size_t>(e) + 9 * CellBlocks<64>::pair(a, b);
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) {
+                        if (!isfinite(H[t])) st |= ST_NONFINITE_OUT;
+                        o[t] = static_cast<R>(H[t]);
+                    }
                 }
-                __syncthreads();
-            }
         }
-        if (s_bad) st |= ST_NONFINITE_OUT;
-        // Reconstruction from the fewer of the negative and positive eigenpairs, staged in the
-        // (now free) shared matrix 96 vectors at a time.
-        int nneg = 0;
-        for (int i = 0; i < n; ++i) nneg += d[i] < 0.0;
-        const bool from_neg = nneg <= n / 2;
-        constexpr int kStage = 96;
-        // Each thread keeps its entries' partial sums in the FP64 record itself (`in` is scratch:
-        // it is read and rewritten by the same thread, entry by entry).
-        double* acc_rec = in + kHermiteRecord * static_cast<size_t>(e);
-        for (int base = 0; base < n; base += kStage) {
-            // Stage eigenvectors base .. base + kStage - 1 that take part, scaled by their eigenvalue.
-            __syncthreads();
-            for (int t = tid; t < kStage * n; t += bd) {
-                const int mm = base + t / n, r = t % n;
-                double v = 0.0;
-                if (mm < n) {
-                    const double lm = d[mm];
-                    const bool use = from_neg ? lm < 0.0 : lm > 0.0;
-                    v = use ? Q[static_cast<size_t>(mm) * n + r] : 0.0;
-                }
-                Ap[t] = v;
-            }
-            __syncthreads();
-            for (int t = tid; t < kHermiteRecord; t += bd) {
-                const int pr = t / 9, ic = t - 9 * (t / 9);
-                int a, b;
-                hermite_pair(pr, a, b);
-                int r = 3 * a + ic / 3, c = 3 * b + ic % 3;
-                if (a == b && r > c) { // diagonal blocks: the lower entry mirrors the upper one
-                    const int tmp = r;
-                    r = c;
-                    c = tmp;
-                }
-                double sum = 0.0;
-                for (int k2 = 0; k2 < kStage && base + k2 < n; ++k2)
-                    sum = fma(d[base + k2] * Ap[k2 * n + r], Ap[k2 * n + c], sum);
-                // The element pass stores diagonal blocks bitwise symmetric, so entry t itself holds
-                // the mirrored value.
-                const double prev = base == 0 ? (from_neg ? acc_rec[t] : 0.0) : acc_rec[t];
-                acc_rec[t] = from_neg ? prev - sum : prev + sum;
-            }
-        }
-        __syncthreads();
-        for (int t = tid; t < kHermiteRecord; t += bd) {
-            const double v = acc_rec[t];
-            if (!isfinite(v)) st |= ST_NONFINITE_OUT;
-            o[t] = static_cast<R>(v);
-        }
-        __syncthreads();
     }
     st = __reduce_or_sync(0xffffffffu, st);
     if ((tid & 31) == 0 && st) atomicOr(status, st);
+}
+
+// ---------------------------------------------------------------------------
+// Projected Hessian of tricubic Hermite hexes: V max(L, 0) V^T of each element's 192 x 192 Hessian
+// (mesh_energy.cpp:16-27, there Eigen's SelfAdjointEigenSolver), one block per element (BlockEig). The
+// record in `in` (FP64) is replaced by, or written in the precision's type to, `out`.
+// Bound by the chains of the tridiagonalisation (190 steps of five barriers), of the Sturm counts and of
+// the inverse iterations: one element per SM. 80 elements at
+// 64 points: 23.7 ms (tridiagonalisation and a QL iteration whose rotations one thread generated) -> 1.28 ms.
+// ---------------------------------------------------------------------------
+template <typename R>
+__global__ void __launch_bounds__(BlockEig::kThreads) hermite_psd_kernel(int T, const double* in, R* out,
+                                                                        double* __restrict__ scratch, unsigned* status) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BlockEig& B = *reinterpret_cast<BlockEig*>(smem_raw);
+    __shared__ double s_max[BlockEig::kWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double* mine = scratch + BlockEig::kScratch * blockIdx.x;
+    unsigned st = 0;
+    for (int e = blockIdx.x; e < T; e += gridDim.x) {
+        const double* rec = in + kHermiteRecord * static_cast<size_t>(e);
+        R* o = out + kHermiteRecord * static_cast<size_t>(e);
+        double amax = 0; // infinite where an entry is not finite
+        for (int t = tid; t < kHermiteRecord; t += BlockEig::kThreads) {
+            const double v = fabs(rec[t]);
+            amax = v < INFINITY ? fmax(amax, v) : INFINITY;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+        if (lane == 0) s_max[warp] = amax;
+        __syncthreads();
+        amax = s_max[0];
+        for (int q = 1; q < BlockEig::kWarps; ++q) amax = fmax(amax, s_max[q]);
+        int kind = 0, k = 0;
+        double up = 1.0;
+        if (amax > 0.0 && amax < INFINITY) {
+            // Exact power-of-two scaling to max |entry| in [0.5, 1).
+            int ex;
+            frexp(amax, &ex);
+            const double down = ldexp(1.0, -ex);
+            up = ldexp(1.0, ex);
+            // Block (a, b), a <= b, entry (i, c) is H(3 a + i, 3 b + c): the blocks of a are consecutive.
+            for (int a = warp; a < 64; a += BlockEig::kWarps) {
+                const double* ra = rec + 9 * (a * 64 - a * (a - 1) / 2);
+                for (int t = lane; t < 9 * (64 - a); t += 32) {
+                    const int b = a + t / 9, ic = t - 9 * (t / 9), r = 3 * a + ic / 3, c = 3 * b + ic % 3;
+                    if (c >= r) B.A[BlockEig::at(c, r)] = down * ra[t];
+                }
+            }
+            __syncthreads();
+            k = B.project(mine, kind);
+        }
+        if (kind < 0 || !(amax < INFINITY)) st |= ST_NONFINITE_OUT;
+        if (kind <= 0) {
+            if (static_cast<const void*>(o) != static_cast<const void*>(rec))
+                for (int t = tid; t < kHermiteRecord; t += BlockEig::kThreads) o[t] = static_cast<R>(rec[t]);
+        } else {
+            // H+ = [H +] sum_c z_c z_c^T, a 2 x 2 tile of node pairs per thread.
+            for (int t = tid; t < kHermTiles; t += BlockEig::kThreads) {
+                int tr, tc;
+                herm_tile(t, tr, tc);
+                double acc[6][6];
+#pragma unroll
+                for (int i = 0; i < 6; ++i)
+#pragma unroll
+                    for (int j = 0; j < 6; ++j) acc[i][j] = 0;
+#pragma unroll 1
+                for (int c = 0; c < k; ++c) {
+                    const double* z = B.A + BlockEig::kStride * c;
+                    double zr[6], zc[6];
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) zr[i] = z[6 * tr + i], zc[i] = z[6 * tc + i];
+#pragma unroll
+                    for (int i = 0; i < 6; ++i)
+#pragma unroll
+                        for (int j = 0; j < 6; ++j) acc[i][j] = fma(zr[i], zc[j], acc[i][j]);
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) {
+                        const int a = 2 * tr + x, b = 2 * tc + y;
+                        if (b < a) continue;
+                        const size_t at = 9 * static_cast<size_t>(CellBlocks<64>::pair(a, b));
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                const double p = up * acc[3 * x + i][3 * y + c];
+                                const double v = kind == 1 ? rec[at + 3 * i + c] + p : p;
+                                if (!isfinite(v)) st |= ST_NONFINITE_OUT;
+                                o[at + 3 * i + c] = static_cast<R>(v);
+                            }
+                    }
+            }
+        }
+        __syncthreads(); // the next element reuses the shared memory
+    }
+    st = __reduce_or_sync(0xffffffffu, st);
+    if (lane == 0 && st) atomicOr(status, st);
 }
 
 // Force-response parameter VJP of Hermite hexes (the hex pass's, over the 64 nodes): per element
@@ -3531,7 +3383,7 @@ void launch_hex_deformation_gradients(const DevMesh& m, const double* u, double*
 }
 
 void launch_hex_material_eval(const DevMesh& m, int precision, int hessian, const double* W, const double* P,
-                              const double* A, double* elemE, double* per_elem, void* blocks, int* flags,
+                              const double* A, double* elemE, double* per_elem, void* blocks,
                               const EvalArgs& a, cudaStream_t s) {
     const bool projected = hessian == LPG_HESSIAN_PROJECTED;
     if (m.T > 0) {
@@ -3541,15 +3393,11 @@ void launch_hex_material_eval(const DevMesh& m, int precision, int hessian, cons
         if (a.hess && projected) {
             double* records = static_cast<double*>(blocks);
             hex_material_kernel<double><<<grid, 128, 0, s>>>(m, W, P, A, elemE, per_grad, records, a.status);
-            LPG_CUDA(cudaMemsetAsync(flags, 0, static_cast<size_t>(m.T) * sizeof(int), s));
-            const size_t points = static_cast<size_t>(m.T) * m.nq;
-            hex_material_tangent_test_kernel<<<static_cast<int>((points + 127) / 128), 128, 0, s>>>(m, A, flags);
-            const int pgrid = (m.T + kHexPsdWarps - 1) / kHexPsdWarps;
             if (precision == LPG_PRECISION_F64) {
-                hex_psd_kernel<double><<<pgrid, 32 * kHexPsdWarps, 0, s>>>(m.T, records, records, flags, a.status);
+                launch_hex_psd<double>(m, records, records, a.status, s);
             } else {
                 float* out = reinterpret_cast<float*>(records + kHexRecord * static_cast<size_t>(m.T));
-                hex_psd_kernel<float><<<pgrid, 32 * kHexPsdWarps, 0, s>>>(m.T, records, out, flags, a.status);
+                launch_hex_psd<float>(m, records, out, a.status, s);
                 blocks = out;
             }
         } else if (precision == LPG_PRECISION_F64 || !a.hess) {
@@ -3581,43 +3429,45 @@ size_t hermite_blocks_bytes(const DevMesh& m, int precision, bool projected) {
     return records * (projected ? sizeof(double) + sizeof(float) : sizeof(float));
 }
 
+namespace {
 int hermite_psd_grid(const DevMesh& m) {
     int dev = 0, sms = 0;
     LPG_CUDA(cudaGetDevice(&dev));
     LPG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     return std::max(1, std::min(m.T, sms));
 }
+template <typename R>
+void launch_hermite_psd(const DevMesh& m, const double* in, R* out, double* scratch, unsigned* status, cudaStream_t s) {
+    thread_local LaunchCache cache;
+    resident_grid(hermite_psd_kernel<R>, BlockEig::kThreads, sizeof(BlockEig), cache);
+    hermite_psd_kernel<R><<<hermite_psd_grid(m), BlockEig::kThreads, sizeof(BlockEig), s>>>(m.T, in, out, scratch, status);
+}
+} // namespace
+
+size_t hermite_scratch_doubles(const DevMesh& m) { return BlockEig::kScratch * static_cast<size_t>(hermite_psd_grid(m)); }
 
 void launch_hermite_eval(const DevMesh& m, int precision, bool projected, const double* u, double* elemE,
-                         double* per_elem, void* blocks, int* flags, double* qbuf, const EvalArgs& a, cudaStream_t s) {
+                         double* per_elem, void* blocks, double* scratch, const EvalArgs& a, cudaStream_t s) {
     if (m.T > 0) {
         if (a.ev_begin) LPG_CUDA(cudaEventRecord(a.ev_begin, s));
         double* per_grad = a.grad ? per_elem : nullptr;
         if (a.hess && projected) {
-            // FP64 element Hessians with the per-point pre-test, then the clamp of the flagged
-            // elements into the precision's records.
+            // FP64 element Hessians, projected into the precision's records.
             double* records = static_cast<double*>(blocks);
-            hermite_element_kernel<double><<<m.T, kHermiteThreads, 0, s>>>(m, u, elemE, per_grad, records, a.status,
-                                                                            flags);
-            const int grid = hermite_psd_grid(m);
+            hermite_element_kernel<double><<<kHermParts * m.T, kHermThreads, 0, s>>>(m, u, elemE, per_grad, records,
+                                                                                     a.status);
             if (precision == LPG_PRECISION_F64) {
-                thread_local LaunchCache cache;
-                resident_grid(hermite_psd_kernel<double>, kHermPsdThreads, kHermPsdSmem, cache);
-                hermite_psd_kernel<double><<<grid, kHermPsdThreads, kHermPsdSmem, s>>>(m.T, records, records, flags,
-                                                                                      qbuf, a.status);
+                launch_hermite_psd<double>(m, records, records, scratch, a.status, s);
             } else {
                 float* out = reinterpret_cast<float*>(records + kHermiteRecord * static_cast<size_t>(m.T));
-                thread_local LaunchCache cache;
-                resident_grid(hermite_psd_kernel<float>, kHermPsdThreads, kHermPsdSmem, cache);
-                hermite_psd_kernel<float><<<grid, kHermPsdThreads, kHermPsdSmem, s>>>(m.T, records, out, flags, qbuf,
-                                                                                     a.status);
+                launch_hermite_psd<float>(m, records, out, scratch, a.status, s);
                 blocks = out;
             }
         } else if (precision == LPG_PRECISION_F64 || !a.hess)
-            hermite_element_kernel<double><<<m.T, kHermiteThreads, 0, s>>>(
+            hermite_element_kernel<double><<<kHermParts * m.T, kHermThreads, 0, s>>>(
                 m, u, elemE, per_grad, a.hess ? static_cast<double*>(blocks) : nullptr, a.status);
         else
-            hermite_element_kernel<float><<<m.T, kHermiteThreads, 0, s>>>(m, u, elemE, per_grad,
+            hermite_element_kernel<float><<<kHermParts * m.T, kHermThreads, 0, s>>>(m, u, elemE, per_grad,
                                                                           static_cast<float*>(blocks), a.status);
         if (a.grad) vertex_gather_kernel<64><<<std::min(m.ncl, 148 * 8), 128, 0, s>>>(m, per_elem, 1.0, a.grad);
         if (a.hess) {
@@ -3643,32 +3493,27 @@ size_t hex_blocks_bytes(const DevMesh& m, int precision, bool projected) {
 }
 
 void launch_hex_eval(const DevMesh& m, int precision, bool projected, const double* u, double* elemE,
-                     double* per_elem, void* blocks, int* flags, const EvalArgs& a, cudaStream_t s) {
+                     double* per_elem, void* blocks, const EvalArgs& a, cudaStream_t s) {
     if (m.T > 0) {
-        const size_t threads = 36 * static_cast<size_t>(m.T);
-        const int grid = static_cast<int>((threads + 127) / 128);
+        const int grid = (m.T + kHexEl - 1) / kHexEl;
         if (a.ev_begin) LPG_CUDA(cudaEventRecord(a.ev_begin, s));
         double* per_grad = a.grad ? per_elem : nullptr;
         if (a.hess && projected) {
             // FP64 element Hessians, projected into the precision's records.
             double* records = static_cast<double*>(blocks);
-            hex_element_kernel<double><<<grid, 128, 0, s>>>(m, u, elemE, per_grad, records, a.status);
-            LPG_CUDA(cudaMemsetAsync(flags, 0, static_cast<size_t>(m.T) * sizeof(int), s));
-            const size_t points = static_cast<size_t>(m.T) * m.nq;
-            hex_tangent_test_kernel<<<static_cast<int>((points + 127) / 128), 128, 0, s>>>(m, u, flags);
-            const int pgrid = (m.T + kHexPsdWarps - 1) / kHexPsdWarps;
+            hex_element_kernel<double><<<grid, kHexThreads, 0, s>>>(m, u, elemE, per_grad, records, a.status);
             if (precision == LPG_PRECISION_F64) {
-                hex_psd_kernel<double><<<pgrid, 32 * kHexPsdWarps, 0, s>>>(m.T, records, records, flags, a.status);
+                launch_hex_psd<double>(m, records, records, a.status, s);
             } else {
                 float* out = reinterpret_cast<float*>(records + kHexRecord * static_cast<size_t>(m.T));
-                hex_psd_kernel<float><<<pgrid, 32 * kHexPsdWarps, 0, s>>>(m.T, records, out, flags, a.status);
+                launch_hex_psd<float>(m, records, out, a.status, s);
                 blocks = out;
             }
         } else if (precision == LPG_PRECISION_F64) {
-            hex_element_kernel<double><<<grid, 128, 0, s>>>(m, u, elemE, per_grad,
+            hex_element_kernel<double><<<grid, kHexThreads, 0, s>>>(m, u, elemE, per_grad,
                                                            a.hess ? static_cast<double*>(blocks) : nullptr, a.status);
         } else {
-            hex_element_kernel<float><<<grid, 128, 0, s>>>(m, u, elemE, per_grad,
+            hex_element_kernel<float><<<grid, kHexThreads, 0, s>>>(m, u, elemE, per_grad,
                                                           a.hess ? static_cast<float*>(blocks) : nullptr, a.status);
         }
         if (a.grad) vertex_gather_kernel<8><<<std::min(m.ncl, 148 * 8), 128, 0, s>>>(m, per_elem, 1.0, a.grad);
