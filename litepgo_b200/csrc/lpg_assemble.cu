@@ -90,10 +90,10 @@ template <typename R> struct Kin {
 };
 
 // Returns status bits. u is FP64; edge differences are formed in FP64 and rounded once.
-// FP64: det F and log det F as the reference computes them (neo_hookean.cpp:14-23). FP32:
-// det F - 1 from the invariants of the displacement gradient and log1p, which keeps log J
-// accurate near the rest state. Validity is checked once on J; the rare failure path then
-// tells a non-finite input from a non-finite F and from det F <= 0.
+// FP64: det F as the reference computes it (neo_hookean.cpp:14-23), log det F and |F|^2 - 3 with the
+// digits that the displacement gradient still has. FP32: det F - 1 from its invariants and log1p.
+// Validity is checked once on J; the rare failure path then tells a non-finite input from a non-finite F
+// and from det F <= 0.
 template <typename R>
 __device__ __forceinline__ unsigned kinematics_of(const DevMesh& m, int e, const R (&rec)[12], const double (&uu)[4][3],
                                                   Kin<R>& k);
@@ -186,28 +186,39 @@ __device__ __forceinline__ unsigned kinematics_ds(const DevMesh& m, int e, const
     C[6] = F[1] * F[5] - F[2] * F[4];
     C[7] = F[2] * F[3] - F[0] * F[5];
     C[8] = F[0] * F[4] - F[1] * F[3];
-    R J, sqm3;
-    if (sizeof(R) == 8 || fpi != nullptr) {
-        J = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
-        k.logJ = X::log_(J);
-        R ff = 0;
-#pragma unroll
-        for (int t = 0; t < 9; ++t) ff = X::fma(F[t], F[t], ff);
-        sqm3 = ff - R(3);
-    } else {
+    // det F - 1 and |F|^2 - 3 from the displacement gradient's invariants, which keep W's digits near the
+    // rest state (its terms of order mu cancel to order mu strain^2); with a plastic field F alone is known.
+    R J, sqm3, Jm1 = 0;
+    const bool small = fpi == nullptr;
+    if (small) {
         const R c1 = H[0] + H[4] + H[8];
         const R c2 = (H[0] * H[4] - H[1] * H[3]) + (H[0] * H[8] - H[2] * H[6]) + (H[4] * H[8] - H[5] * H[7]);
         const R c3 = H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) +
                      H[2] * (H[3] * H[7] - H[4] * H[6]);
-        const R Jm1 = c1 + c2 + c3;
-        J = R(1) + Jm1;
-        k.logJ = X::log1p_(Jm1);
+        Jm1 = c1 + c2 + c3;
         R hh = 0;
 #pragma unroll
         for (int t = 0; t < 9; ++t) hh = X::fma(H[t], H[t], hh);
         sqm3 = R(2) * c1 + hh;
+    } else {
+        R ff = 0;
+#pragma unroll
+        for (int t = 0; t < 9; ++t) ff = X::fma(F[t], F[t], ff);
+        sqm3 = ff - R(3);
     }
+    if (sizeof(R) == 8 || !small)
+        J = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
+    else
+        J = R(1) + Jm1;
     const R iJ = R(1) / J;
+    if (sizeof(R) == 8) {
+        // log J of the determinant that is checked, corrected to first order by what rounding F and its
+        // products lost (about 1e-16, worth 1e-16 mu in W); J - 1 is exact where this is used.
+        k.logJ = X::log_(J);
+        if (small && J > R(0.5) && J < R(2)) k.logJ = X::fma(Jm1 - (J - R(1)), iJ, k.logJ);
+    } else {
+        k.logJ = small ? X::log1p_(Jm1) : X::log_(J);
+    }
 #pragma unroll
     for (int t = 0; t < 9; ++t) k.FiT[t] = C[t] * iJ;
     k.psi = R(0.5) * k.mu * sqm3 - k.mu * k.logJ + R(0.5) * k.lam * k.logJ * k.logJ;

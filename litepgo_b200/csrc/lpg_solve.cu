@@ -1183,6 +1183,10 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
         return;
     }
     double gnorm0 = -1;
+    // The line search compares energies of the energy-only pass: the trial's with the one at x (the
+    // accepted trial of the iteration before), so that both carry the same rounding of the same sum.
+    double Ex = 0;
+    bool have_Ex = false;
     bool exact = false; // the exact_below switch, decided on the previous iteration's gradient
     for (int it = 0;; ++it) {
         const int hk = exact ? LPG_HESSIAN_EXACT : o.hessian;
@@ -1301,6 +1305,8 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
         }
         step.feasible_step = alpha;
         bool accepted = false;
+        if (!have_Ex) Ex = S.energy(x, f, nullptr);
+        have_Ex = true;
         for (int j = 0; j < o.max_line_search_steps; ++j) {
             LPG_CUDA(cudaMemsetAsync(moved, 0, sizeof(int), s));
             axpy_trial<<<grid(n), kThreads, 0, s>>>(x, alpha, d, trial, n, moved);
@@ -1311,10 +1317,11 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
             ++R.line_search_evaluations;
             ++step.line_search_evaluations;
             const double Et = S.energy(trial, f, nullptr);
-            const double noise = 16.0 * kEps * std::max(1.0, std::abs(E));
+            const double noise = 16.0 * kEps * std::max(1.0, std::abs(Ex));
             const double armijo = o.accept_rule == 1 ? 1e-4 * alpha * gd : 0.0;
-            if (Et <= E + armijo + noise) {
+            if (Et <= Ex + armijo + noise) {
                 accepted = true;
+                Ex = Et;
                 break;
             }
             alpha *= o.line_search_shrink;
@@ -2102,7 +2109,7 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
     double* al = h.d_alpha.as<double>(1);
     // Per-mesh state on the host.
     std::vector<int> status(M, -1), act(M, 1), iters(M, 0), take(M, 0), pending(M, 0);
-    std::vector<double> E(M, 0), g2(M, 0), gmax(M, 0), g0(M, -1), secs(M, 0), alpha(M, 0), gd(M, 0);
+    std::vector<double> Ex(M, 0), E(M, 0), g2(M, 0), gmax(M, 0), g0(M, -1), secs(M, 0), alpha(M, 0), gd(M, 0);
     {
         std::vector<double> mh;
         B.down(mh, mask, n);
@@ -2210,6 +2217,8 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
             pending[m] = act[m];
             alpha[m] = act[m] ? amin[m] : 0.0;
         }
+        // As in newton_solve, the trial energies are compared with the energy-only pass's at x.
+        if (it == 0) Ex = B.energies(x, f, nullptr, LPG_HESSIAN_NONE, LPG_PRECISION_F64, nullptr);
         for (int j = 0; j < o.max_line_search_steps; ++j) {
             if (std::none_of(pending.begin(), pending.end(), [](int v) { return v != 0; })) break;
             std::vector<double> a(M);
@@ -2229,11 +2238,12 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
             for (int m = 0; m < M; ++m) {
                 take[m] = 0;
                 if (!pending[m]) continue;
-                const double noise = 16.0 * kEps * std::max(1.0, std::abs(E[m]));
+                const double noise = 16.0 * kEps * std::max(1.0, std::abs(Ex[m]));
                 const double armijo = o.accept_rule == 1 ? 1e-4 * alpha[m] * gd[m] : 0.0;
-                if (Et[m] <= E[m] + armijo + noise) {
+                if (Et[m] <= Ex[m] + armijo + noise) {
                     take[m] = 1;
                     pending[m] = 0;
+                    Ex[m] = Et[m];
                 } else {
                     alpha[m] *= o.line_search_shrink;
                 }
