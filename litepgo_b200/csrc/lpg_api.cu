@@ -216,7 +216,7 @@ lpg_fem::~lpg_fem() {
 
 void lpg_fem::create_result() {
     LPG_CUDA(cudaMemset(d_result.as<EvalResult>(1), 0, sizeof(EvalResult)));
-    LPG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host_result), sizeof(EvalResult), cudaHostAllocDefault));
+    LPG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host_result), 4096, cudaHostAllocDefault));
 }
 
 void lpg_fem::sync() { LPG_CUDA(cudaStreamSynchronize(stream)); }

@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(1024) stats_final(const double* __restrict__ p
 struct PcgState {
     double rz, pAp, alpha, beta, rr, bb, tol2;
     int done, breakdown, iters, max_iters;
+    int lost; // the one-launch PCG gave up waiting for another block
     unsigned count_a, count_b; // completion counters of the last-block reductions
 };
 
@@ -601,6 +602,12 @@ __global__ void __launch_bounds__(kThreads) pcg_update(PcgState* st, const R* __
     }
 }
 
+} // namespace
+} // namespace lpg
+#include "lpg_pcg.cuh"
+namespace lpg {
+namespace {
+
 template <typename A, typename B> __global__ void convert_kernel(const A* __restrict__ a, B* __restrict__ b, size_t n) {
     const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (i < n) b[i] = static_cast<B>(a[i]);
@@ -796,8 +803,9 @@ struct Solver {
         stats_final<<<1, 1024, 0, s>>>(part, nb, out);
         LPG_CUDA(cudaGetLastError());
         std::array<double, 4> r{};
-        LPG_CUDA(cudaMemcpyAsync(r.data(), out, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
+        LPG_CUDA(cudaMemcpyAsync(h.host_sums(), out, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
         LPG_CUDA(cudaStreamSynchronize(s));
+        std::copy(h.host_sums(), h.host_sums() + 4, r.begin());
         return r;
     }
 
@@ -907,6 +915,75 @@ struct Solver {
         }
     }
 
+    // The plan of the one-launch PCG; false where this mesh does not use it in precision R: its chunks
+    // exceed one per warp of one block per SM (a row's state then no longer fits a lane), or a block's z
+    // its shared memory. Below that line it is the faster one at every size measured: whole Newton solves,
+    // graph then one launch, 4^3 cubes FP64 32 and 15 ms, 30^3 FP64 200 and 105, 36^3 FP64 (50,653 vertices,
+    // most values read from L2 each iteration) 261 and 171, 40x40x36 mixed 167 and 93.
+    template <typename R> bool one_launch(PcgPlan& plan) {
+        const DevMesh& m = h.dm;
+        if (h.pcg_plan_state == 0) {
+            h.pcg_plan_state = -1;
+            int sms = 0, optin = 0, coop = 0;
+            LPG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h.device));
+            LPG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h.device));
+            LPG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h.device));
+            sms = std::min(sms, kPcgMaxBlocks);
+            if (coop && m.n_sell > 0 && m.n_sell <= kPcgWarps * sms) {
+                const int per = (m.n_sell + sms - 1) / sms, blocks = (m.n_sell + per - 1) / per;
+                const size_t bits = 2 * sizeof(unsigned) * ((static_cast<size_t>(V) + 31) / 32);
+                int32_t* count = h.pl_count.as<int32_t>(static_cast<size_t>(blocks));
+                pcg_plan_kernel<<<blocks, kPcgThreads, bits, s>>>(m, blocks, nullptr, 0, count, nullptr, nullptr);
+                std::vector<int32_t> n(static_cast<size_t>(blocks));
+                LPG_CUDA(cudaMemcpyAsync(n.data(), count, n.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+                LPG_CUDA(cudaStreamSynchronize(s));
+                const int most = *std::max_element(n.begin(), n.end());
+                const auto fits = [&](size_t halo) { return kPcgFixed + halo <= static_cast<size_t>(optin); };
+                if (most < 65536 && fits(pcg_halo_bytes<float>(most))) {
+                    h.pcg_plan_state = fits(pcg_halo_bytes<double>(most)) ? 2 : 1;
+                    h.pcg_plan_blocks = blocks;
+                    h.pcg_plan_stride = most;
+                    pcg_plan_kernel<<<blocks, kPcgThreads, bits, s>>>(
+                        m, blocks, h.pl_halo.as<int32_t>(static_cast<size_t>(blocks) * most), most, count,
+                        h.pl_own.as<uint16_t>(std::max<size_t>(h.plan.sell_col.size(), 1)),
+                        h.pl_bor.as<uint16_t>(std::max<size_t>(h.plan.sell_bref.size() / 2, 1)));
+                    // The exchange's words and number, and z's words. Nothing else writes them, so what
+                    // is left in one from before carries an older number than any that is waited for.
+                    LPG_CUDA(cudaMemsetAsync(h.pl_words.as<unsigned char>(words_bytes()), 0, words_bytes(), s));
+                    LPG_CUDA(cudaMemsetAsync(h.pl_z.as<double>(4 * static_cast<size_t>(V)), 0,
+                                             4 * sizeof(double) * static_cast<size_t>(V), s));
+                }
+                LPG_CUDA(cudaGetLastError());
+            }
+        }
+        if (h.pcg_plan_state < (sizeof(R) == 8 ? 2 : 1)) return false;
+        plan.blocks = h.pcg_plan_blocks;
+        plan.halo_stride = h.pcg_plan_stride;
+        plan.halo = static_cast<const int32_t*>(h.pl_halo.ptr);
+        plan.halo_count = static_cast<const int32_t*>(h.pl_count.ptr);
+        plan.idx_own = static_cast<const uint16_t*>(h.pl_own.ptr);
+        plan.idx_bor = static_cast<const uint16_t*>(h.pl_bor.ptr);
+        return true;
+    }
+    static constexpr size_t words_bytes() { return 6 * sizeof(uint4) * kPcgMaxBlocks + 64; }
+    // One PCG solve in one cooperative launch (x4 from b4, state in st).
+    template <typename R>
+    void launch_one(const PcgPlan& plan, const R* K, const R* dinv, const R* mask4, const R* b4, R* x4, PcgState* st,
+                    double tol, int max_iters) {
+        int optin = 0;
+        LPG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h.device));
+        LPG_CUDA(cudaFuncSetAttribute(pcg_solve_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        unsigned char* words = static_cast<unsigned char*>(h.pl_words.ptr);
+        PcgArgs<R> a{K, dinv, mask4, b4, x4, static_cast<R*>(h.pl_z.ptr), st, reinterpret_cast<uint4*>(words),
+                     reinterpret_cast<unsigned*>(words + 6 * sizeof(uint4) * kPcgMaxBlocks), tol, max_iters,
+                     static_cast<size_t>(optin)};
+        DevMesh dm = h.dm;
+        PcgPlan pl = plan;
+        void* args[] = {&dm, &pl, &a};
+        LPG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(pcg_solve_kernel<R>), dim3(plan.blocks),
+                                             dim3(kPcgThreads), args, static_cast<size_t>(optin), s));
+    }
+
     // Solves mask K x = mask b (FP64 b, x): inner PCG in precision R on Kin (values of type R),
     // FP64 residual refinement against Kres (FP64 values when res64, else Kin's values). The
     // iterations run as a replayed CUDA graph of 32 iterations; the host checks the device
@@ -936,6 +1013,8 @@ struct Solver {
         const double bnorm = std::sqrt(stats<double, double>(b64, nullptr, mask)[1]);
         if (bnorm == 0) return out;
         pad_rhs<R><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(mask, mask, mask4, V); // 0/1 values: mask^2 = mask
+        PcgPlan plan;
+        const bool one = one_launch<R>(plan);
         // The graph of 16 iteration pairs, captured on the handle's own stream and cached.
         constexpr int kPairs = 16;
         constexpr int kKey = 12;
@@ -945,7 +1024,7 @@ struct Solver {
         bool same = h.pcg_graph != nullptr;
         for (int i = 0; i < kKey && same; ++i) same = h.pcg_graph_key[i] == key[i];
         cudaStream_t gs = h.own_stream;
-        if (!same) {
+        if (!one && !same) {
             if (h.pcg_graph) {
                 cudaGraphExecDestroy(h.pcg_graph);
                 h.pcg_graph = nullptr;
@@ -964,25 +1043,41 @@ struct Solver {
         for (int ref = 0; ref <= max_refine; ++ref) {
             const double inner_tol = std::min(0.5, std::max(tol * bnorm / rnorm, sizeof(R) == 4 ? 1e-6 : 1e-14));
             pad_rhs<R><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(r64, mask, bR, V);
-            pcg_init<R><<<vg, kThreads, 0, s>>>(bR, dinv, x, r, z, pA, V, part);
-            pcg_start<<<1, 1024, 0, s>>>(st, part, vg, inner_tol, max_iters - static_cast<int>(out.iters));
-            LPG_CUDA(cudaGetLastError());
             PcgState hs{};
-            for (;;) {
-                LPG_CUDA(cudaEventRecord(ev, s));
-                LPG_CUDA(cudaStreamWaitEvent(gs, ev, 0));
-                LPG_CUDA(cudaGraphLaunch(h.pcg_graph, gs));
-                LPG_CUDA(cudaEventRecord(ev, gs));
-                LPG_CUDA(cudaStreamWaitEvent(s, ev, 0));
-                LPG_CUDA(cudaMemcpyAsync(&hs, st, sizeof hs, cudaMemcpyDeviceToHost, s));
+            auto read_state = [&]() {
+                LPG_CUDA(cudaMemcpyAsync(h.host_pcg(), st, sizeof hs, cudaMemcpyDeviceToHost, s));
                 LPG_CUDA(cudaStreamSynchronize(s));
-                if (hs.done) break;
+                std::memcpy(&hs, h.host_pcg(), sizeof hs);
+            };
+            if (one) {
+                launch_one<R>(plan, static_cast<const R*>(Kin), dinv, mask4, bR, x, st, inner_tol,
+                              max_iters - static_cast<int>(out.iters));
+                read_state();
+                if (hs.lost) {
+                    // The blocks' numbers may differ now: start over.
+                    LPG_CUDA(cudaMemsetAsync(h.pl_words.ptr, 0, words_bytes(), s));
+                    LPG_CUDA(cudaMemsetAsync(h.pl_z.ptr, 0, 4 * sizeof(double) * static_cast<size_t>(V), s));
+                    fail(LPG_ECUDA, "PCG: the solve's blocks lost one another");
+                }
+            } else {
+                pcg_init<R><<<vg, kThreads, 0, s>>>(bR, dinv, x, r, z, pA, V, part);
+                pcg_start<<<1, 1024, 0, s>>>(st, part, vg, inner_tol, max_iters - static_cast<int>(out.iters));
+                LPG_CUDA(cudaGetLastError());
+                for (;;) {
+                    LPG_CUDA(cudaEventRecord(ev, s));
+                    LPG_CUDA(cudaStreamWaitEvent(gs, ev, 0));
+                    LPG_CUDA(cudaGraphLaunch(h.pcg_graph, gs));
+                    LPG_CUDA(cudaEventRecord(ev, gs));
+                    LPG_CUDA(cudaStreamWaitEvent(s, ev, 0));
+                    read_state();
+                    if (hs.done) break;
+                }
             }
             out.iters += hs.iters;
             if (hs.breakdown) {
                 out.breakdown = true;
                 // Negative curvature on the first step: keep the preconditioned residual direction.
-                if (hs.iters == 0) LPG_CUDA(cudaMemcpyAsync(x, pB, n4 * sizeof(R), cudaMemcpyDeviceToDevice, s));
+                if (!one && hs.iters == 0) LPG_CUDA(cudaMemcpyAsync(x, pB, n4 * sizeof(R), cudaMemcpyDeviceToDevice, s));
             }
             add_kernel<R><<<grid(n), kThreads, 0, s>>>(x64, x, n);
             residual_spmv(Kres, res64, x64, mask, y64);

@@ -55,6 +55,10 @@ struct lpg_fem {
     // CUDA graph of a chunk of PCG iterations, reused while its pointers stay the same.
     cudaGraphExec_t pcg_graph = nullptr;
     const void* pcg_graph_key[12] = {};
+    // Plan of the one-launch PCG (lpg_pcg.cuh), built at the first solve: 0 not built, 1 usable in FP32
+    // only, 2 in both precisions, -1 not usable for this mesh.
+    int pcg_plan_state = 0, pcg_plan_blocks = 0, pcg_plan_stride = 0;
+    lpg::DeviceBuffer pl_halo, pl_count, pl_own, pl_bor, pl_words, pl_z;
     cudaGraphExec_t batch_graph = nullptr; // the batched (per-mesh) PCG iterations
     const void* batch_graph_key[12] = {};
     // What an evaluation leaves for the host, one 16-byte record on the device (d_result) and its
@@ -65,6 +69,9 @@ struct lpg_fem {
         unsigned done;   // block counter of the energy sum (zero between launches)
     };
     EvalResult* host_result = nullptr;
+    // The rest of the pinned block: landing places of the solvers' read-backs (sums, PCG state).
+    double* host_sums() { return reinterpret_cast<double*>(host_result) + 8; }
+    void* host_pcg() { return reinterpret_cast<double*>(host_result) + 16; }
     EvalResult* result() { return static_cast<EvalResult*>(d_result.ptr); }
     double* energy_word() { return &result()->energy; }
     unsigned* status_word() { return &result()->status; }
