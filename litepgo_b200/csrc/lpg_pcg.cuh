@@ -7,19 +7,23 @@
 // preconditioner block in registers for the whole solve, and a block its chunks' matrix values as far as
 // they fit (both triangles, borrowed blocks transposed once): the first slots of a warp in registers, up to
 // 16 more in shared memory, the rest read from L2. What crosses blocks is z and three sums:
-// - z = D r of the block's rows and their neighbours (the halo) is staged in shared memory. A vertex's z is
-//   one 16-byte word (two in FP64) that carries the iteration's number, so a reader polls the word itself:
-//   no fence, no flag, one L2 round trip.
+// - z = D r of the block's rows goes to shared memory, and to L2 for the blocks that have it as a neighbour
+//   (their halo). A vertex's z is one 16-byte word (two in FP64) that carries the iteration's number, so a
+//   reader polls the word itself: no fence, no flag, one L2 round trip.
 // - CG in the form with one reduction (Chronopoulos and Gear, below): gamma, delta and r.r of a block are
-//   published as numbered words too, and three warps of every block poll all of them and add them in block
+//   published as numbered words too, and 15 warps of every block poll all of them and add them in block
 //   order, so that all blocks hold bitwise the same sums and results do not depend on scheduling.
 // Between the two exchanges every block has read what it waits for, so z is kept once and the sums twice
 // (by the number's parity). An iteration is then two L2 round trips, the products and FP64 latency.
 //
-// Measured per iteration, B200 (launch-per-step, then this kernel): 648 vertices FP64 14.2 and 4.5 us;
-// 4,896 FP64 16.4 and 6.4; 62,197 FP32 15.6 and 9.3, where the products (18 slots a lane) and the wait for
-// the slowest block are half. A build that spilled 300 bytes a thread took 14 at the last: beside 227 KB of
-// shared memory the L1 holds no spills, hence KR, G and the scalars in shared memory below.
+// A batch of meshes is one launch too: every mesh has blocks of its own (one block exchanges nothing), its
+// own sums, tolerance and end, where the launches per step run all meshes in lockstep to the slowest.
+//
+// Measured per iteration, B200 (launch-per-step, then this kernel): 648 vertices FP64 14.2 and 4.2 us;
+// 4,896 FP64 16.4 and 6; 62,197 FP32 15.6 and 8.8, where the products (18 slots a lane) and the wait for
+// the slowest block are half; lockstep of 48 boxes of 4 to 16 cubes a side, 64,000 vertices, 24, and all
+// their solves at once 7.8. A build that spilled 300 bytes a thread took 14 at 62,197: beside 227 KB of
+// shared memory the L1 holds no spills, hence KR, G, the scalars in shared memory and one word per lane.
 #pragma once
 
 namespace lpg {
@@ -29,25 +33,43 @@ constexpr int kPcgThreads = 512, kPcgWarps = kPcgThreads / 32;
 constexpr int kPcgMaxBlocks = 160;     // five slots per polling lane
 constexpr unsigned kPcgSpins = 1u << 22; // polls of one exchange before it gives up (seconds)
 
-// Plan of the launch, built once per handle: per block the vertices whose direction it keeps (its
-// columns, ascending) and every slot's index into that list (indexed as sell_col and sell_bref).
+// One linear system of a launch: a mesh's chunks and vertices (a chunk at a mesh's ends may hold rows of its
+// neighbours, which are passed over) and the blocks that work on it. Groups know nothing of one another.
+struct PcgGroup {
+    int c0, c1, v0, v1; // chunks and vertices
+    int b0, blocks;
+};
+// Plan of the launch. A block keeps z of its own rows (32 per chunk, in the chunks' order), then of the other
+// vertices that are columns of them (its halo, ascending); every slot of the sliced ELL has its column's
+// position in that list (indexed as sell_col and sell_bref).
 struct PcgPlan {
-    int blocks = 0, halo_stride = 0;
+    const PcgGroup* groups = nullptr;
+    const int32_t* of_block = nullptr;   // group of each block
+    int halo_stride = 0, blocks = 0;
     const int32_t* halo = nullptr;       // [blocks][halo_stride]
     const int32_t* halo_count = nullptr; // [blocks]
     const uint16_t* idx_own = nullptr;
     const uint16_t* idx_bor = nullptr;
 };
-__host__ __device__ inline int pcg_first_chunk(int n_sell, int blocks, int b) {
-    return static_cast<int>(static_cast<int64_t>(n_sell) * b / blocks);
+__host__ __device__ inline int pcg_first_chunk(const PcgGroup& g, int rank) {
+    return g.c0 + static_cast<int>(static_cast<int64_t>(g.c1 - g.c0) * rank / g.blocks);
 }
 
-// One block per plan block: marks the columns of its chunks in a bitmap over the vertices, numbers them
-// in ascending order and writes the list (when halo is not null) and the slots' indices.
-__global__ void __launch_bounds__(kPcgThreads) pcg_plan_kernel(const DevMesh m, int blocks, int32_t* halo, int stride,
-                                                               int32_t* count, uint16_t* idx_own, uint16_t* idx_bor) {
+// Position of every vertex in the sliced-ELL row order.
+__global__ void row_position_kernel(const DevMesh m, int32_t* pos) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 32 * m.n_sell && m.sell_row[i] >= 0) pos[m.sell_row[i]] = i;
+}
+
+// One block per block of the plan: marks the other vertices that its rows refer to in a bitmap over the
+// group's vertices, numbers them in ascending order and writes the list (when halo is not null) and the
+// slots' positions.
+__global__ void __launch_bounds__(kPcgThreads)
+    pcg_plan_kernel(const DevMesh m, const PcgGroup* groups, const int32_t* of_block, const int32_t* pos, int32_t* halo,
+                    int stride, int32_t* count, uint16_t* idx_own, uint16_t* idx_bor) {
     extern __shared__ unsigned s_bits[]; // bitmap, then the number of marks before each word
-    const int words = (m.V + 31) / 32;
+    const PcgGroup g = groups[of_block[blockIdx.x]];
+    const int words = (g.v1 - g.v0 + 31) / 32;
     unsigned* before = s_bits + words;
     __shared__ unsigned s_sum[kPcgWarps];
     __shared__ unsigned s_base;
@@ -55,14 +77,20 @@ __global__ void __launch_bounds__(kPcgThreads) pcg_plan_kernel(const DevMesh m, 
     for (int i = tid; i < words; i += kPcgThreads) s_bits[i] = 0;
     if (tid == 0) s_base = 0;
     __syncthreads();
-    const int c0 = pcg_first_chunk(m.n_sell, blocks, blockIdx.x), c1 = pcg_first_chunk(m.n_sell, blocks, blockIdx.x + 1);
-    const int o0 = m.sell_ptr[c0], o1 = m.sell_ptr[c1], b0 = m.sell_bptr[c0], b1 = m.sell_bptr[c1];
-    for (int c = c0 + warp; c < c1; c += kPcgWarps) {
-        const int row = m.sell_row[32 * static_cast<size_t>(c) + lane];
-        if (row >= 0) atomicOr(s_bits + (row >> 5), 1u << (row & 31));
-    }
-    for (int i = o0 + tid; i < o1; i += kPcgThreads) atomicOr(s_bits + (m.sell_col[i] >> 5), 1u << (m.sell_col[i] & 31));
-    for (int i = b0 + tid; i < b1; i += kPcgThreads) atomicOr(s_bits + (m.sell_bref[i].y >> 5), 1u << (m.sell_bref[i].y & 31));
+    const int rank = blockIdx.x - g.b0, c0 = pcg_first_chunk(g, rank), c1 = pcg_first_chunk(g, rank + 1);
+    const int p0 = 32 * c0, p1 = 32 * c1;
+    const auto each_slot = [&](auto&& own, auto&& bor) {
+        for (int c = c0 + warp; c < c1; c += kPcgWarps) {
+            const int row = m.sell_row[32 * static_cast<size_t>(c) + lane];
+            if (row < g.v0 || row >= g.v1) continue;
+            for (int i = m.sell_ptr[c] + lane; i < m.sell_ptr[c + 1]; i += 32) own(i, m.sell_col[i]);
+            for (int i = m.sell_bptr[c] + lane; i < m.sell_bptr[c + 1]; i += 32) bor(i, m.sell_bref[i].y);
+        }
+    };
+    const auto mark = [&](int, int v) {
+        if (pos[v] < p0 || pos[v] >= p1) atomicOr(s_bits + ((v - g.v0) >> 5), 1u << ((v - g.v0) & 31));
+    };
+    each_slot(mark, mark);
     __syncthreads();
     for (int i0 = 0; i0 < words; i0 += kPcgThreads) { // exclusive prefix sums of the words' counts
         const int i = i0 + tid;
@@ -86,13 +114,14 @@ __global__ void __launch_bounds__(kPcgThreads) pcg_plan_kernel(const DevMesh m, 
     if (halo == nullptr) return;
     for (int i = tid; i < words; i += kPcgThreads) {
         unsigned b = s_bits[i], at = before[i];
-        for (; b; b &= b - 1) halo[static_cast<size_t>(stride) * blockIdx.x + at++] = 32 * i + __ffs(b) - 1;
+        for (; b; b &= b - 1) halo[static_cast<size_t>(stride) * blockIdx.x + at++] = g.v0 + 32 * i + __ffs(b) - 1;
     }
-    auto rank = [&](int v) {
-        return static_cast<uint16_t>(before[v >> 5] + __popc(s_bits[v >> 5] & ((1u << (v & 31)) - 1u)));
+    const auto at = [&](int v) {
+        if (pos[v] >= p0 && pos[v] < p1) return static_cast<uint16_t>(pos[v] - p0);
+        const int w = (v - g.v0) >> 5, bit = (v - g.v0) & 31;
+        return static_cast<uint16_t>(p1 - p0 + before[w] + __popc(s_bits[w] & ((1u << bit) - 1u)));
     };
-    for (int i = o0 + tid; i < o1; i += kPcgThreads) idx_own[i] = rank(m.sell_col[i]);
-    for (int i = b0 + tid; i < b1; i += kPcgThreads) idx_bor[i] = rank(m.sell_bref[i].y);
+    each_slot([&](int i, int v) { idx_own[i] = at(v); }, [&](int i, int v) { idx_bor[i] = at(v); });
 }
 
 // 16-byte words that carry their own validity: single 128-bit accesses, so a reader that finds the number
@@ -139,22 +168,26 @@ template <> struct Pending<double> {
 
 // Values per staged vertex: float4 in FP32, three doubles in FP64.
 template <typename R> constexpr int pcg_stride() { return sizeof(R) == 4 ? 4 : 3; }
-// Shared memory of the staged z and its vertex list.
-template <typename R> constexpr size_t pcg_halo_bytes(int n) {
-    return (static_cast<size_t>(n) * (pcg_stride<R>() * sizeof(R) + sizeof(int32_t)) + 15) / 16 * 16;
+// Shared memory of the staged z (own rows and halo) and the halo's vertex list.
+template <typename R> constexpr size_t pcg_z_bytes(int rows, int halo) {
+    return (static_cast<size_t>(rows + halo) * pcg_stride<R>() * sizeof(R) + halo * sizeof(int32_t) + 15) / 16 * 16;
 }
 // Shared memory of one slot of a chunk (32 blocks).
 template <typename R> constexpr size_t pcg_slot_bytes() { return 32 * 9 * sizeof(R); }
-constexpr size_t kPcgFixed = (4 * kPcgWarps + 16 + 3 * 32 * kPcgWarps) * sizeof(double); // sums, split rows' parts
+constexpr size_t kPcgFixed = (4 * kPcgWarps + 26 + 3 * 32 * kPcgWarps) * sizeof(double); // sums, split rows' parts
 
 template <typename R> struct PcgArgs {
     const R *val, *dinv, *mask4, *b4;
     R *x4, *z4;
-    PcgState* st;
-    uint4* words;     // [2][3][blocks]
-    unsigned* number; // exchanges so far (device)
+    PcgState* st;     // per group, zero before the launch
+    uint4* words;     // [2][3][blocks of the plan]
+    unsigned* number; // per group: exchanges so far
+    const double* tols; // per group, or null: tol
+    const int* act;     // per group (0: x = 0 and nothing else), or null
     double tol;
     int max_iters;
+    int first_block;        // the plan's first block of this launch
+    bool first_direction;   // on negative curvature at the first step, x is the preconditioned residual
     size_t smem;
 };
 
@@ -209,29 +242,42 @@ __device__ __forceinline__ double shfl_xor_add(double keep, double send, int o) 
 template <typename R>
 __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh m, const PcgPlan plan, const PcgArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int PS = pcg_stride<R>(), KR = sizeof(R) == 4 ? 2 : 0, G = sizeof(R) == 4 ? 2 : 1;
+    constexpr int PS = pcg_stride<R>(), KR = sizeof(R) == 4 ? 2 : 1, G = sizeof(R) == 4 ? 3 : 1;
     constexpr int MS = 16; // most slots of a warp in shared memory (their column indices are in registers)
-    double* red = reinterpret_cast<double*>(smem_raw); // [4 values][warps], then the three sums
-    double* total = red + 4 * kPcgWarps;
-    volatile int* s_lost = reinterpret_cast<volatile int*>(total + 4);
+    double* red = reinterpret_cast<double*>(smem_raw); // [4 values][warps], then the groups of blocks' sums
+    double* total = red + 4 * kPcgWarps; // [warp]
+    volatile int* s_lost = reinterpret_cast<volatile int*>(total + 16);
     // Scalars of thread 0: 1 / gamma and 1 / alpha of the iteration before (by parity), then its gamma and
     // p.Ap, the squared tolerance and |b|^2.
-    double* scal = total + 8;
-    R* parts = reinterpret_cast<R*>(total + 16); // [warp][3][32]
+    double* scal = total + 18;
+    R* parts = reinterpret_cast<R*>(total + 26); // [warp][3][32]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int blocks = plan.blocks;
-    const int c0 = pcg_first_chunk(m.n_sell, blocks, blockIdx.x), c1 = pcg_first_chunk(m.n_sell, blocks, blockIdx.x + 1);
+    const int block = a.first_block + blockIdx.x, grp = plan.of_block[block];
+    const PcgGroup g = plan.groups[grp];
+    const int blocks = g.blocks, rank = block - g.b0;
+    const int c0 = pcg_first_chunk(g, rank), c1 = pcg_first_chunk(g, rank + 1);
     const int nc = c1 - c0; // at most kPcgWarps
-    const int L = plan.halo_count[blockIdx.x];
+    const auto row_of = [&](int c) { // the lane's row, -1 past the end or in another mesh
+        const int row = m.sell_row[32 * static_cast<size_t>(c) + lane];
+        return row >= g.v0 && row < g.v1 ? row : -1;
+    };
+    if (a.act != nullptr && a.act[grp] == 0) { // the whole group leaves
+        const int row = warp < nc ? row_of(c0 + warp) : -1;
+        if (row >= 0) st4(a.x4 + 4 * static_cast<size_t>(row), R(0), R(0), R(0));
+        return;
+    }
+    const int L = plan.halo_count[block], own_rows = 32 * nc;
     R* zs = reinterpret_cast<R*>(smem_raw + kPcgFixed);
-    int32_t* list = reinterpret_cast<int32_t*>(zs + static_cast<size_t>(PS) * L);
-    unsigned char* rest = smem_raw + kPcgFixed + pcg_halo_bytes<R>(L);
+    int32_t* list = reinterpret_cast<int32_t*>(zs + static_cast<size_t>(PS) * (own_rows + L));
+    unsigned char* rest = smem_raw + kPcgFixed + pcg_z_bytes<R>(own_rows, L);
     // `sub` warps share a chunk (its slots dealt round robin); the first of them owns the rows.
     int sub = 1;
     while (2 * sub * nc <= kPcgWarps && sub < 4) sub *= 2;
     const int ch = warp / sub, part = warp - sub * ch;
     const bool on = ch < nc;
     const int c = c0 + (on ? ch : 0);
+    const int lane_row = row_of(c); // of every warp that shares the chunk
+    unsigned free = lane_row >= 0 ? 8u : 0u; // bit 3: the lane has a row; bit i: its component i is free
     const int s0 = m.sell_ptr[c], w0 = (m.sell_ptr[c + 1] - s0) >> 5;
     const int t0 = m.sell_bptr[c], bw = (m.sell_bptr[c + 1] - t0) >> 5;
     const int ns = on ? w0 + bw : 0;
@@ -241,7 +287,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
     const auto slots_of = [&](int k) {
         return (m.sell_ptr[c0 + k + 1] - m.sell_ptr[c0 + k] + m.sell_bptr[c0 + k + 1] - m.sell_bptr[c0 + k]) >> 5;
     };
-    const size_t room = (a.smem - kPcgFixed - pcg_halo_bytes<R>(L)) / pcg_slot_bytes<R>();
+    const size_t room = (a.smem - kPcgFixed - pcg_z_bytes<R>(own_rows, L)) / pcg_slot_bytes<R>();
     int cap = 0;
     for (int most = 1 << 12; most > 0; most >>= 1) {
         size_t need = 0;
@@ -257,7 +303,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
     const auto load_slot = [&](int q, R k9[9], int& at) {
         const bool own = q < w0;
         const int2 ref = own ? make_int2(9 * s0 + 288 * q + lane, 0) : __ldg(m.sell_bref + t0 + 32 * (q - w0) + lane);
-        at = own ? plan.idx_own[s0 + 32 * q + lane] : plan.idx_bor[t0 + 32 * (q - w0) + lane];
+        at = !(free & 8u) ? 0 : own ? plan.idx_own[s0 + 32 * q + lane]
+                                  : plan.idx_bor[t0 + 32 * (q - w0) + lane];
         R v[9];
 #pragma unroll
         for (int e = 0; e < 9; ++e) v[e] = __ldg(a.val + static_cast<size_t>(ref.x) + 32 * e);
@@ -285,12 +332,11 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
             packed[j / 2] |= static_cast<unsigned>(at) << (16 * (j & 1));
         }
     }
-    for (int i = tid; i < L; i += kPcgThreads) list[i] = plan.halo[static_cast<size_t>(plan.halo_stride) * blockIdx.x + i];
+    for (int i = tid; i < L; i += kPcgThreads) list[i] = plan.halo[static_cast<size_t>(plan.halo_stride) * block + i];
     for (int i = tid; i < 4 * kPcgWarps; i += kPcgThreads) red[i] = 0.0;
     // The row's state.
-    const int row = on && part == 0 ? m.sell_row[32 * static_cast<size_t>(c) + lane] : -1;
+    const int row = on && part == 0 ? lane_row : -1;
     R x[3] = {0, 0, 0}, r[3] = {0, 0, 0}, z[3] = {0, 0, 0}, p[3] = {0, 0, 0}, s[3] = {0, 0, 0}, D[6];
-    unsigned free = 0; // bit i: component i of the row is free
 #pragma unroll
     for (int t = 0; t < 6; ++t) D[t] = R(0);
     if (row >= 0) {
@@ -307,26 +353,30 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
         ld4(a.dinv + 12 * static_cast<size_t>(row) + 8, d);
         D[5] = d[2];
     }
-    unsigned number = __ldcg(a.number);
+    unsigned number = __ldcg(a.number + grp);
     if (tid == 0) *s_lost = 0;
-    if (blockIdx.x == 0 && tid == 0) a.st->lost = 0;
     __syncthreads();
-    int iters = 0, breakdown = 0;
-    bool lost = false;
-    for (;;) {
-        // z = D r, published under this iteration's number.
+    // z = D r, published under the next iteration's number and put to the block's own rows.
+    const auto publish_z = [&]() {
         ++number;
         z[0] = D[0] * r[0] + D[1] * r[1] + D[2] * r[2];
         z[1] = D[1] * r[0] + D[3] * r[1] + D[4] * r[2];
         z[2] = D[2] * r[0] + D[4] * r[1] + D[5] * r[2];
-        if (row >= 0) publish3(a.z4 + 4 * static_cast<size_t>(row), z, number);
+        if (row >= 0 && blocks > 1) publish3(a.z4 + 4 * static_cast<size_t>(row), z, number);
+        if (on && part == 0) sts3(zs + PS * static_cast<size_t>(32 * ch + lane), z);
+    };
+    int iters = 0, breakdown = 0;
+    double rr = 0;
+    bool lost = false;
+    publish_z();
+    for (;;) {
         if (tid == 0) { // off the path between two exchanges: 1 / gamma and 1 / alpha = p.Ap / gamma
             double* next = scal + 2 * (iters & 1);
             const double ig = iters > 0 ? 1.0 / scal[4] : 0.0;
             next[0] = ig;
             next[1] = iters > 0 ? scal[5] * ig : 0.0;
         }
-        // z of the block's rows and their neighbours, waiting for each word; G words are in flight per thread.
+        // z of the halo, waiting for each word; G words are in flight per thread.
         for (int i0 = tid; i0 < L; i0 += G * kPcgThreads) {
             Pending<R> zv[G];
             unsigned missing = 0;
@@ -347,7 +397,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
                         missing &= ~(1u << j);
                         R t[3];
                         zv[j].get(t);
-                        sts3(zs + PS * static_cast<size_t>(i0 + j * kPcgThreads), t);
+                        sts3(zs + PS * static_cast<size_t>(own_rows + i0 + j * kPcgThreads), t);
                     }
             }
         }
@@ -409,54 +459,50 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
             t = shfl_xor_add(t, t, 1);
             if (part == 0 && (lane & 7) == 0) red[kPcgWarps * (lane >> 3) + warp] = t;
             __syncthreads();
-            uint4* all = a.words + static_cast<size_t>(number & 1u) * 3 * blocks;
-            if (warp < 3) { // warp v: the block's value v, then everyone's
-                static_assert(kPcgWarps == 16, "one value per lane below 16");
-                double b = lane < kPcgWarps ? red[kPcgWarps * warp + lane] : 0.0;
+            // Warp v < 3 sums the block's value v and publishes it; then warp v + 3 j polls and adds the values
+            // v of blocks 32 j to 32 j + 31 (one word a lane: five in flight cost the loop 30 registers).
+            const int val = warp % 3, from = 32 * (warp / 3);
+            if (from < blocks && from < kPcgMaxBlocks) {
+                static_assert(kPcgWarps == 16 && kPcgMaxBlocks == 160, "15 warps of 32 words");
+                uint4* all = a.words + static_cast<size_t>(3 * (number & 1u) + val) * plan.blocks + g.b0;
+                double b = 0;
+                if (warp < 3) {
+                    b = lane < kPcgWarps ? red[kPcgWarps * warp + lane] : 0.0;
 #pragma unroll
-                for (int o = 8; o > 0; o >>= 1) b = shfl_xor_add(b, b, o);
-                if (lane == 0) st_word(all + blocks * warp + blockIdx.x, __double2loint(b), __double2hiint(b), 0u, number);
-                constexpr int kPer = kPcgMaxBlocks / 32;
-                double g[kPer];
-                unsigned missing = 0;
-#pragma unroll
-                for (int j = 0; j < kPer; ++j) {
-                    g[j] = 0;
-                    if (lane + 32 * j < blocks) missing |= 1u << j;
+                    for (int o = 8; o > 0; o >>= 1) b = shfl_xor_add(b, b, o);
+                    if (lane == 0 && blocks > 1) st_word(all + rank, __double2loint(b), __double2hiint(b), 0u, number);
                 }
-                for (unsigned spin = 0; missing != 0; ++spin) {
-                    if (spin >= kPcgSpins) {
-                        *s_lost = 1;
-                        break;
-                    }
-                    uint4 u[kPer];
-#pragma unroll
-                    for (int j = 0; j < kPer; ++j)
-                        if ((missing >> j) & 1u) u[j] = ld_word(all + blocks * warp + lane + 32 * j);
-#pragma unroll
-                    for (int j = 0; j < kPer; ++j)
-                        if (((missing >> j) & 1u) && u[j].w == number) {
-                            g[j] = __hiloint2double(u[j].y, u[j].x);
-                            missing &= ~(1u << j);
+                if (blocks > 1) {
+                    b = 0;
+                    if (from + lane < blocks) {
+                        uint4 u = ld_word(all + from + lane);
+                        for (unsigned spin = 0; u.w != number; ++spin) {
+                            if (spin >= kPcgSpins) {
+                                *s_lost = 1;
+                                break;
+                            }
+                            u = ld_word(all + from + lane);
                         }
+                        b = __hiloint2double(u.y, u.x);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) b = shfl_xor_add(b, b, o);
                 }
-                __syncwarp();
-                double sum = 0;
-#pragma unroll
-                for (int j = 0; j < kPer; ++j) sum += g[j];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) sum = shfl_xor_add(sum, sum, o);
-                if (lane == 0) total[warp] = sum;
+                if (lane == 0) total[warp] = b;
             }
             __syncthreads();
             gamma = total[0], delta = total[1];
+            for (int k = 1; 32 * k < blocks; ++k) gamma += total[3 * k], delta += total[3 * k + 1];
             lost = *s_lost != 0;
         }
         if (lost) break;
         {
-            const double rr = total[2];
+            rr = total[2];
+            for (int k = 1; 32 * k < blocks; ++k) rr += total[3 * k + 2];
             if (iters == 0) {
-                if (tid == 0) scal[6] = a.tol * a.tol * rr, scal[7] = rr;
+                const double tol = a.tols != nullptr ? a.tols[grp] : a.tol;
+                if (tid == 0) scal[6] = tol * tol * rr, scal[7] = rr;
                 if (rr == 0.0 || a.max_iters <= 0) break;
             } else if (rr <= scal[6] || iters >= a.max_iters || !isfinite(rr)) {
                 break;
@@ -466,8 +512,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
         const double pAp = fma(-beta * gamma, scal[2 * (iters & 1) + 1], delta);
         if (!(pAp > 0.0) || !isfinite(pAp)) {
             breakdown = 1;
-            // Negative curvature on the first step: the preconditioned residual is the direction.
-            if (iters == 0)
+            if (iters == 0 && a.first_direction)
 #pragma unroll
                 for (int i = 0; i < 3; ++i) x[i] = z[i];
             break;
@@ -476,24 +521,27 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
         const R al = static_cast<R>(alpha), be = static_cast<R>(beta);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            p[i] = z[i] + be * p[i];
             s[i] = y[i] + be * s[i];
-            x[i] += al * p[i];
             r[i] = r[i] - al * s[i];
+            p[i] = z[i] + be * p[i];
         }
+        publish_z();
+#pragma unroll
+        for (int i = 0; i < 3; ++i) x[i] += al * p[i]; // while the words travel
         ++iters;
         if (tid == 0) scal[4] = gamma, scal[5] = pAp;
     }
     if (row >= 0) st4(a.x4 + 4 * static_cast<size_t>(row), x[0], x[1], x[2]);
-    if (blockIdx.x == 0 && tid == 0) {
-        a.st->rr = total[2];
-        a.st->bb = scal[7];
-        a.st->iters = iters;
-        a.st->breakdown = breakdown;
-        a.st->done = 1;
-        *a.number = number;
+    if (rank == 0 && tid == 0) {
+        PcgState* st = a.st + grp;
+        st->rr = rr;
+        st->bb = scal[7];
+        st->iters = iters;
+        st->breakdown = breakdown;
+        st->done = 1;
+        a.number[grp] = number;
     }
-    if (lost && tid == 0) a.st->lost = 1;
+    if (lost && tid == 0) a.st[grp].lost = 1;
 }
 
 } // namespace

@@ -23,6 +23,13 @@ struct DeviceBuffer {
 
 void raise_status(unsigned st);
 
+struct PcgPlanStore {
+    int state = 0; // 0 not built, 1 usable in FP32 only, 2 in both precisions, -1 not usable
+    int groups = 0, blocks = 0, stride = 0;
+    std::vector<int> first; // first block of each launch, then the number of blocks
+    DeviceBuffer group, of_block, pos, halo, count, own, bor, words, z;
+};
+
 } // namespace lpg
 
 struct lpg_fem {
@@ -55,10 +62,9 @@ struct lpg_fem {
     // CUDA graph of a chunk of PCG iterations, reused while its pointers stay the same.
     cudaGraphExec_t pcg_graph = nullptr;
     const void* pcg_graph_key[12] = {};
-    // Plan of the one-launch PCG (lpg_pcg.cuh), built at the first solve: 0 not built, 1 usable in FP32
-    // only, 2 in both precisions, -1 not usable for this mesh.
-    int pcg_plan_state = 0, pcg_plan_blocks = 0, pcg_plan_stride = 0;
-    lpg::DeviceBuffer pl_halo, pl_count, pl_own, pl_bor, pl_words, pl_z;
+    // Plans of the one-launch PCG (lpg_pcg.cuh): of the whole mesh, built at the first solve, and of the
+    // meshes of a batched solve, built by each call.
+    lpg::PcgPlanStore pcg_plan, batch_plan;
     cudaGraphExec_t batch_graph = nullptr; // the batched (per-mesh) PCG iterations
     const void* batch_graph_key[12] = {};
     // What an evaluation leaves for the host, one 16-byte record on the device (d_result) and its
