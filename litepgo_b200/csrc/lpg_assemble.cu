@@ -27,6 +27,7 @@
 
 #include "lpg_internal.h"
 #include "lpg_clamp9.h"
+#include "lpg_tri9.h"
 #include "lpg_eig.cuh"
 #include "lpg_psd.h"
 
@@ -750,10 +751,10 @@ __host__ __device__ constexpr int pair10(int a, int b) {
 // the orthonormal basis q (packed upper triangle, index 3 j' + i):
 //   H_ab(i, k) = sum_{j', l'} q_a(j') q_b(l') M(3 j' + i, 3 l' + k),
 // as Y_a(i, c) = sum_j' q_a(j') M(3 j' + i, c), then H_ab(i, k) = sum_l' q_b(l') Y_a(i, 3 l' + k).
-// MA is any array-like of 45 values (registers or shared memory); out receives 90 values.
-template <typename R, typename MA> __device__ __forceinline__ void blocks_from_q(const MA& Mq, R* __restrict__ out) {
+// Rows a0 to a1 - 1 of the upper triangle only, into out from their first block on.
+template <int a0, int a1, typename R> __device__ __forceinline__ void blocks_from_q(const R (&Mq)[45], R* __restrict__ out) {
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
+    for (int a = a0; a < a1; ++a) {
         R Y[3][9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
@@ -761,12 +762,12 @@ template <typename R, typename MA> __device__ __forceinline__ void blocks_from_q
             for (int c = 0; c < 9; ++c) {
                 R y = 0;
 #pragma unroll
-                for (int jp = 0; jp < 3; ++jp) y = fma(qbasis<R>(a, jp), static_cast<R>(Mq[sym9(3 * jp + i, c)]), y);
+                for (int jp = 0; jp < 3; ++jp) y = fma(qbasis<R>(a, jp), Mq[sym9(3 * jp + i, c)], y);
                 Y[i][c] = y;
             }
 #pragma unroll
         for (int b = a; b < 4; ++b) {
-            R* o = out + 9 * pair10(a, b);
+            R* o = out + 9 * (pair10(a, b) - pair10(a0, a0));
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -781,8 +782,31 @@ template <typename R, typename MA> __device__ __forceinline__ void blocks_from_q
 }
 
 constexpr int kProjThreads = 64;
-constexpr int kProjStride = 127; // 45 (M) + 81 (V) + 1: odd stride, conflict-free 8-byte lanes
 
+// The first `count` values of the shared rows of this warp's marked lanes (`stride` apart, this lane's at row)
+// to their records out: 90 scattered stores a thread would each touch 32 sectors.
+template <int stride, int count, typename R>
+__device__ __forceinline__ void copy_rows(const R* row, R* out, bool marked) {
+    const int lane = threadIdx.x & 31;
+    const R* rows = row - stride * lane;
+    __syncwarp();
+    if (__any_sync(0xffffffffu, marked))
+        for (int i = lane; i < 32 * count; i += 32) { // every lane runs `count` turns
+            const int l = i / count, v = i - l * count;
+            const unsigned long long to = __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(marked ? out : nullptr), l);
+            if (to != 0) reinterpret_cast<R*>(to)[v] = rows[stride * l + v];
+        }
+    __syncwarp();
+}
+
+// The ten blocks of the marked lanes' tangents, through the lanes' shared rows (54 values used).
+template <int stride, typename R>
+__device__ __forceinline__ void store_blocks(const R (&M)[45], R* row, R* out, bool marked) {
+    if (marked) blocks_from_q<0, 1>(M, row);
+    copy_rows<stride, 36>(row, out, marked);
+    if (marked) blocks_from_q<1, 4>(M, row);
+    copy_rows<stride, 54>(row, out + 36, marked);
+}
 
 // Tangent sources of the projection pass: each forms the element's 9x9 tangent M in the q basis
 // (packed upper triangle into A; V is 81 values of per-thread scratch) and returns status bits.
@@ -890,6 +914,41 @@ __device__ __forceinline__ unsigned form_tangent(const MatTangent& src, const De
     return st;
 }
 
+// Whether M + tol I is positive definite, tol = 64 eps max |diag M| (round-off of a singular semi-definite M,
+// e.g. the rotation modes near rest): LDL^T without pivoting, stable on a positive definite matrix, in
+// registers. Such an M is its own clamp up to that round-off. M is overwritten.
+template <typename R> __device__ __forceinline__ bool semidefinite9(R (&M)[45]) {
+    R scale = 0;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) scale = fmax(scale, fabs(M[sym9(r, r)]));
+    const R tol = R(64) * Eps<R>::v * scale;
+    bool pd = scale < R(INFINITY);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const R d = M[sym9(k, k)] + tol;
+        pd = pd && d > R(0);
+        const R inv = R(1) / d;
+#pragma unroll
+        for (int i = k + 1; i < 9; ++i) {
+            const R l = M[sym9(k, i)] * inv;
+#pragma unroll
+            for (int j = i; j < 9; ++j) M[sym9(i, j)] -= l * M[sym9(k, j)];
+        }
+    }
+    return pd;
+}
+
+// Values of a thread's shared row: the neo-Hookean tangent lives in registers and needs it for M and the
+// blocks; a material's is formed there (45), with 81 of scratch. Odd: conflict-free.
+template <class Src> constexpr int proj_stride() { return 127; }
+template <> constexpr int proj_stride<NhTangent>() { return 55; }
+
+// Forms every element's tangent. A semi-definite one (or one to be kept exact) is final and its blocks are
+// stored; otherwise M is, and the element is listed for clamp_kernel, which runs the eigenvalue clamp on the
+// listed elements only (a warp here then never waits on another lane's iteration).
+// Bound by its arithmetic and stores. With M and its factors in shared memory, a pivoted test of run-time
+// indices and 90 scattered stores a thread it took 131 us for 178,200 tets in FP32 and 62 for 52,800 in FP64;
+// this takes 38 and 16.
 template <typename R, class Src>
 __global__ void __launch_bounds__(kProjThreads) project_kernel(const DevMesh m, const Src src,
                                                                R* __restrict__ proj, unsigned* status,
@@ -897,89 +956,98 @@ __global__ void __launch_bounds__(kProjThreads) project_kernel(const DevMesh m, 
                                                                const int* __restrict__ mesh_exact, int* list,
                                                                unsigned* count) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R* A = reinterpret_cast<R*>(smem_raw) + kProjStride * threadIdx.x;
-    R* V = A + 45;
+    constexpr int stride = proj_stride<Src>();
+    constexpr bool closed = std::is_same<Src, NhTangent>::value;
+    R* row = reinterpret_cast<R*>(smem_raw) + stride * threadIdx.x;
+    const int lane = threadIdx.x & 31;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned st = 0;
     // Per-mesh state of a batched solve: 0 projected, 1 exact, 2 finished (the element is skipped).
     const int state = (e < m.T && emesh != nullptr) ? mesh_exact[emesh[e]] : 0;
-    if (e < m.T && state != 2) {
-        st |= form_tangent<R>(src, m, e, A, V);
-        // Elements of a mesh marked exact keep their tangent unclamped (the Exact Hessian).
-        const bool keep = keeps_exact(src) || state == 1;
-        // Positive semi-definiteness test: LDL^T with diagonal pivoting on a copy in the V area
-        // (row-major 9x9). Pivots above tol are eliminated; once none is left, M is semi-definite
-        // if the remaining Schur complement is below tol everywhere (tol = 64 eps max|diag M|:
-        // round-off of a singular semi-definite M, e.g. the rotation modes near rest). Such an M is
-        // its own clamp up to that round-off; any other goes to clamp_kernel.
-        bool pd = true;
-        if (!keep) {
-            R scale = 0;
-            for (int r = 0; r < 9; ++r) {
-                scale = fmax(scale, fabs(A[sym9(r, r)]));
-                for (int c = 0; c < 9; ++c) V[9 * r + c] = A[sym9(r, c)];
-            }
-            pd = semidefinite_ldlt<9>(V, R(64) * Eps<R>::v * scale);
-            if (!(scale < R(INFINITY))) pd = false;
-        }
-        // Semi-definite (or kept exact): final. Otherwise the unclamped tangent is stored and
-        // the element is listed for clamp_kernel, which runs the eigenvalue clamp on the listed
-        // elements only (a warp of pass 1 then never waits on another lane's Jacobi sweeps).
-        R* out = proj + kProjRecord * static_cast<size_t>(e);
-        if (pd || keep) {
-            blocks_from_q<R>(A, out);
-        } else {
-            for (int t = 0; t < 45; ++t) out[t] = A[t]; // the clamp reads M here and writes the blocks
-            list[atomicAdd(count, 1u)] = e;
-        }
-    }
-    st = __reduce_or_sync(0xffffffffu, st);
-    if ((threadIdx.x & 31) == 0 && st) atomicOr(status, st);
-}
-
-// Eigenvalue clamp of the listed elements' 9x9 tangents (parallel-ordered cyclic Jacobi):
-// M = V max(Lambda, 0) V^T, in place; grid-stride over the list whose length pass 1 counted.
-// One thread per element with the packed matrix and the rotations in registers; in FP64 the
-// eigenvectors V live in shared memory (81 doubles per thread, an odd stride: conflict-free),
-// since A and V together would exceed the register file.
-template <typename R, bool VREG, typename VA>
-__device__ __forceinline__ void clamp9(R* __restrict__ out, VA& V) {
-    R A[45];
+    const bool on = e < m.T && state != 2;
+    // Elements of a mesh marked exact keep their tangent unclamped (the Exact Hessian).
+    const bool keep = keeps_exact(src) || state == 1;
+    bool final = false;
+    R M[45];
+    if (on) {
+        if constexpr (closed) {
+            st |= form_tangent<R>(src, m, e, M, row);
 #pragma unroll
-    for (int t = 0; t < 45; ++t) A[t] = out[t];
-    clamp9_packed<R, VREG>(A, V);
-    blocks_from_q<R>(A, out); // the clamped M's ten blocks replace M in the element's record
-}
-
-constexpr int kClampVStride = 81;
-// Resident 64-thread blocks per SM the FP32 clamp's register allocation must allow (6: at most
-// 170 registers, a few of them spilled; A, V and the relabelling copy need about 187).
-#ifndef LPG_CLAMP_MIN_BLOCKS_F32
-#define LPG_CLAMP_MIN_BLOCKS_F32 6
-#endif
-
-// Register-budget variants of the clamp (autotuner): FP32 at LPG_CLAMP_MIN_BLOCKS_F32 resident
-// blocks or unconstrained (about 187 registers, no spill); FP64 has one.
-template <typename R> constexpr int clamp_minb(int v) {
-    return sizeof(R) == 8 ? 1 : (v == 0 ? LPG_CLAMP_MIN_BLOCKS_F32 : 1);
-}
-
-template <typename R, int MINB>
-__global__ void __launch_bounds__(kProjThreads, MINB) clamp_kernel(R* __restrict__ proj, const int* __restrict__ list,
-                                                                   const unsigned* __restrict__ count) {
-    const unsigned n = *count;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        R* out = proj + kProjRecord * static_cast<size_t>(list[i]);
-        if constexpr (sizeof(R) == 8) {
-            extern __shared__ __align__(16) unsigned char smem_raw[];
-            // volatile: every access goes to shared memory (cached copies would need the
-            // registers this layout is there to save).
-            volatile R* V = reinterpret_cast<R*>(smem_raw) + kClampVStride * threadIdx.x;
-            clamp9<R, false>(out, V);
+            for (int t = 0; t < 45; ++t) row[t] = M[t];
         } else {
-            R V[81];
-            clamp9<R, true>(out, V);
+            st |= form_tangent<R>(src, m, e, row, row + 45);
+#pragma unroll
+            for (int t = 0; t < 45; ++t) M[t] = row[t];
         }
+        final = keep || semidefinite9<R>(M);
+    }
+    R* out = proj + kProjRecord * static_cast<size_t>(on ? e : 0);
+    copy_rows<stride, 45>(row, out, on && !final);
+    const unsigned listed = __ballot_sync(0xffffffffu, on && !final);
+    if (listed != 0) {
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(count, static_cast<unsigned>(__popc(listed)));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(listed & ((1u << lane) - 1u));
+        if (on && !final) list[at] = e;
+    }
+    if (on && final)
+#pragma unroll
+        for (int t = 0; t < 45; ++t) M[t] = row[t];
+    store_blocks<stride>(M, row, out, on && final);
+    st = __reduce_or_sync(0xffffffffu, st);
+    if (lane == 0 && st) atomicOr(status, st);
+}
+
+// One warp a block: a thread's scratch rows, not its registers, then bound the resident warps in FP64 (11).
+constexpr int kClampThreads = 32;
+// Register-budget variants of the clamp (autotuner), as resident blocks per SM: FP32 at 16 (128 registers) or
+// 12 (168, no spill); FP64 has one, at what its shared memory allows.
+template <typename R> constexpr int clamp_minb(int v) {
+    return sizeof(R) == 8 ? 11 : (v == 0 ? 16 : 12);
+}
+
+// The clamp by the cyclic Jacobi method (lpg_clamp9.h) of the few tangents that tri9_clamp gives up on (none
+// of 150,000 in a sheared box, a few in a million of random states): M from the record, M+ to row. Out of
+// line, so that its 170 registers do not burden the kernel.
+template <typename R> __device__ __noinline__ void clamp9_jacobi(const R* record, R* row) {
+    R A[45], V[81];
+#pragma unroll
+    for (int t = 0; t < 45; ++t) A[t] = record[t];
+    clamp9_packed<R, true>(A, V);
+#pragma unroll
+    for (int t = 0; t < 45; ++t) row[t] = A[t];
+}
+
+// Eigenvalue clamp of the listed elements' 9x9 tangents, M+ = V max(Lambda, 0) V^T, and their blocks;
+// grid-stride over the list whose length pass 1 counted, one thread per element, by the few eigenpairs of one
+// sign (lpg_tri9.h). Bound by latency (dependent FP64 or FP32 operations at 11 to 16 warps an SM).
+// The Jacobi method on all of them took 340 us for 52,800 tangents in FP64 and 203 for 152,000 in FP32; this
+// takes 110 and 95.
+template <typename R, int MINB>
+__global__ void __launch_bounds__(kClampThreads, MINB) clamp_kernel(R* __restrict__ proj, const int* __restrict__ list,
+                                                                    const unsigned* __restrict__ count) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    R* row = reinterpret_cast<R*>(smem_raw) + kTri9Scratch * threadIdx.x;
+    const unsigned n = *count, lane = threadIdx.x;
+    for (unsigned i0 = blockIdx.x * kClampThreads; i0 < n; i0 += gridDim.x * kClampThreads) {
+        const bool on = i0 + lane < n;
+        R* out = proj + kProjRecord * static_cast<size_t>(on ? list[i0 + lane] : 0);
+        R A[45];
+        if (on) {
+#pragma unroll
+            for (int t = 0; t < 45; ++t) A[t] = out[t];
+            const int how = tri9_clamp<R>(A, row);
+            if (how == 1) {
+#pragma unroll
+                for (int t = 0; t < 45; ++t) A[t] += out[t];
+            } else if (how == 0) {
+                clamp9_jacobi<R>(out, row);
+#pragma unroll
+                for (int t = 0; t < 45; ++t) A[t] = row[t];
+            }
+        }
+        __syncwarp();
+        store_blocks<kTri9Scratch>(A, row, out, on);
     }
 }
 
@@ -3240,11 +3308,11 @@ size_t project_bytes(const DevMesh& m, int precision) {
 namespace {
 template <typename R, int MINB>
 void launch_clamp_t(R* proj, const int* list, const unsigned* count, int max_count, cudaStream_t s) {
-    const size_t clamp_sm = sizeof(R) == 8 ? sizeof(R) * kClampVStride * kProjThreads : 0;
+    const size_t clamp_sm = sizeof(R) * kTri9Scratch * kClampThreads;
     thread_local LaunchCache cache; // one wave of this variant
-    const int clamp_grid = resident_grid(clamp_kernel<R, MINB>, kProjThreads, clamp_sm, cache);
-    const int blocks = (max_count + kProjThreads - 1) / kProjThreads;
-    if (blocks > 0) clamp_kernel<R, MINB><<<std::min(clamp_grid, blocks), kProjThreads, clamp_sm, s>>>(proj, list, count);
+    const int clamp_grid = resident_grid(clamp_kernel<R, MINB>, kClampThreads, clamp_sm, cache);
+    const int blocks = (max_count + kClampThreads - 1) / kClampThreads;
+    if (blocks > 0) clamp_kernel<R, MINB><<<std::min(clamp_grid, blocks), kClampThreads, clamp_sm, s>>>(proj, list, count);
 }
 template <typename R>
 void launch_clamp_v(R* proj, const int* list, const unsigned* count, int max_count, int variant, cudaStream_t s) {
@@ -3257,7 +3325,7 @@ void launch_clamp_v(R* proj, const int* list, const unsigned* count, int max_cou
 template <typename R, class Src>
 void launch_project_t(const DevMesh& m, const Src& src, R* proj, unsigned* status, cudaStream_t s, const int* emesh,
                       const int* mesh_exact, int* list, unsigned* count, int clamp_variant) {
-    const size_t sm = sizeof(R) * kProjStride * kProjThreads;
+    const size_t sm = sizeof(R) * proj_stride<Src>() * kProjThreads;
     thread_local LaunchCache cache;
     resident_grid(project_kernel<R, Src>, kProjThreads, sm, cache);
     const int blocks = (m.T + kProjThreads - 1) / kProjThreads;
