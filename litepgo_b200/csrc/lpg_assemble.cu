@@ -1908,6 +1908,12 @@ template <int K> __device__ __forceinline__ uint32_t contributor(const uint16_t*
     return en[c];
 }
 
+// The gather of the elements' blocks into the Hessian, one slot per thread; a diagonal slot, which has about
+// 24 contributors in a tet mesh where an edge has five, is summed by four lanes: part k takes contributors
+// [cnt k / 4, cnt (k + 1) / 4), added as (p0 + p1) + (p2 + p3). Bound by the latency and the sectors of
+// its scattered loads. One lane a slot throughout took 45 us for 52,800 tets in FP64, 71 for 178,200 in FP32
+// and 74 for 27 tricubic hexes; this takes 32, 65 and 52. Blocks padded for 16-byte loads gain another 6 us
+// in FP32 here and lose 15 in the kernels that write them; two contributors at a time cost registers: 35, 69.
 template <typename R, int K = 4>
 __global__ void __launch_bounds__(kClThreads) block_gather_kernel(const DevMesh m, const EvalArgs a) {
     using CB = CellBlocks<K>;
@@ -1948,27 +1954,22 @@ __global__ void __launch_bounds__(kClThreads) block_gather_kernel(const DevMesh 
         __syncthreads();
         // The solver layout skips the slots left of the diagonal.
         const int first = a.layout == kLayoutSell ? __ldg(m.cl_ntr + cl) : 0;
-        for (int s = first + tid; s < ns; s += bd) {
-            const uint32_t d = sslot[s], de = sslote[s];
-            const int j = d & 0xffu, q = (d >> 8) & 0x3fffffu;
-            const uint16_t* en = sent + (de & 0xfffffu);
-            const int cnt = static_cast<int>(de >> 20);
-            R acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            for (int c = 0; c < cnt; ++c) {
+        // Sum of contributors [c0, c1) of the slot whose list is en.
+        const auto sum = [&](const uint16_t* en, int c0, int c1, R (&acc)[9]) {
+#pragma unroll 1
+            for (int c = c0; c < c1; ++c) {
                 const uint32_t w = contributor<K>(en, c);
                 const int el = static_cast<int>(w >> (2 * CB::shift)), la = (w >> CB::shift) & (K - 1), lb = w & (K - 1);
                 const R* blk = blocks + CB::record * static_cast<size_t>(sel[el]) + 9 * CB::pair(la, lb);
                 R bv[9];
 #pragma unroll
                 for (int t = 0; t < 9; ++t) bv[t] = __ldg(blk + t);
-                if (la <= lb) {
 #pragma unroll
-                    for (int t = 0; t < 9; ++t) acc[t] += bv[t];
-                } else {
-#pragma unroll
-                    for (int t = 0; t < 9; ++t) acc[t] += bv[3 * (t % 3) + t / 3];
-                }
+                for (int t = 0; t < 9; ++t) acc[t] += la <= lb ? bv[t] : bv[3 * (t % 3) + t / 3];
             }
+        };
+        const auto write = [&](uint32_t d, const R (&acc)[9]) {
+            const int j = d & 0xffu, q = (d >> 8) & 0x3fffffu;
             const bool tr = (d >> 30) & 1u;
             const int slot0 = rt[j], nb = rt[kClusterRows + j], sb = rt[2 * kClusterRows + j];
 #pragma unroll
@@ -1977,6 +1978,25 @@ __global__ void __launch_bounds__(kClThreads) block_gather_kernel(const DevMesh 
                 if (!(val == val) || val == R(INFINITY) || val == R(-INFINITY)) st |= ST_NONFINITE_OUT;
                 hout[cl_pos(a.layout, slot0, nb, sb, q, t)] = static_cast<HT>(val);
             }
+        };
+        // The diagonal slots are the last nr; they go first, four lanes each, in whole warps.
+        const int nd = (4 * nr + 31) & ~31, no = ns - nr - first;
+        for (int i = tid; i < nd + no; i += bd) {
+            R acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+            const bool diag = i < nd;
+            const int s = diag ? ns - nr + (i >> 2) : first + i - nd;
+            if (s < ns) {
+                const uint32_t de = sslote[s];
+                const int cnt = static_cast<int>(de >> 20), part = i & 3;
+                sum(sent + (de & 0xfffffu), diag ? cnt * part / 4 : 0, diag ? cnt * (part + 1) / 4 : cnt, acc);
+            }
+            if (diag)
+#pragma unroll
+                for (int t = 0; t < 9; ++t) {
+                    acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 1);
+                    acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 2);
+                }
+            if (s < ns && (!diag || (i & 3) == 0)) write(sslot[s], acc);
         }
         __syncthreads(); // the next cluster reuses the shared tables
     }
