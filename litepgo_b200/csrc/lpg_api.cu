@@ -211,12 +211,25 @@ lpg_fem::~lpg_fem() {
     if (pcg_graph) cudaGraphExecDestroy(pcg_graph);
     if (batch_graph) cudaGraphExecDestroy(batch_graph);
     if (host_result) cudaFreeHost(host_result);
+    if (host_block) cudaFreeHost(host_block);
     if (own_stream) cudaStreamDestroy(own_stream);
 }
 
 void lpg_fem::create_result() {
     LPG_CUDA(cudaMemset(d_result.as<EvalResult>(1), 0, sizeof(EvalResult)));
     LPG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host_result), 4096, cudaHostAllocDefault));
+}
+
+double* lpg_fem::host_values(size_t count) {
+    if (count > host_block_size) {
+        sync(); // kernels may still write the old block
+        if (host_block) cudaFreeHost(host_block);
+        host_block = nullptr;
+        host_block_size = 0;
+        LPG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&host_block), count * sizeof(double), cudaHostAllocDefault));
+        host_block_size = count;
+    }
+    return host_block;
 }
 
 void lpg_fem::sync() { LPG_CUDA(cudaStreamSynchronize(stream)); }

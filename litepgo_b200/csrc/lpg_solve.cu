@@ -899,35 +899,40 @@ struct Solver {
     explicit Solver(lpg_fem& hh, const Potential* p = nullptr)
         : h(hh), s(hh.stream), n(3 * static_cast<size_t>(hh.dm.V)), V(hh.dm.V), P(p) {}
 
-    // {sum m a b, sum m a^2, max m|a|, sum m b^2}
-    template <typename TA, typename TB> std::array<double, 4> stats(const TA* a, const TB* b, const double* mask) {
+    // What the host decides on is written by the kernels into slots of pinned memory and read after one
+    // synchronisation: four of them an iteration. With a copy and a wait for each value (12) and a residual
+    // that no one read, an iteration of 648 vertices took 385 us beside its PCG, 270 so.
+    enum Slot { kXf, kXAx, kGrad, kDirection, kResidual, kOther };
+    // {sum m a b, sum m a^2, max m|a|, sum m b^2} into the slot.
+    template <typename TA, typename TB> void stats_async(const TA* a, const TB* b, const double* mask, Slot slot) {
         const int nb = red_blocks(n);
         double* part = h.s_part.as<double>(4 * 1024);
-        double* out = h.s_scal.as<double>(64) + 32;
         stats_partial<TA, TB><<<nb, kThreads, 0, s>>>(a, b, mask, n, part);
-        stats_final<<<1, 1024, 0, s>>>(part, nb, out);
+        stats_final<<<1, 1024, 0, s>>>(part, nb, h.host_sums(slot));
         LPG_CUDA(cudaGetLastError());
+    }
+    template <typename TA, typename TB> std::array<double, 4> stats(const TA* a, const TB* b, const double* mask) {
+        stats_async(a, b, mask, kOther);
+        h.sync();
         std::array<double, 4> r{};
-        LPG_CUDA(cudaMemcpyAsync(h.host_sums(), out, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
-        LPG_CUDA(cudaStreamSynchronize(s));
-        std::copy(h.host_sums(), h.host_sums() + 4, r.begin());
+        std::copy(h.host_sums(kOther), h.host_sums(kOther) + 4, r.begin());
         return r;
     }
 
-    double energy_dot_f(const double* x, const double* f) {
-        if (!f) return 0.0;
-        return stats<double, double>(x, f, nullptr)[0];
-    }
-
-    // E(x) (FP64) with optional gradient g (FP64, load included); throws on bad status.
-    double energy(const double* x, const double* f, double* g) {
+    // Enqueues E(x) (FP64) with optional gradient g (FP64, load included).
+    void energy_async(const double* x, const double* f, double* g) {
         eval_elastic_async(h, P ? P->t : nullptr, x, g, LPG_HESSIAN_NONE, LPG_PRECISION_F64, LPG_LAYOUT_BSR, nullptr);
-        return compose(x, f, g);
+        compose_async(x, f, g);
+    }
+    // The same and its value; throws on bad status.
+    double energy(const double* x, const double* f, double* g) {
+        energy_async(x, f, g);
+        raise_status(h.take_status());
+        return energy_value(f);
     }
     // The potential from the elastic evaluation just enqueued (energy in h.result(), gradient
     // in g if given): weight, quadratic term, load and constant.
-    double compose(const double* x, const double* f, double* g) {
-        double aq = 0;
+    void compose_async(const double* x, const double* f, double* g) {
         if (P && (P->w != 1.0 || P->n > 0)) {
             if (P->n > 0)
                 csr_apply_kernel<<<grid(static_cast<size_t>(P->n)), kThreads, 0, s>>>(P->ptr, P->col, P->val, x, P->Ax,
@@ -936,11 +941,14 @@ struct Solver {
             LPG_CUDA(cudaGetLastError());
         }
         if (g && f) load_gradient<<<grid(n), kThreads, 0, s>>>(g, f, n);
-        raise_status(h.take_status());
+        if (P && P->n > 0) stats_async<double, double>(x, P->Ax, nullptr, kXAx);
+        if (f) stats_async<double, double>(x, f, nullptr, kXf);
+    }
+    // The potential enqueued by compose_async, after take_status().
+    double energy_value(const double* f) {
         double e = h.host_result->energy;
-        if (P && P->n > 0) aq = 0.5 * stats<double, double>(x, P->Ax, nullptr)[0];
-        if (P) e = P->w * e + aq + P->c;
-        return e - energy_dot_f(x, f);
+        if (P) e = P->w * e + (P->n > 0 ? 0.5 * h.host_sums(kXAx)[0] : 0.0) + P->c;
+        return f ? e - h.host_sums(kXf)[0] : e;
     }
     // The quadratic term and weight applied to a solver-layout Hessian of precision R.
     template <typename R> void compose_hessian(R* K) {
@@ -975,7 +983,7 @@ struct Solver {
     struct PcgOut {
         int64_t iters = 0;
         bool breakdown = false;
-        double rel = 0; // final ||b - K x|| / ||b|| in FP64
+        double rel = 0; // final ||b - K x|| / ||b|| in FP64 (not formed for a direction)
     };
 
     // Enqueues `pairs` x 2 PCG iterations on stream gs (two launches per iteration; p_new and
@@ -1025,13 +1033,13 @@ struct Solver {
         return h.pcg_plan.state >= (sizeof(R) == 8 ? 2 : 1);
     }
 
-    // Solves mask K x = mask b (FP64 b, x): inner PCG in precision R on Kin (values of type R),
-    // FP64 residual refinement against Kres (FP64 values when res64, else Kin's values). The
-    // iterations run as a replayed CUDA graph of 32 iterations; the host checks the device
-    // state after each replay.
+    // Solves mask K x = mask b (FP64 b of norm bnorm, x): inner PCG in precision R on Kin (values of type R),
+    // FP64 residual refinement against Kres (FP64 values when res64, else Kin's values). The iterations run
+    // in one launch, or as a replayed CUDA graph of 32 iterations, where the host checks the device state
+    // after each replay. A direction needs no residual of its last solve.
     template <typename R>
     PcgOut pcg(const void* Kin, const R* dinv, const void* Kres, bool res64, const double* mask, const double* b64,
-               double* x64, double tol, int max_iters, int max_refine) {
+               double bnorm, double* x64, double tol, int max_iters, int max_refine, bool direction) {
         PcgOut out;
         // The PCG vectors are padded to 4 values per vertex (4th value zero).
         const size_t n4 = 4 * static_cast<size_t>(V);
@@ -1051,7 +1059,6 @@ struct Solver {
         PcgState* st = reinterpret_cast<PcgState*>(h.s_scal.as<double>(64));
         LPG_CUDA(cudaMemsetAsync(x64, 0, n * sizeof(double), s));
         LPG_CUDA(cudaMemcpyAsync(r64, b64, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        const double bnorm = std::sqrt(stats<double, double>(b64, nullptr, mask)[1]);
         if (bnorm == 0) return out;
         pad_rhs<R><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(mask, mask, mask4, V); // 0/1 values: mask^2 = mask
         const bool one = one_launch<R>();
@@ -1084,10 +1091,20 @@ struct Solver {
             const double inner_tol = std::min(0.5, std::max(tol * bnorm / rnorm, sizeof(R) == 4 ? 1e-6 : 1e-14));
             pad_rhs<R><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(r64, mask, bR, V);
             PcgState hs{};
+            auto copy_state = [&]() { LPG_CUDA(cudaMemcpyAsync(h.host_pcg(), st, sizeof hs, cudaMemcpyDeviceToHost, s)); };
             auto read_state = [&]() {
-                LPG_CUDA(cudaMemcpyAsync(h.host_pcg(), st, sizeof hs, cudaMemcpyDeviceToHost, s));
-                LPG_CUDA(cudaStreamSynchronize(s));
+                h.sync();
                 std::memcpy(&hs, h.host_pcg(), sizeof hs);
+            };
+            const bool residual = !direction || ref < max_refine;
+            auto update = [&]() {
+                add_kernel<R><<<grid(n), kThreads, 0, s>>>(x64, x, n);
+                if (residual) {
+                    residual_spmv(Kres, res64, x64, mask, y64);
+                    residual_kernel<<<grid(n), kThreads, 0, s>>>(b64, y64, mask, r64, n);
+                    stats_async<double, double>(r64, nullptr, mask, kResidual);
+                }
+                LPG_CUDA(cudaGetLastError());
             };
             if (one) {
                 PcgArgs<R> a{};
@@ -1096,6 +1113,8 @@ struct Solver {
                 a.max_iters = max_iters - static_cast<int>(out.iters);
                 a.first_direction = true;
                 launch_pcg<R>(h, h.pcg_plan, a);
+                copy_state();
+                update();
                 read_state();
                 if (hs.lost) {
                     clear_words(h, h.pcg_plan); // the blocks' numbers may differ now
@@ -1111,21 +1130,20 @@ struct Solver {
                     LPG_CUDA(cudaGraphLaunch(h.pcg_graph, gs));
                     LPG_CUDA(cudaEventRecord(ev, gs));
                     LPG_CUDA(cudaStreamWaitEvent(s, ev, 0));
+                    copy_state();
                     read_state();
                     if (hs.done) break;
                 }
+                // Negative curvature on the first step: keep the preconditioned residual direction.
+                if (hs.breakdown && hs.iters == 0)
+                    LPG_CUDA(cudaMemcpyAsync(x, pB, n4 * sizeof(R), cudaMemcpyDeviceToDevice, s));
+                update();
+                if (residual) h.sync();
             }
             out.iters += hs.iters;
-            if (hs.breakdown) {
-                out.breakdown = true;
-                // Negative curvature on the first step: keep the preconditioned residual direction.
-                if (!one && hs.iters == 0) LPG_CUDA(cudaMemcpyAsync(x, pB, n4 * sizeof(R), cudaMemcpyDeviceToDevice, s));
-            }
-            add_kernel<R><<<grid(n), kThreads, 0, s>>>(x64, x, n);
-            residual_spmv(Kres, res64, x64, mask, y64);
-            residual_kernel<<<grid(n), kThreads, 0, s>>>(b64, y64, mask, r64, n);
-            LPG_CUDA(cudaGetLastError());
-            rnorm = std::sqrt(stats<double, double>(r64, nullptr, mask)[1]);
+            if (hs.breakdown) out.breakdown = true;
+            if (!residual) break;
+            rnorm = std::sqrt(h.host_sums(kResidual)[1]);
             out.rel = rnorm / bnorm;
             if (out.breakdown || !(rnorm > tol * bnorm) || out.iters >= max_iters || !std::isfinite(rnorm)) break;
         }
@@ -1332,15 +1350,17 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
         step.iteration = it;
         step.pattern_changed = it == 0;
         // Energy and FP64 gradient (the Newton residual).
-        double E;
         if (f64) {
             eval_elastic_async(h, terms, x, g, hk, LPG_PRECISION_F64, kLayoutSell, K);
-            E = S.compose(x, f, g);
+            S.compose_async(x, f, g);
             S.compose_hessian(static_cast<double*>(K));
         } else {
-            E = S.energy(x, f, g);
+            S.energy_async(x, f, g);
         }
-        const auto gs = S.stats<double, double>(g, nullptr, mask);
+        S.stats_async<double, double>(g, nullptr, mask, Solver::kGrad);
+        raise_status(h.take_status());
+        const double E = S.energy_value(f);
+        const double* gs = h.host_sums(Solver::kGrad);
         const double g2 = std::sqrt(gs[1]), gmax = gs[2];
         if (gnorm0 < 0) gnorm0 = g2;
         if (o.exact_below > 0 && g2 <= o.exact_below * gnorm0) exact = true;
@@ -1367,20 +1387,10 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
         }
         // Descent direction with diagonal shifts (newton.cpp:55-72).
         neg_mask<<<grid(n), kThreads, 0, s>>>(g, mask, rhs, n);
-        double dscale = 1.0;
-        {
-            const int vb = grid(static_cast<size_t>(V));
-            double* part = h.s_part.as<double>(std::max(4 * 1024, vb));
-            double* outm = h.s_scal.as<double>(64) + 40;
-            diag_absmax_partial<<<vb, kThreads, 0, s>>>(h.dm, f64 ? static_cast<double*>(K) : nullptr,
-                                                       f64 ? nullptr : static_cast<float*>(K), mask, part);
-            max_final<<<1, 32, 0, s>>>(part, vb, outm);
-            double m = 0;
-            LPG_CUDA(cudaMemcpyAsync(&m, outm, sizeof m, cudaMemcpyDeviceToHost, s));
-            LPG_CUDA(cudaStreamSynchronize(s));
-            dscale = std::max(1.0, m);
-        }
-        double shift = 1e-8 * dscale;
+        double shift = 0; // from the largest diagonal entry, at the first shift
+        const int nb = feasible_blocks(h.dm);
+        double* bm = h.d_block.as<double>(std::max(nb, 1));
+        const bool own_step = terms && terms->feasible;
         const double eta = std::min(o.cg_tolerance, std::sqrt(g2 / gnorm0));
         bool found = false;
         double gd = 0;
@@ -1389,20 +1399,34 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
             if (f64) {
                 block_jacobi<double, double><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(
                     h.dm, static_cast<double*>(K), mask, static_cast<double*>(dinv), V);
-                po = S.pcg<double>(K, static_cast<double*>(dinv), K, true, mask, rhs, d, eta, o.cg_max_iterations, 0);
+                po = S.pcg<double>(K, static_cast<double*>(dinv), K, true, mask, rhs, g2, d, eta, o.cg_max_iterations, 0, true);
             } else {
                 block_jacobi<float, float><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(
                     h.dm, static_cast<float*>(K), mask, static_cast<float*>(dinv), V);
-                po = S.pcg<float>(K, static_cast<float*>(dinv), K, false, mask, rhs, d, eta, o.cg_max_iterations, 3);
+                po = S.pcg<float>(K, static_cast<float*>(dinv), K, false, mask, rhs, g2, d, eta, o.cg_max_iterations, 3, true);
             }
             R.cg_iterations += po.iters;
-            gd = S.stats<double, double>(g, d, mask)[0];
+            // g . d, and the feasible step along d, whose status counts only where d is taken.
+            S.stats_async<double, double>(g, d, mask, Solver::kDirection);
+            if (!own_step) launch_feasible(h.dm, x, d, bm, nb, h.host_step(), h.status_word(), s);
+            const unsigned status = h.take_status();
+            gd = h.host_sums(Solver::kDirection)[0];
             step.diagonal_shifts = shifts;
             if (gd < 0.0 && std::isfinite(gd)) {
+                raise_status(status);
                 found = true;
                 break;
             }
             if (shifts == 10) break;
+            if (shifts == 0) {
+                const int vb = grid(static_cast<size_t>(V));
+                double* part = h.s_part.as<double>(std::max(4 * 1024, vb));
+                diag_absmax_partial<<<vb, kThreads, 0, s>>>(h.dm, f64 ? static_cast<double*>(K) : nullptr,
+                                                           f64 ? nullptr : static_cast<float*>(K), mask, part);
+                max_final<<<1, 32, 0, s>>>(part, vb, h.host_sums(Solver::kOther));
+                h.sync();
+                shift = 1e-8 * std::max(1.0, h.host_sums(Solver::kOther)[0]);
+            }
             shift_diag<<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(h.dm, f64 ? static_cast<double*>(K) : nullptr,
                                                                        f64 ? nullptr : static_cast<float*>(K), shift);
             shift *= 10.0;
@@ -1413,11 +1437,8 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
             return finish(3);
         }
         // Line search (newton.cpp:92-108) from the feasible step.
-        const int nb = feasible_blocks(h.dm);
-        double* bm = h.d_block.as<double>(std::max(nb, 1));
-        double* al = h.d_alpha.as<double>(1);
-        double alpha = 1;
-        if (terms && terms->feasible) {
+        double alpha = own_step ? 1.0 : *h.host_step();
+        if (own_step) {
             const bool hex = h.dm.K == 8;
             const size_t rows = static_cast<size_t>(h.dm.T) * (hex ? h.dm.nq : 1);
             double* Fx = h.d_mat[4].as<double>(std::max<size_t>(9 * rows, 1));
@@ -1435,25 +1456,27 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
                 fail(LPG_ESTOPPED, "newton_solve: the feasible-step callback stopped the solve");
             if (!(alpha >= 0.0 && alpha <= 1.0))
                 fail(LPG_ELOGIC, "Energy::max_feasible_step: the energy returned a value outside [0, 1]");
-        } else {
-            launch_feasible(h.dm, x, d, bm, nb, al, h.status_word(), s);
-            LPG_CUDA(cudaMemcpyAsync(&alpha, al, sizeof alpha, cudaMemcpyDeviceToHost, s));
-            raise_status(h.take_status());
         }
         step.feasible_step = alpha;
         bool accepted = false;
+        const bool callbacks = terms && terms->material;
         if (!have_Ex) Ex = S.energy(x, f, nullptr);
         have_Ex = true;
         for (int j = 0; j < o.max_line_search_steps; ++j) {
             LPG_CUDA(cudaMemsetAsync(moved, 0, sizeof(int), s));
             axpy_trial<<<grid(n), kThreads, 0, s>>>(x, alpha, d, trial, n, moved);
-            int mv = 0;
-            LPG_CUDA(cudaMemcpyAsync(&mv, moved, sizeof mv, cudaMemcpyDeviceToHost, s));
-            LPG_CUDA(cudaStreamSynchronize(s));
-            if (!mv) break;
+            LPG_CUDA(cudaMemcpyAsync(h.host_moved(), moved, sizeof(int), cudaMemcpyDeviceToHost, s));
+            if (callbacks) {
+                h.sync(); // a point that has not moved is not shown to the caller
+                if (!*h.host_moved()) break;
+            }
+            S.energy_async(trial, f, nullptr);
+            const unsigned status = h.take_status();
+            if (!*h.host_moved()) break; // the trial is x
+            raise_status(status);
             ++R.line_search_evaluations;
             ++step.line_search_evaluations;
-            const double Et = S.energy(trial, f, nullptr);
+            const double Et = S.energy_value(f);
             const double noise = 16.0 * kEps * std::max(1.0, std::abs(Ex));
             const double armijo = o.accept_rule == 1 ? 1e-4 * alpha * gd : 0.0;
             if (Et <= Ex + armijo + noise) {
@@ -1514,13 +1537,13 @@ void adjoint_solve(lpg_fem& h, const double* u_star, const double* dLdu, const i
     if (precision == LPG_PRECISION_F64) {
         double* dinv = h.s_dinv.as<double>(12 * static_cast<size_t>(std::max(V, 1)));
         block_jacobi<double, double><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(h.dm, K64, mask, dinv, V);
-        po = S.pcg<double>(K64, dinv, K64, true, mask, rhs, lam, cg_tolerance, 200000, 2);
+        po = S.pcg<double>(K64, dinv, K64, true, mask, rhs, std::sqrt(ws[1]), lam, cg_tolerance, 200000, 2, false);
     } else {
         float* K32 = h.s_hess.as<float>(std::max<size_t>(nv, 1));
         if (nv) convert_kernel<double, float><<<grid(nv), kThreads, 0, s>>>(K64, K32, nv);
         float* dinv = h.s_dinv.as<float>(12 * static_cast<size_t>(std::max(V, 1)));
         block_jacobi<float, float><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(h.dm, K32, mask, dinv, V);
-        po = S.pcg<float>(K32, dinv, K64, true, mask, rhs, lam, cg_tolerance, 200000, 30);
+        po = S.pcg<float>(K32, dinv, K64, true, mask, rhs, std::sqrt(ws[1]), lam, cg_tolerance, 200000, 30, false);
     }
     if (po.breakdown) fail(LPG_EDOMAIN, "StaticEquilibriumResponse: singular or indefinite equilibrium stiffness");
     // Residual check (static_equilibrium_response.cpp:61-68) in FP64 with the exact Hessian.
@@ -1639,10 +1662,11 @@ namespace {
 
 // One block per mesh over the DOFs [3 voff[m], 3 voff[m+1]): out[4m..] = {sum w a b, sum w a^2,
 // max w |a|, sum w b^2} with w = mask (1 where mask is null) and b = 0 where b is null.
-__global__ void __launch_bounds__(256) seg_stats(const double* __restrict__ a, const double* __restrict__ b,
+constexpr int kSegThreads = 1024; // at 256 a thread has up to 58 loads in a row: 13.6 and 16.3 us, 9.9 and 9.6 so
+__global__ void __launch_bounds__(kSegThreads) seg_stats(const double* __restrict__ a, const double* __restrict__ b,
                                                  const double* __restrict__ mask, const int* __restrict__ voff,
                                                  double* __restrict__ out) {
-    __shared__ double sh[4][8];
+    __shared__ double sh[4][kSegThreads / 32];
     const int m = blockIdx.x;
     const size_t lo = 3 * static_cast<size_t>(voff[m]), hi = 3 * static_cast<size_t>(voff[m + 1]);
     double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
@@ -1677,9 +1701,9 @@ __global__ void __launch_bounds__(256) seg_stats(const double* __restrict__ a, c
 
 // One block per mesh over its elements [eoff[m], eoff[m+1]): sum (min_mode 0) or minimum
 // starting from 1 (min_mode 1) of a per-element value.
-__global__ void __launch_bounds__(256) seg_elem(const double* __restrict__ x, const int* __restrict__ eoff,
+__global__ void __launch_bounds__(kSegThreads) seg_elem(const double* __restrict__ x, const int* __restrict__ eoff,
                                                 int min_mode, double* __restrict__ out) {
-    __shared__ double sh[8];
+    __shared__ double sh[kSegThreads / 32];
     const int m = blockIdx.x;
     double v = min_mode ? 1.0 : 0.0;
     for (int e = eoff[m] + threadIdx.x; e < eoff[m + 1]; e += blockDim.x) v = min_mode ? fmin(v, x[e]) : v + x[e];
@@ -1957,7 +1981,7 @@ struct BatchDev {
     int *voff = nullptr, *eoff = nullptr, *mov = nullptr, *emesh = nullptr;
     int *act = nullptr, *take = nullptr, *exact = nullptr;
     unsigned char *tc_skip = nullptr, *cl_skip = nullptr;
-    double *stats = nullptr, *esum = nullptr, *fdot = nullptr, *amin = nullptr, *alpha = nullptr, *tol = nullptr;
+    double *alpha = nullptr, *tol = nullptr;
     double *rowdot = nullptr, *rowdot2 = nullptr, *elem = nullptr;
     BatchPcg pcg{};
 };
@@ -1979,28 +2003,37 @@ struct BatchSolver {
     template <typename T> void up(T* p, const std::vector<T>& v) {
         if (!v.empty()) LPG_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
     }
-    // Per-mesh {sum w a b, sum w a^2, max w|a|, sum w b^2}.
-    std::vector<double> stats(const double* a, const double* b, const double* mask) {
-        seg_stats<<<M, 256, 0, s>>>(a, b, mask, d.voff, d.stats);
+    // Per-mesh values in pinned memory, read after the next synchronisation (Solver::Slot's reasons).
+    enum Slot { kXf = 0, kGrad = 4, kOther = 8, kEnergy = 12, kStep = 13, kState = 14, kSlots = 26 };
+    static_assert(sizeof(PcgState) <= (kSlots - kState) * sizeof(double), "the PCG states' place");
+    double* values(int slot) const { return h.host_values(kSlots * static_cast<size_t>(M)) + slot * static_cast<size_t>(M); }
+    // {sum w a b, sum w a^2, max w|a|, sum w b^2} of each mesh.
+    void stats_async(const double* a, const double* b, const double* mask, Slot slot) {
+        seg_stats<<<M, kSegThreads, 0, s>>>(a, b, mask, d.voff, values(slot));
         LPG_CUDA(cudaGetLastError());
-        std::vector<double> r;
-        down(r, d.stats, 4 * static_cast<size_t>(M));
-        return r;
     }
-    // Per-mesh energy at x: element energies summed per mesh, minus f . x.
-    std::vector<double> energies(const double* x, const double* f, double* g, int hk, int precision, void* K) {
+    std::vector<double> read(int slot, int per = 4) const {
+        const double* v = values(slot);
+        return std::vector<double>(v, v + per * static_cast<size_t>(M));
+    }
+    // Per-mesh energy at x: element energies summed per mesh, minus f . x (after take_status()).
+    void energies_async(const double* x, const double* f, double* g, int hk, int precision, void* K) {
         h.eval_async(x, g, hk, precision, kLayoutSell, K, d.elem, nullptr, nullptr, d.emesh, d.exact, d.tc_skip,
                      d.cl_skip);
-        seg_elem<<<M, 256, 0, s>>>(d.elem, d.eoff, 0, d.esum);
+        seg_elem<<<M, kSegThreads, 0, s>>>(d.elem, d.eoff, 0, values(kEnergy));
         LPG_CUDA(cudaGetLastError());
-        raise_status(h.take_status());
-        std::vector<double> e;
-        down(e, d.esum, M);
-        if (f) {
-            const auto fx = stats(x, f, nullptr);
-            for (int m = 0; m < M; ++m) e[m] -= fx[4 * m];
-        }
+        if (f) stats_async(x, f, nullptr, kXf);
+    }
+    std::vector<double> energies_read(const double* f) const {
+        std::vector<double> e = read(kEnergy, 1);
+        if (f)
+            for (int m = 0; m < M; ++m) e[m] -= values(kXf)[4 * m];
         return e;
+    }
+    std::vector<double> energies(const double* x, const double* f, double* g, int hk, int precision, void* K) {
+        energies_async(x, f, g, hk, precision, K);
+        raise_status(h.take_status());
+        return energies_read(f);
     }
 
     struct PcgOut {
@@ -2023,11 +2056,12 @@ struct BatchSolver {
             }
     }
 
-    // Solves mask K x = mask b per active mesh (tolerance tol[m] relative to ||b_m||): inner PCG in
+    // Solves mask K x = mask b per active mesh (tolerance tol[m] relative to ||b_m|| = bnorm[m]): inner PCG in
     // precision R on Kin, FP64 refinement against Kres; the iterations replay a cached graph.
     template <typename R>
     PcgOut pcg(const void* Kin, const R* dinv, const void* Kres, bool res64, const double* mask, const double* b64,
-               double* x64, const std::vector<double>& tol, std::vector<int> act, int max_iters, int max_refine) {
+               const std::vector<double>& bnorm, double* x64, const std::vector<double>& tol, std::vector<int> act,
+               int max_iters, int max_refine) {
         PcgOut out;
         out.breakdown.assign(M, 0);
         const size_t n4 = 4 * static_cast<size_t>(V);
@@ -2043,11 +2077,9 @@ struct BatchSolver {
         double* y64 = h.s_b64.as<double>(n);
         LPG_CUDA(cudaMemsetAsync(x64, 0, n * sizeof(double), s));
         LPG_CUDA(cudaMemcpyAsync(r64, b64, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        const auto bs = stats(b64, nullptr, mask);
-        std::vector<double> bnorm(M), rnorm(M);
+        std::vector<double> rnorm(bnorm);
         bool any = false;
         for (int m = 0; m < M; ++m) {
-            bnorm[m] = rnorm[m] = std::sqrt(bs[4 * m + 1]);
             act[m] = act[m] && bnorm[m] > 0;
             any = any || act[m];
         }
@@ -2078,7 +2110,7 @@ struct BatchSolver {
         LPG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         std::vector<double> itol(M);
         std::vector<int> done, iters, brk;
-        std::vector<PcgState> states;
+        const PcgState* states = reinterpret_cast<const PcgState*>(values(kState));
         PcgState* st = one ? h.s_scal.as<PcgState>(static_cast<size_t>(M)) : nullptr;
         int used = 0;
         for (int ref = 0; ref <= max_refine; ++ref) {
@@ -2094,12 +2126,8 @@ struct BatchSolver {
                 a.tols = d.tol, a.act = d.act;
                 a.max_iters = d.pcg.max_iters;
                 launch_pcg<R>(h, h.batch_plan, a);
-                down(states, st, static_cast<size_t>(M));
-                iters.resize(M), brk.resize(M);
-                for (int m = 0; m < M; ++m) {
-                    if (states[m].lost) fail(LPG_ECUDA, "PCG: the solve's blocks lost one another");
-                    iters[m] = states[m].iters, brk[m] = states[m].breakdown;
-                }
+                LPG_CUDA(cudaMemcpyAsync(values(kState), st, static_cast<size_t>(M) * sizeof(PcgState),
+                                         cudaMemcpyDeviceToHost, s));
             } else {
                 pcg_b_init<R><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(bR, dinv, x, r, z, pA, V, d.rowdot2);
                 pcg_b_start<<<M, 256, 0, s>>>(d.pcg, d.rowdot2, d.voff, d.tol, d.act);
@@ -2116,6 +2144,29 @@ struct BatchSolver {
                 down(iters, d.pcg.iters, M);
                 down(brk, d.pcg.brk, M);
             }
+            const bool residual = ref < max_refine; // the last solve's is not looked at
+            add_kernel<R><<<grid(n), kThreads, 0, s>>>(x64, x, n);
+            if (residual) {
+                if (res64)
+                    spmv_sell<double, double, double, false, false, 3>
+                        <<<std::max(1, (h.dm.n_sell + 7) / 8), kThreads, 0, s>>>(h.dm, static_cast<const double*>(Kres), x64,
+                                                                                nullptr, mask, y64, nullptr, nullptr, nullptr);
+                else
+                    spmv_sell<float, double, double, false, false, 3>
+                        <<<std::max(1, (h.dm.n_sell + 7) / 8), kThreads, 0, s>>>(h.dm, static_cast<const float*>(Kres), x64,
+                                                                                nullptr, mask, y64, nullptr, nullptr, nullptr);
+                residual_kernel<<<grid(n), kThreads, 0, s>>>(b64, y64, mask, r64, n);
+                LPG_CUDA(cudaGetLastError());
+                stats_async(r64, nullptr, mask, kOther);
+            }
+            h.sync();
+            if (one) {
+                iters.resize(M), brk.resize(M);
+                for (int m = 0; m < M; ++m) {
+                    if (states[m].lost) fail(LPG_ECUDA, "PCG: the solve's blocks lost one another");
+                    iters[m] = states[m].iters, brk[m] = states[m].breakdown;
+                }
+            }
             int mx = 0;
             for (int m = 0; m < M; ++m) {
                 if (!act[m]) continue;
@@ -2124,18 +2175,8 @@ struct BatchSolver {
             }
             used += mx;
             out.iters += mx;
-            add_kernel<R><<<grid(n), kThreads, 0, s>>>(x64, x, n);
-            if (res64)
-                spmv_sell<double, double, double, false, false, 3>
-                    <<<std::max(1, (h.dm.n_sell + 7) / 8), kThreads, 0, s>>>(h.dm, static_cast<const double*>(Kres), x64,
-                                                                            nullptr, mask, y64, nullptr, nullptr, nullptr);
-            else
-                spmv_sell<float, double, double, false, false, 3>
-                    <<<std::max(1, (h.dm.n_sell + 7) / 8), kThreads, 0, s>>>(h.dm, static_cast<const float*>(Kres), x64,
-                                                                            nullptr, mask, y64, nullptr, nullptr, nullptr);
-            residual_kernel<<<grid(n), kThreads, 0, s>>>(b64, y64, mask, r64, n);
-            LPG_CUDA(cudaGetLastError());
-            const auto rs = stats(r64, nullptr, mask);
+            if (!residual) break;
+            const auto rs = read(kOther);
             any = false;
             for (int m = 0; m < M; ++m) {
                 rnorm[m] = std::sqrt(rs[4 * m + 1]);
@@ -2207,19 +2248,15 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
     d.pcg.done = pcg_ints;
     d.pcg.iters = pcg_ints + M + 1;
     d.pcg.brk = pcg_ints + 2 * M + 1;
-    double* dbl = h.bt_dbl[0].as<double>(16 * static_cast<size_t>(M));
-    d.stats = dbl;
-    d.esum = dbl + 4 * M;
-    d.fdot = dbl + 5 * M;
-    d.amin = dbl + 6 * M;
-    d.alpha = dbl + 7 * M;
-    d.tol = dbl + 8 * M;
-    d.pcg.rz = dbl + 9 * M;
-    d.pcg.rr = dbl + 10 * M;
-    d.pcg.bb = dbl + 11 * M;
-    d.pcg.tol2 = dbl + 12 * M;
-    d.pcg.alpha = dbl + 13 * M;
-    d.pcg.beta = dbl + 14 * M;
+    double* dbl = h.bt_dbl[0].as<double>(8 * static_cast<size_t>(M));
+    d.alpha = dbl;
+    d.tol = dbl + M;
+    d.pcg.rz = dbl + 2 * M;
+    d.pcg.rr = dbl + 3 * M;
+    d.pcg.bb = dbl + 4 * M;
+    d.pcg.tol2 = dbl + 5 * M;
+    d.pcg.alpha = dbl + 6 * M;
+    d.pcg.beta = dbl + 7 * M;
     d.rowdot = h.bt_dbl[1].as<double>(std::max(V, 1));
     d.rowdot2 = h.bt_dbl[2].as<double>(2 * static_cast<size_t>(std::max(V, 1)));
     d.elem = h.bt_dbl[3].as<double>(std::max(T, 1));
@@ -2311,10 +2348,12 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
         bool all_exact = true;
         for (int m = 0; m < M; ++m) all_exact = all_exact && (exact[m] || !act[m]);
         const int hk = all_exact ? LPG_HESSIAN_EXACT : LPG_HESSIAN_PROJECTED;
-        const std::vector<double> e = f64 ? B.energies(x, f, g, hk, LPG_PRECISION_F64, K)
-                                          : B.energies(x, f, g, LPG_HESSIAN_NONE, LPG_PRECISION_F64, nullptr);
+        B.energies_async(x, f, g, f64 ? hk : LPG_HESSIAN_NONE, LPG_PRECISION_F64, f64 ? K : nullptr);
         if (f) load_gradient<<<grid(n), kThreads, 0, s>>>(g, f, n);
-        const auto gs = B.stats(g, nullptr, mask);
+        B.stats_async(g, nullptr, mask, BatchSolver::kGrad);
+        raise_status(h.take_status());
+        const std::vector<double> e = B.energies_read(f);
+        const auto gs = B.read(BatchSolver::kGrad);
         for (int m = 0; m < M; ++m) {
             if (status[m] >= 0) continue; // finished: skipped by this iteration's evaluation
             E[m] = e[m];
@@ -2346,23 +2385,30 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
         // Descent directions: per-mesh PCG on the block-diagonal system, forcing term per mesh.
         B.up(d.act, act);
         seg_rhs<<<grid(n), kThreads, 0, s>>>(g, mask, d.act, d.mov, rhs, n);
-        std::vector<double> tol(M, 1.0);
+        std::vector<double> tol(M, 1.0), bnorm(M, 0.0);
         for (int m = 0; m < M; ++m)
-            if (act[m]) tol[m] = std::min(o.cg_tolerance, std::sqrt(g2[m] / g0[m]));
+            if (act[m]) bnorm[m] = g2[m], tol[m] = std::min(o.cg_tolerance, std::sqrt(g2[m] / g0[m]));
         BatchSolver::PcgOut po;
         if (f64) {
             block_jacobi<double, double><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(
                 h.dm, static_cast<double*>(K), mask, static_cast<double*>(dinv), V);
-            po = B.pcg<double>(K, static_cast<double*>(dinv), K, true, mask, rhs, dir, tol, act, o.cg_max_iterations, 0);
+            po = B.pcg<double>(K, static_cast<double*>(dinv), K, true, mask, rhs, bnorm, dir, tol, act, o.cg_max_iterations, 0);
         } else {
             block_jacobi<float, float><<<grid(static_cast<size_t>(V)), kThreads, 0, s>>>(
                 h.dm, static_cast<float*>(K), mask, static_cast<float*>(dinv), V);
-            po = B.pcg<float>(K, static_cast<float*>(dinv), K, false, mask, rhs, dir, tol, act, o.cg_max_iterations, 3);
+            po = B.pcg<float>(K, static_cast<float*>(dinv), K, false, mask, rhs, bnorm, dir, tol, act, o.cg_max_iterations, 3);
         }
         R.cg_iterations += po.iters;
         // A mesh whose direction is not a descent direction (negative curvature at the first PCG
         // step) takes the steepest-descent direction -g for this iteration.
-        auto gds = B.stats(g, dir, mask);
+        const auto feasible = [&]() {
+            launch_feasible(h.dm, x, dir, bm, nfeas, al, h.status_word(), s, d.elem, d.emesh, d.exact);
+            seg_elem<<<M, kSegThreads, 0, s>>>(d.elem, d.eoff, 1, B.values(BatchSolver::kStep));
+            return h.take_status();
+        };
+        B.stats_async(g, dir, mask, BatchSolver::kOther);
+        unsigned feasible_status = feasible();
+        auto gds = B.read(BatchSolver::kOther);
         bool fallback = false;
         for (int m = 0; m < M; ++m) {
             take[m] = act[m] && !(gds[4 * m] < 0.0 && std::isfinite(gds[4 * m]));
@@ -2371,15 +2417,14 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
         if (fallback) {
             B.up(d.take, take);
             seg_take<<<grid(n), kThreads, 0, s>>>(dir, rhs, d.take, d.mov, n);
-            gds = B.stats(g, dir, mask);
+            B.stats_async(g, dir, mask, BatchSolver::kOther);
+            feasible_status = feasible();
+            gds = B.read(BatchSolver::kOther);
         }
         for (int m = 0; m < M; ++m) gd[m] = gds[4 * m];
         // Line search per mesh from its feasible step.
-        launch_feasible(h.dm, x, dir, bm, nfeas, al, h.status_word(), s, d.elem, d.emesh, d.exact);
-        seg_elem<<<M, 256, 0, s>>>(d.elem, d.eoff, 1, d.amin);
-        raise_status(h.take_status());
-        std::vector<double> amin;
-        B.down(amin, d.amin, M);
+        raise_status(feasible_status);
+        const std::vector<double> amin = B.read(BatchSolver::kStep, 1);
         for (int m = 0; m < M; ++m) {
             pending[m] = act[m];
             alpha[m] = act[m] ? amin[m] : 0.0;
@@ -2392,7 +2437,10 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
             for (int m = 0; m < M; ++m) a[m] = pending[m] ? alpha[m] : 0.0;
             B.up(d.alpha, a);
             seg_axpy<<<grid(n), kThreads, 0, s>>>(x, d.alpha, d.mov, dir, trial, diff, n);
-            const auto mv = B.stats(diff, nullptr, nullptr);
+            B.stats_async(diff, nullptr, nullptr, BatchSolver::kOther);
+            B.energies_async(trial, f, nullptr, LPG_HESSIAN_NONE, LPG_PRECISION_F64, nullptr);
+            raise_status(h.take_status());
+            const auto mv = B.read(BatchSolver::kOther);
             for (int m = 0; m < M; ++m)
                 if (pending[m] && !(mv[4 * m + 2] > 0)) {
                     pending[m] = 0;
@@ -2401,7 +2449,7 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
                     secs[m] = elapsed();
                 }
             ++R.line_search_evaluations;
-            std::vector<double> Et = B.energies(trial, f, nullptr, LPG_HESSIAN_NONE, LPG_PRECISION_F64, nullptr);
+            const std::vector<double> Et = B.energies_read(f);
             for (int m = 0; m < M; ++m) {
                 take[m] = 0;
                 if (!pending[m]) continue;

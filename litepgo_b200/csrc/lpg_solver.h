@@ -75,9 +75,16 @@ struct lpg_fem {
         unsigned done;   // block counter of the energy sum (zero between launches)
     };
     EvalResult* host_result = nullptr;
-    // The rest of the pinned block: landing places of the solvers' read-backs (sums, PCG state).
-    double* host_sums() { return reinterpret_cast<double*>(host_result) + 8; }
-    void* host_pcg() { return reinterpret_cast<double*>(host_result) + 16; }
+    // The rest of the pinned block: where the solvers' kernels write what the host reads after the next
+    // synchronisation (sums, 4 values per slot; the feasible step and the moved flag; the PCG state).
+    double* host_sums(int slot) { return reinterpret_cast<double*>(host_result) + 8 + 4 * slot; }
+    double* host_step() { return reinterpret_cast<double*>(host_result) + 40; }
+    int* host_moved() { return reinterpret_cast<int*>(reinterpret_cast<double*>(host_result) + 41); }
+    void* host_pcg() { return reinterpret_cast<double*>(host_result) + 64; }
+    // Per-mesh values of the batched solves, likewise written by kernels; grows, freed with the handle.
+    double* host_block = nullptr;
+    size_t host_block_size = 0;
+    double* host_values(size_t count);
     EvalResult* result() { return static_cast<EvalResult*>(d_result.ptr); }
     double* energy_word() { return &result()->energy; }
     unsigned* status_word() { return &result()->status; }
