@@ -395,7 +395,7 @@ def run_ours(args):
     ms = max_over_ranks(ms, world)
     ms_per_step = ms / args.steps
     value = whole_job_rate(T * args.steps, ms * 1e-3, world)
-    gpu_launches = 3 * args.steps  # per step: the assembly kernel and the two-stage energy sum
+    gpu_launches = args.steps  # per step: the assembly kernel, which sums the energy too
 
     # Roofline of the assembly kernel: CUDA events on its launching stream, L2 flushed between launches.
     ma, me = ctypes.c_double(), ctypes.c_double()

@@ -412,15 +412,15 @@ typedef struct {
  * num_meshes independent tet meshes (a tet handle; others fail with LPG_EINVAL) stored in one
  * handle as contiguous vertex ranges
  * [vertex_offsets[m], vertex_offsets[m+1]) and element ranges [element_offsets[m],
- * element_offsets[m+1]) (every element inside its mesh's vertices). Assembly and SpMV run once
- * over all meshes; every mesh has its own stop test, PCG scalars (one block-Jacobi PCG per mesh,
- * in lockstep), feasible step and line search, as lpg_newton_solve has for one mesh. Where a
- * mesh's PCG direction is not a descent direction, that iteration takes -g for the mesh instead
- * of lpg_newton_solve's diagonal shifts. With exact_below the Exact Hessian is used once every
- * unfinished mesh meets the threshold. fixed_dofs, f_ext, x0 and x_out are over the whole
- * handle. per_mesh[num_meshes] receives the per-mesh outcomes; result (may be NULL) the totals
- * (status = the worst mesh's, iterations = Newton iterations run, cg_iterations = lockstep PCG
- * iterations, energy = the sum). A finished mesh is skipped by the later iterations' assembly,
+ * element_offsets[m+1]) (every element inside its mesh's vertices). Assembly runs once over
+ * all meshes; every mesh has its own stop test, block-Jacobi PCG (side by side), feasible step
+ * and line search, as lpg_newton_solve has for one mesh. Where a mesh's PCG direction is not a
+ * descent direction, that iteration takes -g for the mesh instead of lpg_newton_solve's diagonal
+ * shifts. With exact_below the Exact Hessian is used once every unfinished mesh meets the
+ * threshold. fixed_dofs, f_ext, x0 and x_out are over the whole handle. per_mesh[num_meshes]
+ * receives the per-mesh outcomes; result (may be NULL) the totals (status = the worst mesh's,
+ * iterations = Newton iterations run, cg_iterations = PCG iterations of each solve's slowest
+ * mesh, energy = the sum). A finished mesh is skipped by the later iterations' assembly,
  * projection, feasible step and PCG.
  */
 int lpg_batch_newton_solve(lpg_fem_t h, int num_meshes, const int32_t* vertex_offsets, const int32_t* element_offsets,

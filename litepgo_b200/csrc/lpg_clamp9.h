@@ -1,8 +1,8 @@
 // Eigenvalue clamp of a symmetric 9x9 matrix, M -> V max(Lambda, 0) V^T, by the cyclic Jacobi
 // method in a parallel (round-robin) ordering: the projected Hessian's clamp of a tet's tangent in
-// the q basis (mesh_energy.cpp:16-27 clamps each element Hessian's eigenvalues at zero). One
-// thread per matrix on the GPU (clamp_kernel); compiled for the host as well, where a test checks
-// it against an eigensolver.
+// the q basis (mesh_energy.cpp:16-27 clamps each element Hessian's eigenvalues at zero) where the
+// faster clamp of lpg_tri9.h gives up. One thread per matrix on the GPU (clamp9_jacobi); compiled for
+// the host as well, where a test checks it against an eigensolver.
 #pragma once
 #ifndef __CUDA_ARCH__
 #include <cmath>
@@ -52,10 +52,9 @@ template <typename R> LPG_C9 R c9_rsqrt(R x) {
 // A is kept relabelled by the round, A_cur(i, j) = A((i + r) mod 9, (j + r) mod 9), so every
 // round rotates the fixed pairs (1, 8), (2, 7), (3, 6), (4, 5) of A_cur with literal register
 // indices; after the round A_cur is shifted by one label. The loop over rounds therefore stays
-// a loop (a fully unrolled sweep of nine rounds overflows the instruction cache). V (register
-// array, VREG) is shifted with A; V in shared memory is addressed with the round's offset.
-template <typename R, bool VREG, typename VA>
-LPG_C9 void jacobi_round(R (&A)[45], VA& V, const int rd) {
+// a loop (a fully unrolled sweep of nine rounds overflows the instruction cache). V is shifted with A.
+template <typename R>
+LPG_C9 void jacobi_round(R (&A)[45], R (&V)[81]) {
     R c[4], sn[4], t[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -99,16 +98,11 @@ LPG_C9 void jacobi_round(R (&A)[45], VA& V, const int rd) {
         A[sym9(P, P)] -= t[k] * apq;
         A[sym9(Q, Q)] += t[k] * apq;
         A[sym9(P, Q)] = R(0);
-        int vp_col = P, vq_col = Q;
-        if constexpr (!VREG) {
-            vp_col = P + rd >= 9 ? P + rd - 9 : P + rd;
-            vq_col = Q + rd >= 9 ? Q + rd - 9 : Q + rd;
-        }
 #pragma unroll
         for (int x = 0; x < 9; ++x) {
-            const R vp = V[9 * x + vp_col], vq = V[9 * x + vq_col];
-            V[9 * x + vp_col] = c[k] * vp - sn[k] * vq;
-            V[9 * x + vq_col] = sn[k] * vp + c[k] * vq;
+            const R vp = V[9 * x + P], vq = V[9 * x + Q];
+            V[9 * x + P] = c[k] * vp - sn[k] * vq;
+            V[9 * x + Q] = sn[k] * vp + c[k] * vq;
         }
     }
     // Relabel for the next round: A_next(i, j) = A_cur(i + 1, j + 1) (indices mod 9).
@@ -119,21 +113,20 @@ LPG_C9 void jacobi_round(R (&A)[45], VA& V, const int rd) {
     for (int i = 0; i < 9; ++i)
 #pragma unroll
         for (int j = i; j < 9; ++j) A[sym9(i, j)] = B[sym9((i + 1) % 9, (j + 1) % 9)];
-    if constexpr (VREG) {
 #pragma unroll
-        for (int x = 0; x < 9; ++x) {
-            const R v0 = V[9 * x];
+    for (int x = 0; x < 9; ++x) {
+        const R v0 = V[9 * x];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) V[9 * x + j] = V[9 * x + j + 1];
-            V[9 * x + 8] = v0;
-        }
+        for (int j = 0; j < 8; ++j) V[9 * x + j] = V[9 * x + j + 1];
+        V[9 * x + 8] = v0;
     }
 }
 
-// The clamp of the packed upper triangle A (45 values), in place: A <- V max(Lambda, 0) V^T. V
-// is 81 values of scratch (a register array when VREG; in FP64 on the GPU, shared memory).
-template <typename R, bool VREG, typename VA>
-LPG_C9 void clamp9_packed(R (&A)[45], VA& V) {
+// The clamp of the packed upper triangle A (45 values), in place: A <- V max(Lambda, 0) V^T. V is 81 values
+// of scratch, in registers as A is (the bool says so to a caller that spells it out).
+template <typename R, bool kRegisters = true>
+LPG_C9 void clamp9_packed(R (&A)[45], R (&V)[81]) {
+    static_assert(kRegisters, "V is a register array");
     R amax = 0;
 #pragma unroll
     for (int t = 0; t < 45; ++t) amax = C9F(fmax)(amax, C9F(fabs)(A[t]));
@@ -159,7 +152,7 @@ LPG_C9 void clamp9_packed(R (&A)[45], VA& V) {
             for (int c = r + 1; c < 9; ++c) off += A[sym9(r, c)] * A[sym9(r, c)];
         if (!(off > thr)) break;
 #pragma unroll 1
-        for (int rd = 0; rd < 9; ++rd) jacobi_round<R, VREG>(A, V, rd);
+        for (int rd = 0; rd < 9; ++rd) jacobi_round<R>(A, V);
     }
     R lam[9];
 #pragma unroll
