@@ -392,7 +392,10 @@ void build_tet_clusters(HostPlan& p, const int32_t* tets, const std::vector<int3
         std::stable_sort(diag.begin(), diag.end(), by_count);
         std::stable_sort(edge.begin(), edge.end(), by_count);
         const size_t ent0 = p.tc_ents.size();
-        for (const auto* group : {&diag, &edge}) {
+        int ndent = 0;
+        for (const Item& it : diag) ndent += it.cnt;
+        p.tc_dent.push_back((ndent + 7) & ~7);
+        for (const auto* group : {&diag, &edge})
             for (const Item& it : *group) {
                 const size_t first = p.tc_ents.size() - ent0;
                 if (first >= (1u << 20) || it.cnt >= (1 << 12))
@@ -401,8 +404,6 @@ void build_tet_clusters(HostPlan& p, const int32_t* tets, const std::vector<int3
                                   {it.w0, it.w1, static_cast<uint32_t>(first) | (static_cast<uint32_t>(it.cnt) << 20), it.w3});
                 p.tc_ents.insert(p.tc_ents.end(), pool.begin() + it.start, pool.begin() + it.start + it.cnt);
             }
-            if (group == &diag) p.tc_dent.push_back(static_cast<int32_t>((p.tc_ents.size() - ent0 + 7) & ~size_t(7)));
-        }
         while (p.tc_ents.size() % 8 != 0) p.tc_ents.push_back(0); // 16-byte aligned per cluster
         p.tc_ndiag.push_back(static_cast<int32_t>(diag.size()));
         p.tc_el_ptr.push_back(static_cast<int32_t>(p.tc_els.size()));
