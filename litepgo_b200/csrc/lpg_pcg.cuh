@@ -3,27 +3,35 @@
 // helpers and PcgState it uses.
 //
 // The launch-per-step iteration (spmv_sell and pcg_update in a graph) is bound at these sizes by its two
-// launches and its chain of gathers and reductions through L2. Here a lane keeps its row's x, r, p, s and
+// launches and its chain of gathers and reductions through L2. Here a lane keeps its row's x, r, z, p and
 // preconditioner block in registers for the whole solve, and a block its chunks' matrix values as far as
 // they fit (both triangles, borrowed blocks transposed once): the first slots of a warp in registers, up to
 // 16 more in shared memory, the rest read from L2. What crosses blocks is z and three sums:
-// - z = D r of the block's rows goes to shared memory, and to L2 for the blocks that have it as a neighbour
-//   (their halo). A vertex's z is one 16-byte word (two in FP64) that carries the iteration's number, so a
-//   reader polls the word itself: no fence, no flag, one L2 round trip.
-// - CG in the form with one reduction (Chronopoulos and Gear, below): gamma, delta and r.r of a block are
-//   published as numbered words too, and 15 warps of every block poll all of them and add them in block
-//   order, so that all blocks hold bitwise the same sums and results do not depend on scheduling.
-// Between the two exchanges every block has read what it waits for, so z is kept once and the sums twice
-// (by the number's parity). An iteration is then two L2 round trips, the products and FP64 latency.
+// - z = D r of the block's rows goes to L2 for the blocks that have it as a neighbour (their halo), which form
+//   p = z + beta p of the halo themselves, bit by bit as its owner does; p of both is in shared memory. A
+//   vertex's z is one 16-byte word (two in FP64) that carries the iteration's number, so a reader polls the
+//   word itself: no fence, no flag, one L2 round trip.
+// - The sums r.z and r.r of a block travel at the same time as z, then p.Ap: published as numbered words too;
+//   warps of every block poll all of them and add them in block order, so that all blocks hold bitwise the
+//   same sums and results do not depend on scheduling.
+// Every block has read what an exchange brings before it publishes in the next one, and a word is rewritten
+// only after a whole exchange in between: one copy of each suffices. An iteration is then two L2 round trips,
+// the products and FP64 latency.
+//
+// The recurrences are those of the launches per step. The form with one reduction (Chronopoulos and Gear,
+// 1989), which takes p.Ap from z.Az and the sums before and A p from a recurrence, is no faster here, since p
+// of the halo costs no exchange, and not stable enough in FP32: on blocks with a Poisson ratio of 0.4999 it
+// took 60 % more iterations, from 0.499975 on it lost the sign of p.Ap, and so it did on columns of 60 cubes.
 //
 // A batch of meshes is one launch too: every mesh has blocks of its own (one block exchanges nothing), its
 // own sums, tolerance and end, where the launches per step run all meshes in lockstep to the slowest.
 //
-// Measured per iteration, B200 (launch-per-step, then this kernel): 648 vertices FP64 14.2 and 4.2 us;
-// 4,896 FP64 16.4 and 6; 62,197 FP32 15.6 and 8.8, where the products (18 slots a lane) and the wait for
-// the slowest block are half; lockstep of 48 boxes of 4 to 16 cubes a side, 64,000 vertices, 24, and all
-// their solves at once 7.8. A build that spilled 300 bytes a thread took 14 at 62,197: beside 227 KB of
-// shared memory the L1 holds no spills, hence KR, G, the scalars in shared memory and one word per lane.
+// Measured per iteration, B200 (launch-per-step, then this kernel): 648 vertices FP64 14.2 and 4.0 us; 4,896
+// FP64 16.4 and 5.4; 62,197 FP32 15.6 and 7.5, where the products (18 slots a lane) and the wait for the
+// slowest block are half; 48 boxes of 4 to 16 cubes, 64,000 vertices, 24 in lockstep and 9.4 side by side. Three
+// slots of a lane are in registers in FP32 (KR), which spills 56 bytes: with two the slowest block waits for
+// one more slot from L2 (a Newton solve of 62,197 vertices 90 ms instead of 82), with four the spills cost more
+// (86). Beside 227 KB of shared memory there is hardly any L1 to hold them, hence G and one word per lane.
 #pragma once
 
 namespace lpg {
@@ -166,21 +174,28 @@ template <> struct Pending<double> {
     }
 };
 
-// Values per staged vertex: float4 in FP32, three doubles in FP64.
+// Values per vertex of p in shared memory: float4 in FP32, three doubles in FP64.
 template <typename R> constexpr int pcg_stride() { return sizeof(R) == 4 ? 4 : 3; }
-// Shared memory of the staged z (own rows and halo) and the halo's vertex list.
-template <typename R> constexpr size_t pcg_z_bytes(int rows, int halo) {
-    return (static_cast<size_t>(rows + halo) * pcg_stride<R>() * sizeof(R) + halo * sizeof(int32_t) + 15) / 16 * 16;
+// Shared memory of the split rows' parts, which the halo's z is staged in as it arrives (3 values a vertex).
+template <typename R> constexpr size_t pcg_stage_bytes(int halo) {
+    constexpr size_t parts = 3 * 32 * kPcgWarps * sizeof(R);
+    const size_t z = (3 * halo * sizeof(R) + 15) / 16 * 16;
+    return z > parts ? z : parts;
+}
+// Shared memory of p (own rows and halo), of the halo's vertex list and of the parts.
+template <typename R> constexpr size_t pcg_p_bytes(int rows, int halo, bool staged) {
+    return (static_cast<size_t>(rows + halo) * pcg_stride<R>() * sizeof(R) + halo * sizeof(int32_t) + 15) / 16 * 16 +
+           pcg_stage_bytes<R>(staged ? halo : 0);
 }
 // Shared memory of one slot of a chunk (32 blocks).
 template <typename R> constexpr size_t pcg_slot_bytes() { return 32 * 9 * sizeof(R); }
-constexpr size_t kPcgFixed = (4 * kPcgWarps + 26 + 3 * 32 * kPcgWarps) * sizeof(double); // sums, split rows' parts
+constexpr size_t kPcgFixed = (2 * kPcgWarps + 22) * sizeof(double); // sums and scalars
 
 template <typename R> struct PcgArgs {
     const R *val, *dinv, *mask4, *b4;
     R *x4, *z4;
     PcgState* st;     // per group, zero before the launch
-    uint4* words;     // [2][3][blocks of the plan]
+    uint4* words;     // [3][blocks of the plan]
     unsigned* number; // per group: exchanges so far
     const double* tols; // per group, or null: tol
     const int* act;     // per group (0: x = 0 and nothing else), or null
@@ -236,21 +251,15 @@ __device__ __forceinline__ double shfl_xor_add(double keep, double send, int o) 
     return keep + __shfl_xor_sync(0xffffffffu, send, o);
 }
 
-// The iteration is CG with one reduction (Chronopoulos and Gear, "s-step iterative methods for symmetric
-// linear systems", 1989): with w = A z, gamma = r.z and delta = z.w, p^T A p = delta - beta gamma / alpha_old,
-// and A p follows from A z by the recurrence of p itself, s = w + beta s.
 template <typename R>
 __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh m, const PcgPlan plan, const PcgArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int PS = pcg_stride<R>(), KR = sizeof(R) == 4 ? 2 : 1, G = sizeof(R) == 4 ? 3 : 1;
+    constexpr int PS = pcg_stride<R>(), KR = sizeof(R) == 4 ? 3 : 1, G = sizeof(R) == 4 ? 3 : 1;
     constexpr int MS = 16; // most slots of a warp in shared memory (their column indices are in registers)
-    double* red = reinterpret_cast<double*>(smem_raw); // [4 values][warps], then the groups of blocks' sums
-    double* total = red + 4 * kPcgWarps; // [warp]
+    double* red = reinterpret_cast<double*>(smem_raw); // [2 values][warps]
+    double* total = red + 2 * kPcgWarps; // [warp]: the sums of 32 blocks
     volatile int* s_lost = reinterpret_cast<volatile int*>(total + 16);
-    // Scalars of thread 0: 1 / gamma and 1 / alpha of the iteration before (by parity), then its gamma and
-    // p.Ap, the squared tolerance and |b|^2.
-    double* scal = total + 18;
-    R* parts = reinterpret_cast<R*>(total + 26); // [warp][3][32]
+    double* scal = total + 18; // 1 / (r.z of the iteration before), the squared tolerance, |b|^2
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int block = a.first_block + blockIdx.x, grp = plan.of_block[block];
     const PcgGroup g = plan.groups[grp];
@@ -267,9 +276,12 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
         return;
     }
     const int L = plan.halo_count[block], own_rows = 32 * nc;
-    R* zs = reinterpret_cast<R*>(smem_raw + kPcgFixed);
-    int32_t* list = reinterpret_cast<int32_t*>(zs + static_cast<size_t>(PS) * (own_rows + L));
-    unsigned char* rest = smem_raw + kPcgFixed + pcg_z_bytes<R>(own_rows, L);
+    const bool staged = kPcgFixed + pcg_p_bytes<R>(own_rows, L, true) <= a.smem;
+    R* parts = reinterpret_cast<R*>(smem_raw + kPcgFixed); // [warp][3][32], or the halo's z [L][3]
+    R* ps = reinterpret_cast<R*>(smem_raw + kPcgFixed + pcg_stage_bytes<R>(staged ? L : 0));
+    int32_t* list = reinterpret_cast<int32_t*>(ps + static_cast<size_t>(PS) * (own_rows + L));
+    const size_t vectors = kPcgFixed + pcg_p_bytes<R>(own_rows, L, staged);
+    unsigned char* rest = smem_raw + vectors;
     // `sub` warps share a chunk (its slots dealt round robin); the first of them owns the rows.
     int sub = 1;
     while (2 * sub * nc <= kPcgWarps && sub < 4) sub *= 2;
@@ -287,7 +299,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
     const auto slots_of = [&](int k) {
         return (m.sell_ptr[c0 + k + 1] - m.sell_ptr[c0 + k] + m.sell_bptr[c0 + k + 1] - m.sell_bptr[c0 + k]) >> 5;
     };
-    const size_t room = (a.smem - kPcgFixed - pcg_z_bytes<R>(own_rows, L)) / pcg_slot_bytes<R>();
+    const size_t room = (a.smem - vectors) / pcg_slot_bytes<R>();
     int cap = 0;
     for (int most = 1 << 12; most > 0; most >>= 1) {
         size_t need = 0;
@@ -333,10 +345,11 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
         }
     }
     for (int i = tid; i < L; i += kPcgThreads) list[i] = plan.halo[static_cast<size_t>(plan.halo_stride) * block + i];
-    for (int i = tid; i < 4 * kPcgWarps; i += kPcgThreads) red[i] = 0.0;
+    for (int i = tid; i < PS * (own_rows + L); i += kPcgThreads) ps[i] = R(0);
+    for (int i = tid; i < 2 * kPcgWarps; i += kPcgThreads) red[i] = 0.0;
     // The row's state.
     const int row = on && part == 0 ? lane_row : -1;
-    R x[3] = {0, 0, 0}, r[3] = {0, 0, 0}, z[3] = {0, 0, 0}, p[3] = {0, 0, 0}, s[3] = {0, 0, 0}, D[6];
+    R x[3] = {0, 0, 0}, r[3] = {0, 0, 0}, z[3] = {0, 0, 0}, p[3] = {0, 0, 0}, D[6];
 #pragma unroll
     for (int t = 0; t < 6; ++t) D[t] = R(0);
     if (row >= 0) {
@@ -356,27 +369,16 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
     unsigned number = __ldcg(a.number + grp);
     if (tid == 0) *s_lost = 0;
     __syncthreads();
-    // z = D r, published under the next iteration's number and put to the block's own rows.
+    // z = D r, published under the next iteration's number.
     const auto publish_z = [&]() {
         ++number;
         z[0] = D[0] * r[0] + D[1] * r[1] + D[2] * r[2];
         z[1] = D[1] * r[0] + D[3] * r[1] + D[4] * r[2];
         z[2] = D[2] * r[0] + D[4] * r[1] + D[5] * r[2];
         if (row >= 0 && blocks > 1) publish3(a.z4 + 4 * static_cast<size_t>(row), z, number);
-        if (on && part == 0) sts3(zs + PS * static_cast<size_t>(32 * ch + lane), z);
     };
-    int iters = 0, breakdown = 0;
-    double rr = 0;
-    bool lost = false;
-    publish_z();
-    for (;;) {
-        if (tid == 0) { // off the path between two exchanges: 1 / gamma and 1 / alpha = p.Ap / gamma
-            double* next = scal + 2 * (iters & 1);
-            const double ig = iters > 0 ? 1.0 / scal[4] : 0.0;
-            next[0] = ig;
-            next[1] = iters > 0 ? scal[5] * ig : 0.0;
-        }
-        // z of the halo, waiting for each word; G words are in flight per thread.
+    // z of the halo, waiting for each word; G words are in flight per thread.
+    const auto each_halo = [&](auto&& use) {
         for (int i0 = tid; i0 < L; i0 += G * kPcgThreads) {
             Pending<R> zv[G];
             unsigned missing = 0;
@@ -397,15 +399,115 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
                         missing &= ~(1u << j);
                         R t[3];
                         zv[j].get(t);
-                        sts3(zs + PS * static_cast<size_t>(own_rows + i0 + j * kPcgThreads), t);
+                        use(i0 + j * kPcgThreads, t);
                     }
             }
+        }
+    };
+    // p = z + beta p of a vertex of the halo, as its owner forms it.
+    const auto advance = [&](int i, const R t[3], R be) {
+        R* at = ps + PS * static_cast<size_t>(own_rows + i);
+        R v[3];
+        lds3(at, v);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) v[e] = fma(be, v[e], t[e]);
+        sts3(at, v);
+    };
+    // The block's sums of NV values, published by warp v as value first + v; then warp v + NV j polls and adds
+    // value v of blocks 32 j to 32 j + 31 (one word a lane: five in flight cost the loop 30 registers).
+    const auto publish_sums = [&](int nv, int first) {
+        if (warp >= nv) return;
+        double b = lane < kPcgWarps ? red[kPcgWarps * warp + lane] : 0.0;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) b = shfl_xor_add(b, b, o);
+        if (lane != 0) return;
+        if (blocks > 1)
+            st_word(a.words + static_cast<size_t>(first + warp) * plan.blocks + block, __double2loint(b), __double2hiint(b), 0u,
+                    number);
+        else
+            total[warp] = b;
+    };
+    const auto poll_sums = [&](int nv, int first) {
+        const int val = warp % nv, from = 32 * (warp / nv);
+        if (blocks <= 1 || from >= blocks) return;
+        double b = 0;
+        if (from + lane < blocks) {
+            const uint4* at = a.words + static_cast<size_t>(first + val) * plan.blocks + g.b0 + from + lane;
+            uint4 u = ld_word(at);
+            for (unsigned spin = 0; u.w != number; ++spin) {
+                if (spin >= kPcgSpins) {
+                    *s_lost = 1;
+                    break;
+                }
+                u = ld_word(at);
+            }
+            b = __hiloint2double(u.y, u.x);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) b = shfl_xor_add(b, b, o);
+        if (lane == 0) total[warp] = b;
+    };
+    static_assert(2 * ((kPcgMaxBlocks + 31) / 32) <= kPcgWarps, "a warp for each value of 32 blocks");
+    const auto sum_of = [&](int nv, int v) {
+        double t = total[v];
+        for (int k = 1; 32 * k < blocks; ++k) t += total[nv * k + v];
+        return t;
+    };
+    int iters = 0, breakdown = 0;
+    double rr = 0, gamma = 1;
+    bool lost = false;
+    publish_z();
+    for (;;) {
+        // gamma = r.z and r.r: over the warp (lanes 0 and 16 end with one each), the block, the group.
+        {
+            double v0 = 0, v1 = 0;
+            if (row >= 0)
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    v0 += static_cast<double>(r[i]) * z[i];
+                    v1 += static_cast<double>(r[i]) * r[i];
+                }
+            const bool up = lane & 16;
+            double t = shfl_xor_add(up ? v1 : v0, up ? v0 : v1, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) t = shfl_xor_add(t, t, o);
+            if (part == 0 && (lane & 15) == 0) red[kPcgWarps * (lane >> 4) + warp] = t;
+        }
+        __syncthreads();
+        publish_sums(2, 0);
+        if (tid == kPcgThreads - 1) scal[0] = 1.0 / gamma; // off the path between two exchanges
+        if (staged)
+            each_halo([&](int i, const R t[3]) {
+#pragma unroll
+                for (int e = 0; e < 3; ++e) parts[3 * static_cast<size_t>(i) + e] = t[e];
+            });
+        poll_sums(2, 0);
+        __syncthreads();
+        gamma = sum_of(2, 0), rr = sum_of(2, 1);
+        lost = *s_lost != 0;
+        if (lost) break;
+        if (iters == 0) {
+            const double tol = a.tols != nullptr ? a.tols[grp] : a.tol;
+            if (tid == 0) scal[1] = tol * tol * rr, scal[2] = rr;
+            if (rr == 0.0 || a.max_iters <= 0) break;
+        } else if (rr <= scal[1] || iters >= a.max_iters || !isfinite(rr)) {
+            break;
+        }
+        const R be = iters > 0 ? static_cast<R>(gamma * scal[0]) : R(0);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) p[i] = fma(be, p[i], z[i]);
+        if (on && part == 0) sts3(ps + PS * static_cast<size_t>(32 * ch + lane), p);
+        if (staged) {
+            for (int i = tid; i < L; i += kPcgThreads) advance(i, parts + 3 * static_cast<size_t>(i), be);
+        } else {
+            each_halo([&](int i, const R t[3]) { advance(i, t, be); });
         }
         __syncthreads();
         R y[3] = {0, 0, 0};
         const auto product = [&](const R k9[9], int at) {
             R v[3];
-            lds3(zs + PS * static_cast<size_t>(at), v);
+            lds3(ps + PS * static_cast<size_t>(at), v);
             y[0] += k9[0] * v[0] + k9[1] * v[1] + k9[2] * v[2];
             y[1] += k9[3] * v[0] + k9[4] * v[1] + k9[5] * v[2];
             y[2] += k9[6] * v[0] + k9[7] * v[1] + k9[8] * v[2];
@@ -437,105 +539,45 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
 #pragma unroll
                     for (int i = 0; i < 3; ++i) y[i] += parts[96 * (warp + k) + 32 * i + lane];
         }
-        // The sums gamma = r.z, delta = z.w and r.r over the block: a transposed tree over the warp (lane
-        // group lane / 8 ends with value lane / 8), then over the warps.
-        double gamma, delta;
         {
-            double v[3] = {0, 0, 0};
+            double v = 0;
             if (row >= 0)
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
                     y[i] = (free >> i) & 1u ? y[i] : R(0);
-                    v[0] += static_cast<double>(r[i]) * z[i];
-                    v[1] += static_cast<double>(z[i]) * y[i];
-                    v[2] += static_cast<double>(r[i]) * r[i];
+                    v += static_cast<double>(p[i]) * y[i];
                 }
-            const bool up = lane & 16, mid = lane & 8;
-            const double k0 = shfl_xor_add(up ? v[2] : v[0], up ? v[0] : v[2], 16);
-            const double k1 = shfl_xor_add(up ? 0.0 : v[1], up ? v[1] : 0.0, 16);
-            double t = shfl_xor_add(mid ? k1 : k0, mid ? k0 : k1, 8);
-            t = shfl_xor_add(t, t, 4);
-            t = shfl_xor_add(t, t, 2);
-            t = shfl_xor_add(t, t, 1);
-            if (part == 0 && (lane & 7) == 0) red[kPcgWarps * (lane >> 3) + warp] = t;
-            __syncthreads();
-            // Warp v < 3 sums the block's value v and publishes it; then warp v + 3 j polls and adds the values
-            // v of blocks 32 j to 32 j + 31 (one word a lane: five in flight cost the loop 30 registers).
-            const int val = warp % 3, from = 32 * (warp / 3);
-            if (from < blocks && from < kPcgMaxBlocks) {
-                static_assert(kPcgWarps == 16 && kPcgMaxBlocks == 160, "15 warps of 32 words");
-                uint4* all = a.words + static_cast<size_t>(3 * (number & 1u) + val) * plan.blocks + g.b0;
-                double b = 0;
-                if (warp < 3) {
-                    b = lane < kPcgWarps ? red[kPcgWarps * warp + lane] : 0.0;
 #pragma unroll
-                    for (int o = 8; o > 0; o >>= 1) b = shfl_xor_add(b, b, o);
-                    if (lane == 0 && blocks > 1) st_word(all + rank, __double2loint(b), __double2hiint(b), 0u, number);
-                }
-                if (blocks > 1) {
-                    b = 0;
-                    if (from + lane < blocks) {
-                        uint4 u = ld_word(all + from + lane);
-                        for (unsigned spin = 0; u.w != number; ++spin) {
-                            if (spin >= kPcgSpins) {
-                                *s_lost = 1;
-                                break;
-                            }
-                            u = ld_word(all + from + lane);
-                        }
-                        b = __hiloint2double(u.y, u.x);
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) b = shfl_xor_add(b, b, o);
-                }
-                if (lane == 0) total[warp] = b;
-            }
-            __syncthreads();
-            gamma = total[0], delta = total[1];
-            for (int k = 1; 32 * k < blocks; ++k) gamma += total[3 * k], delta += total[3 * k + 1];
-            lost = *s_lost != 0;
+            for (int o = 16; o > 0; o >>= 1) v = shfl_xor_add(v, v, o);
+            if (part == 0 && lane == 0) red[warp] = v;
         }
+        __syncthreads();
+        publish_sums(1, 2);
+        poll_sums(1, 2);
+        __syncthreads();
+        const double pAp = sum_of(1, 0);
+        lost = *s_lost != 0;
         if (lost) break;
-        {
-            rr = total[2];
-            for (int k = 1; 32 * k < blocks; ++k) rr += total[3 * k + 2];
-            if (iters == 0) {
-                const double tol = a.tols != nullptr ? a.tols[grp] : a.tol;
-                if (tid == 0) scal[6] = tol * tol * rr, scal[7] = rr;
-                if (rr == 0.0 || a.max_iters <= 0) break;
-            } else if (rr <= scal[6] || iters >= a.max_iters || !isfinite(rr)) {
-                break;
-            }
-        }
-        const double beta = gamma * scal[2 * (iters & 1)];
-        const double pAp = fma(-beta * gamma, scal[2 * (iters & 1) + 1], delta);
         if (!(pAp > 0.0) || !isfinite(pAp)) {
             breakdown = 1;
             if (iters == 0 && a.first_direction)
 #pragma unroll
-                for (int i = 0; i < 3; ++i) x[i] = z[i];
+                for (int i = 0; i < 3; ++i) x[i] = p[i];
             break;
         }
-        const double alpha = gamma / pAp;
-        const R al = static_cast<R>(alpha), be = static_cast<R>(beta);
+        const R al = static_cast<R>(gamma / pAp);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            s[i] = y[i] + be * s[i];
-            r[i] = r[i] - al * s[i];
-            p[i] = z[i] + be * p[i];
-        }
+        for (int i = 0; i < 3; ++i) r[i] = fma(-al, y[i], r[i]);
         publish_z();
 #pragma unroll
-        for (int i = 0; i < 3; ++i) x[i] += al * p[i]; // while the words travel
+        for (int i = 0; i < 3; ++i) x[i] = fma(al, p[i], x[i]); // while the words travel
         ++iters;
-        if (tid == 0) scal[4] = gamma, scal[5] = pAp;
     }
     if (row >= 0) st4(a.x4 + 4 * static_cast<size_t>(row), x[0], x[1], x[2]);
     if (rank == 0 && tid == 0) {
         PcgState* st = a.st + grp;
         st->rr = rr;
-        st->bb = scal[7];
+        st->bb = scal[2];
         st->iters = iters;
         st->breakdown = breakdown;
         st->done = 1;

@@ -611,7 +611,7 @@ namespace {
 inline int grid(size_t n, int threads = kThreads) { return static_cast<int>((n + threads - 1) / threads); }
 
 void clear_words(lpg_fem& h, PcgPlanStore& P) {
-    LPG_CUDA(cudaMemsetAsync(P.words.ptr, 0, 6 * sizeof(uint4) * P.blocks + sizeof(unsigned) * P.groups, h.stream));
+    LPG_CUDA(cudaMemsetAsync(P.words.ptr, 0, 3 * sizeof(uint4) * P.blocks + sizeof(unsigned) * P.groups, h.stream));
     LPG_CUDA(cudaMemsetAsync(P.z.ptr, 0, 4 * sizeof(double) * static_cast<size_t>(h.dm.V), h.stream));
 }
 
@@ -638,7 +638,7 @@ void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, i
         if (g.c1 - g.c0 > kPcgWarps) return false;
         const HostPlan& p = h.plan;
         const size_t slots = (p.sell_ptr[g.c1] - p.sell_ptr[g.c0] + p.sell_bptr[g.c1] - p.sell_bptr[g.c0]) / 32;
-        return kPcgFixed + pcg_z_bytes<double>(32 * (g.c1 - g.c0), 0) + slots * pcg_slot_bytes<double>() <=
+        return kPcgFixed + pcg_p_bytes<double>(32 * (g.c1 - g.c0), 0, true) + slots * pcg_slot_bytes<double>() <=
                static_cast<size_t>(optin);
     };
     const auto blocks_of = [&](const PcgGroup& g, int per) { return resident(g) ? 1 : (g.c1 - g.c0 + per - 1) / per; };
@@ -682,7 +682,7 @@ void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, i
     int rows = 0; // of the largest block
     for (const PcgGroup& g : groups)
         for (int b = 0; b < g.blocks; ++b) rows = std::max(rows, 32 * (pcg_first_chunk(g, b + 1) - pcg_first_chunk(g, b)));
-    if (rows + P.stride >= 65536 || !fits(pcg_z_bytes<float>(rows, P.stride))) return;
+    if (rows + P.stride >= 65536 || !fits(pcg_p_bytes<float>(rows, P.stride, false))) return;
     pcg_plan_kernel<<<P.blocks, kPcgThreads, bits, s>>>(
         m, dg, dof, pos, P.halo.as<int32_t>(static_cast<size_t>(P.blocks) * P.stride), P.stride, count,
         P.own.as<uint16_t>(std::max<size_t>(h.plan.sell_col.size(), 1)),
@@ -690,10 +690,10 @@ void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, i
     LPG_CUDA(cudaGetLastError());
     // The exchange's words, the groups' numbers, and z's words. Nothing else writes them, so what a solve
     // finds there carries an older number than any that it waits for.
-    P.words.ensure(6 * sizeof(uint4) * P.blocks + sizeof(unsigned) * P.groups);
+    P.words.ensure(3 * sizeof(uint4) * P.blocks + sizeof(unsigned) * P.groups);
     P.z.ensure(4 * sizeof(double) * static_cast<size_t>(m.V));
     clear_words(h, P);
-    P.state = fits(pcg_z_bytes<double>(rows, P.stride)) ? 2 : 1;
+    P.state = fits(pcg_p_bytes<double>(rows, P.stride, false)) ? 2 : 1;
 }
 
 // The solve of every group of plan P, one cooperative launch for as many as run at once: x4 from b4, the
@@ -704,7 +704,7 @@ template <typename R> void launch_pcg(lpg_fem& h, PcgPlanStore& P, PcgArgs<R> a)
     LPG_CUDA(cudaFuncSetAttribute(pcg_solve_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     a.z4 = static_cast<R*>(P.z.ptr);
     a.words = static_cast<uint4*>(P.words.ptr);
-    a.number = reinterpret_cast<unsigned*>(a.words + 6 * static_cast<size_t>(P.blocks));
+    a.number = reinterpret_cast<unsigned*>(a.words + 3 * static_cast<size_t>(P.blocks));
     a.smem = static_cast<size_t>(optin);
     PcgPlan plan;
     plan.groups = static_cast<const PcgGroup*>(P.group.ptr);
