@@ -171,6 +171,12 @@ int lpg_fem_create_hex_hermite(int num_vertices, const double* X, int num_cells,
 /* Uses `stream` (a cudaStream_t) for all later work of this handle; NULL = the handle's own stream. */
 int lpg_fem_set_stream(lpg_fem_t h, void* stream);
 
+/*
+ * How often a block of a solver kernel polls for another block's data before it gives up; the solve
+ * then returns LPG_ECUDA and the handle stays usable. 2^22 at first, some seconds.
+ */
+int lpg_fem_set_poll_limit(lpg_fem_t h, uint32_t polls);
+
 /* Sizes: vertices, tets, DOFs (3V), nnzb (3x3 blocks) and nnz (= 9 nnzb). Any pointer may be NULL. */
 int lpg_fem_sizes(lpg_fem_t h, int* num_vertices, int* num_tets, int* num_dofs, int64_t* nnzb, int64_t* nnz);
 

@@ -634,6 +634,13 @@ int lpg_fem_set_stream(lpg_fem_t h, void* stream) {
     });
 }
 
+int lpg_fem_set_poll_limit(lpg_fem_t h, uint32_t polls) {
+    return guarded([&] {
+        if (!h) fail(LPG_EINVAL, "null handle");
+        h->pcg_polls = polls;
+    });
+}
+
 int lpg_fem_sizes(lpg_fem_t h, int* V, int* T, int* n, int64_t* nnzb, int64_t* nnz) {
     return guarded([&] {
         if (!h) fail(LPG_EINVAL, "null handle");

@@ -39,7 +39,6 @@ namespace {
 
 constexpr int kPcgThreads = 512, kPcgWarps = kPcgThreads / 32;
 constexpr int kPcgMaxBlocks = 160;     // five slots per polling lane
-constexpr unsigned kPcgSpins = 1u << 22; // polls of one exchange before it gives up (seconds)
 
 // One linear system of a launch: a mesh's chunks and vertices (a chunk at a mesh's ends may hold rows of its
 // neighbours, which are passed over) and the blocks that work on it. Groups know nothing of one another.
@@ -201,6 +200,7 @@ template <typename R> struct PcgArgs {
     const int* act;     // per group (0: x = 0 and nothing else), or null
     double tol;
     int max_iters;
+    unsigned polls;         // of one word before the block gives up
     int first_block;        // the plan's first block of this launch
     bool first_direction;   // on negative curvature at the first step, x is the preconditioned residual
     size_t smem;
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
             for (int j = 0; j < G; ++j)
                 if (i0 + j * kPcgThreads < L) missing |= 1u << j;
             for (unsigned spin = 0; missing != 0; ++spin) {
-                if (spin >= kPcgSpins) {
+                if (spin >= a.polls) {
                     *s_lost = 1;
                     break;
                 }
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
             const uint4* at = a.words + static_cast<size_t>(first + val) * plan.blocks + g.b0 + from + lane;
             uint4 u = ld_word(at);
             for (unsigned spin = 0; u.w != number; ++spin) {
-                if (spin >= kPcgSpins) {
+                if (spin >= a.polls) {
                     *s_lost = 1;
                     break;
                 }

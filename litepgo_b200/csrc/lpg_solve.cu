@@ -706,6 +706,7 @@ template <typename R> void launch_pcg(lpg_fem& h, PcgPlanStore& P, PcgArgs<R> a)
     a.words = static_cast<uint4*>(P.words.ptr);
     a.number = reinterpret_cast<unsigned*>(a.words + 3 * static_cast<size_t>(P.blocks));
     a.smem = static_cast<size_t>(optin);
+    a.polls = h.pcg_polls;
     PcgPlan plan;
     plan.groups = static_cast<const PcgGroup*>(P.group.ptr);
     plan.of_block = static_cast<const int32_t*>(P.of_block.ptr);
@@ -1095,8 +1096,7 @@ struct Solver {
             cudaGraphDestroy(g);
             for (int i = 0; i < kKey; ++i) h.pcg_graph_key[i] = key[i];
         }
-        cudaEvent_t ev;
-        LPG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        ScopedEvent ev(cudaEventDisableTiming);
         double rnorm = bnorm;
         for (int ref = 0; ref <= max_refine; ++ref) {
             const double inner_tol = std::min(0.5, std::max(tol * bnorm / rnorm, sizeof(R) == 4 ? 1e-6 : 1e-14));
@@ -1158,7 +1158,6 @@ struct Solver {
             out.rel = rnorm / bnorm;
             if (out.breakdown || !(rnorm > tol * bnorm) || out.iters >= max_iters || !std::isfinite(rnorm)) break;
         }
-        cudaEventDestroy(ev);
         return out;
     }
 };
@@ -1296,9 +1295,7 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
         if (terms && terms->on_iteration && terms->on_iteration(&step, terms->user) != 0)
             fail(LPG_ESTOPPED, "newton_solve: the on_iteration callback stopped the solve");
     };
-    cudaEvent_t ev0, ev1;
-    LPG_CUDA(cudaEventCreate(&ev0));
-    LPG_CUDA(cudaEventCreate(&ev1));
+    ScopedEvent ev0, ev1;
     LPG_CUDA(cudaEventRecord(ev0, s));
     double* x = h.s_x.as<double>(std::max<size_t>(n, 1));
     double* g = h.s_g.as<double>(2 * std::max<size_t>(n, 1));
@@ -1339,8 +1336,6 @@ void newton_solve(lpg_fem& h, const int32_t* fixed, int nfixed, const double* f_
         else
             LPG_CUDA(cudaMemcpyAsync(x_out, x, n * sizeof(double), cudaMemcpyDeviceToHost, s));
         LPG_CUDA(cudaStreamSynchronize(s));
-        cudaEventDestroy(ev0);
-        cudaEventDestroy(ev1);
         if (res) *res = R;
     };
     if (nfree == 0) {
@@ -2117,8 +2112,7 @@ struct BatchSolver {
             cudaGraphDestroy(g);
             for (int i = 0; i < 12; ++i) h.batch_graph_key[i] = key[i];
         }
-        cudaEvent_t ev;
-        LPG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        ScopedEvent ev(cudaEventDisableTiming);
         std::vector<double> itol(M);
         std::vector<int> done, iters, brk;
         const PcgState* states = reinterpret_cast<const PcgState*>(values(kState));
@@ -2196,7 +2190,6 @@ struct BatchSolver {
             }
             if (!any || used >= max_iters) break;
         }
-        cudaEventDestroy(ev);
         return out;
     }
 };

@@ -23,6 +23,16 @@ struct DeviceBuffer {
 
 void raise_status(unsigned st);
 
+// A CUDA event that does not outlive the call that made it.
+struct ScopedEvent {
+    cudaEvent_t e = nullptr;
+    explicit ScopedEvent(unsigned flags = cudaEventDefault) { LPG_CUDA(cudaEventCreateWithFlags(&e, flags)); }
+    ~ScopedEvent() { cudaEventDestroy(e); }
+    ScopedEvent(const ScopedEvent&) = delete;
+    ScopedEvent& operator=(const ScopedEvent&) = delete;
+    operator cudaEvent_t() const { return e; }
+};
+
 struct PcgPlanStore {
     int state = 0; // 0 not built, 1 usable in FP32 only, 2 in both precisions, -1 not usable
     int groups = 0, blocks = 0, stride = 0;
@@ -65,6 +75,7 @@ struct lpg_fem {
     // Plans of the one-launch PCG (lpg_pcg.cuh): of the whole mesh, built at the first solve, and of the
     // meshes of a batched solve, built by each call.
     lpg::PcgPlanStore pcg_plan, batch_plan;
+    unsigned pcg_polls = 1u << 22; // polls of one word before a block of it gives up (seconds)
     cudaGraphExec_t batch_graph = nullptr; // the batched (per-mesh) PCG iterations
     const void* batch_graph_key[12] = {};
     // What an evaluation leaves for the host, one 16-byte record on the device (d_result) and its
