@@ -177,6 +177,13 @@ int lpg_fem_set_stream(lpg_fem_t h, void* stream);
  */
 int lpg_fem_set_poll_limit(lpg_fem_t h, uint32_t polls);
 
+/*
+ * The PSD projection of hex (8 nodes) and tricubic Hermite (64 nodes) evaluations on its own: `count` symmetric
+ * element Hessians of 3 nodes rows, each as its 3x3 blocks (row-major) of the node pairs a <= b in row order, host
+ * memory. rounds: passes of inverse iteration before the Jacobi method takes over; -1: as in an evaluation.
+ */
+int lpg_project_hessians(int nodes, int count, const double* H, double* out, int rounds);
+
 /* Sizes: vertices, tets, DOFs (3V), nnzb (3x3 blocks) and nnz (= 9 nnzb). Any pointer may be NULL. */
 int lpg_fem_sizes(lpg_fem_t h, int* num_vertices, int* num_tets, int* num_dofs, int64_t* nnzb, int64_t* nnz);
 

@@ -119,6 +119,7 @@ SIGNATURES = [
     ("lpg_fem_destroy", _int, [_vp]),
     ("lpg_fem_set_stream", _int, [_vp, _vp]),
     ("lpg_fem_set_poll_limit", _int, [_vp, ctypes.c_uint32]),
+    ("lpg_project_hessians", _int, [_int, _int, _dp, _dp, _int]),
     ("lpg_fem_sizes", _int, [_vp, ctypes.POINTER(_int), ctypes.POINTER(_int), ctypes.POINTER(_int), _i64p, _i64p]),
     ("lpg_fem_pattern_bsr", _int, [_vp, _ip, _ip]),
     ("lpg_fem_pattern_csc", _int, [_vp, _ip, _ip]),

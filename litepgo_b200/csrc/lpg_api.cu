@@ -721,6 +721,27 @@ int lpg_fem_eval(lpg_fem_t h, const double* u, int io_mem, double* energy, doubl
     });
 }
 
+int lpg_project_hessians(int nodes, int count, const double* H, double* out, int rounds) {
+    return guarded([&] {
+        if (nodes != 8 && nodes != 64) fail(LPG_EINVAL, "lpg_project_hessians: 8 or 64 nodes per element");
+        if (count < 0 || (count > 0 && (!H || !out))) fail(LPG_EINVAL, "lpg_project_hessians: invalid arguments");
+        if (count == 0) return;
+        const size_t n = 9 * static_cast<size_t>(nodes * (nodes + 1) / 2) * count;
+        DeviceBuffer in, res, scratch, status;
+        double* d_in = in.as<double>(n);
+        double* d_out = res.as<double>(n);
+        unsigned* d_status = status.as<unsigned>(1);
+        LPG_CUDA(cudaMemset(d_status, 0, sizeof(unsigned)));
+        LPG_CUDA(cudaMemcpy(d_in, H, n * sizeof(double), cudaMemcpyHostToDevice));
+        launch_projection(nodes, count, d_in, d_out, scratch.as<double>(std::max<size_t>(projection_scratch_doubles(nodes, count), 1)),
+                          rounds < 0 ? kProjectionRounds : rounds, d_status, nullptr);
+        LPG_CUDA(cudaMemcpy(out, d_out, n * sizeof(double), cudaMemcpyDeviceToHost));
+        unsigned st = 0;
+        LPG_CUDA(cudaMemcpy(&st, d_status, sizeof st, cudaMemcpyDeviceToHost));
+        raise_status(st);
+    });
+}
+
 int lpg_fem_deformation_gradients(lpg_fem_t h, const double* u, int io_mem, double* F) {
     return guarded([&] {
         if (!h || !F) fail(LPG_EINVAL, "lpg_fem_deformation_gradients: null argument");

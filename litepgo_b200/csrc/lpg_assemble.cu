@@ -2637,7 +2637,7 @@ using HexEig = WarpEig<24>;
 
 template <typename R>
 __global__ void __launch_bounds__(32 * kHexPsdWarps, 4) hex_psd_kernel(int T, const double* in, R* out,
-                                                                      unsigned* status) {
+                                                                      int rounds, unsigned* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned short s_at[kHexRecord]; // record entry -> row << 8 | column of its upper entry
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2684,7 +2684,7 @@ __global__ void __launch_bounds__(32 * kHexPsdWarps, 4) hex_psd_kernel(int T, co
             }
         }
         __syncwarp();
-        kind = W.project(lane);
+        kind = W.project(lane, rounds);
         if (kind < 0) {
             using J = PsdJacobi<24>;
             static_assert(J::S == S, "one row stride");
@@ -2720,11 +2720,13 @@ __global__ void __launch_bounds__(32 * kHexPsdWarps, 4) hex_psd_kernel(int T, co
     if (lane == 0 && st) atomicOr(status, st);
 }
 // Each element's FP64 record projected into out's records (which may be the same memory).
-template <typename R> void launch_hex_psd(const DevMesh& m, const double* in, R* out, unsigned* status, cudaStream_t s) {
+template <typename R>
+void launch_hex_psd(const DevMesh& m, const double* in, R* out, unsigned* status, cudaStream_t s,
+                    int rounds = kProjectionRounds) {
     const size_t sm = kHexPsdWarps * sizeof(HexEig);
     thread_local LaunchCache cache;
     resident_grid(hex_psd_kernel<R>, 32 * kHexPsdWarps, sm, cache);
-    hex_psd_kernel<R><<<(m.T + kHexPsdWarps - 1) / kHexPsdWarps, 32 * kHexPsdWarps, sm, s>>>(m.T, in, out, status);
+    hex_psd_kernel<R><<<(m.T + kHexPsdWarps - 1) / kHexPsdWarps, 32 * kHexPsdWarps, sm, s>>>(m.T, in, out, rounds, status);
 }
 
 // Feasible step of a hex mesh: at every quadrature point F and dF (the increment's gradient),
@@ -3040,7 +3042,8 @@ __global__ void __launch_bounds__(kHermThreads, 2) hermite_element_kernel(const 
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(BlockEig::kThreads) hermite_psd_kernel(int T, const double* in, R* out,
-                                                                        double* __restrict__ scratch, unsigned* status) {
+                                                                        double* __restrict__ scratch, int rounds,
+                                                                        unsigned* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BlockEig& B = *reinterpret_cast<BlockEig*>(smem_raw);
     __shared__ double s_max[BlockEig::kWarps];
@@ -3069,19 +3072,10 @@ __global__ void __launch_bounds__(BlockEig::kThreads) hermite_psd_kernel(int T, 
             frexp(amax, &ex);
             const double down = ldexp(1.0, -ex);
             up = ldexp(1.0, ex);
-            // Block (a, b), a <= b, entry (i, c) is H(3 a + i, 3 b + c): the blocks of a are consecutive.
-            for (int a = warp; a < 64; a += BlockEig::kWarps) {
-                const double* ra = rec + 9 * (a * 64 - a * (a - 1) / 2);
-                for (int t = lane; t < 9 * (64 - a); t += 32) {
-                    const int b = a + t / 9, ic = t - 9 * (t / 9), r = 3 * a + ic / 3, c = 3 * b + ic % 3;
-                    if (c >= r) B.A[BlockEig::at(c, r)] = down * ra[t];
-                }
-            }
-            __syncthreads();
-            k = B.project(mine, kind);
+            k = B.project(rec, down, mine, rounds, kind);
         }
-        if (kind < 0 || !(amax < INFINITY)) st |= ST_NONFINITE_OUT;
-        if (kind <= 0) {
+        if (!(amax < INFINITY)) st |= ST_NONFINITE_OUT;
+        if (kind == 0) {
             if (static_cast<const void*>(o) != static_cast<const void*>(rec))
                 for (int t = tid; t < kHermiteRecord; t += BlockEig::kThreads) o[t] = static_cast<R>(rec[t]);
         } else {
@@ -3540,10 +3534,12 @@ int hermite_psd_grid(const DevMesh& m) {
     return std::max(1, std::min(m.T, sms));
 }
 template <typename R>
-void launch_hermite_psd(const DevMesh& m, const double* in, R* out, double* scratch, unsigned* status, cudaStream_t s) {
+void launch_hermite_psd(const DevMesh& m, const double* in, R* out, double* scratch, unsigned* status, cudaStream_t s,
+                        int rounds = kProjectionRounds) {
     thread_local LaunchCache cache;
     resident_grid(hermite_psd_kernel<R>, BlockEig::kThreads, sizeof(BlockEig), cache);
-    hermite_psd_kernel<R><<<hermite_psd_grid(m), BlockEig::kThreads, sizeof(BlockEig), s>>>(m.T, in, out, scratch, status);
+    hermite_psd_kernel<R><<<hermite_psd_grid(m), BlockEig::kThreads, sizeof(BlockEig), s>>>(m.T, in, out, scratch, rounds,
+                                                                                     status);
 }
 } // namespace
 
@@ -3633,6 +3629,23 @@ void launch_hex_eval(const DevMesh& m, int precision, bool projected, const doub
     if (a.grad && m.num_unused > 0)
         zero_rows_kernel<<<(m.num_unused + 255) / 256, 256, 0, s>>>(a.grad, m.unused_rows, m.num_unused);
     launch_sum(elemE, m.T, a, s);
+    LPG_CUDA(cudaGetLastError());
+}
+
+size_t projection_scratch_doubles(int nodes, int count) {
+    DevMesh m;
+    m.T = count;
+    return nodes == 64 ? hermite_scratch_doubles(m) : 0;
+}
+
+void launch_projection(int nodes, int count, const double* in, double* out, double* scratch, int rounds,
+                       unsigned* status, cudaStream_t s) {
+    DevMesh m;
+    m.T = count;
+    if (nodes == 8)
+        launch_hex_psd<double>(m, in, out, status, s, rounds);
+    else
+        launch_hermite_psd<double>(m, in, out, scratch, status, s, rounds);
     LPG_CUDA(cudaGetLastError());
 }
 

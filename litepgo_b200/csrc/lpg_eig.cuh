@@ -9,11 +9,14 @@
 //   2. the inertia and the wanted eigenvalues by Sturm counts (Givens' bisection; Wilkinson, The Algebraic
 //      Eigenvalue Problem, 5.39), several points per eigenvalue and pass;
 //   3. their eigenvectors by inverse iteration with the pivoted LU factors of T - lambda I (Wilkinson
-//      5.54) from seeded starts, then modified Gram-Schmidt, twice (eigenvalues of one cluster span its
-//      eigenspace, since their starts differ);
+//      5.54) from seeded starts, then modified Gram-Schmidt, twice. The solves leave the vectors of a multiple
+//      eigenvalue almost parallel (they grow the most along one of its directions), and Gram-Schmidt then
+//      magnifies the residual of what is left; such vectors are solved and orthogonalised again, up to
+//      `rounds` times, until every residual of T x - lambda x is at round-off. Distinct eigenvalues take one
+//      round, a 12-fold one at most three;
 //   4. the reflectors applied to them, and the rank-k update.
-// A residual of T x - lambda x above round-off or a vector that vanishes under Gram-Schmidt sends a hex to
-// the Jacobi iteration of lpg_psd.h, and a Hermite element to other starts.
+// A matrix that is still off then goes to the Jacobi method. Orthonormal vectors with residuals at round-off
+// for as many eigenvalues of one sign as the Sturm counts say there are span their eigenspace.
 #pragma once
 
 #include <cstdint>
@@ -23,6 +26,7 @@
 namespace lpg {
 
 constexpr double kEigEps = 2.220446049250313e-16;
+constexpr double kEigResidual = 1e-13; // accepted residual of an eigenvector, relative to the norm's bound
 
 // Seeded start of an inverse iteration: entry i of vector c, +-[0.5, 1) (SplitMix64 finaliser).
 __device__ __forceinline__ double eig_start(int i, int c) {
@@ -83,8 +87,8 @@ template <int N> struct WarpEig {
 
     // The projection of M (both triangles staged, scaled to max |entry| < 1): on return M holds P with
     // M+ = M_in + P (the return value 1) or M+ = P (2); 0: M is semi-definite (unchanged M+ = M_in);
-    // -1: not accurate, the caller falls back. A team of 32 lanes, all converged.
-    __device__ int project(int lane) {
+    // -1: not accurate after the given rounds, the caller falls back. A team of 32 lanes, all converged.
+    __device__ int project(int lane, int rounds) {
         const bool own = lane < N;
         {
             double a[N];
@@ -166,14 +170,13 @@ template <int N> struct WarpEig {
         const double lam = __shfl_sync(0xffffffffu, 0.5 * (lo + hi), (lane * ways) & 31);
         const bool vec = lane < k;
         double x[N];
-        bool bad = false;
+        unsigned sw = 0;
+        double* f0 = M + lane;
+        double* f1 = M + K * N + lane;
         if (vec) {
             // LU of T - lam I with row exchanges. Row i keeps 1 / pivot in f0 and in f1 the second
             // entry b of the row, or, where rows i and i + 1 were exchanged (bit i of sw), the entry a
             // that the exchange moved down (the pivot row is then T's row i + 1).
-            double* f0 = M + lane;
-            double* f1 = M + K * N + lane;
-            unsigned sw = 0;
             double a = d[0] - lam, b = e[0];
             const double tiny = kEigEps * nrm;
 #pragma unroll 4
@@ -197,92 +200,96 @@ template <int N> struct WarpEig {
             }
             if (fabs(a) < tiny) a = copysign(tiny, a);
             f0[K * (N - 1)] = 1.0 / a;
+        }
 #pragma unroll
-            for (int i = 0; i < N; ++i) x[i] = eig_start(i, lane);
+        for (int i = 0; i < N; ++i) x[i] = vec ? eig_start(i, lane) : 0.0;
+        bool bad = true;
 #pragma unroll 1
-            for (int it = 0; it < 2; ++it) {
-                if (it > 0) {
+        for (int round = 0; bad && round < rounds; ++round) {
+            if (vec) {
+#pragma unroll 1
+                for (int it = round == 0 ? 0 : 1; it < 2; ++it) { // the first solve has no forward pass
+                    if (it > 0) {
 #pragma unroll
-                    for (int i = 0; i < N - 1; ++i) {
-                        if ((sw >> i) & 1u) {
-                            const double t = x[i];
-                            x[i] = x[i + 1];
-                            x[i + 1] = fma(-(f1[K * i] * f0[K * i]), x[i], t);
-                        } else {
-                            x[i + 1] = fma(-(e[i] * f0[K * i]), x[i], x[i + 1]);
+                        for (int i = 0; i < N - 1; ++i) {
+                            if ((sw >> i) & 1u) {
+                                const double t = x[i];
+                                x[i] = x[i + 1];
+                                x[i + 1] = fma(-(f1[K * i] * f0[K * i]), x[i], t);
+                            } else {
+                                x[i + 1] = fma(-(e[i] * f0[K * i]), x[i], x[i + 1]);
+                            }
                         }
                     }
-                }
 #pragma unroll
-                for (int i = N - 1; i >= 0; --i) {
-                    double s = x[i];
-                    if (i + 1 < N) {
-                        const bool ex = (sw >> i) & 1u;
-                        s = fma(-(ex ? d[i + 1] - lam : f1[K * i]), x[i + 1], s);
-                        if (i + 2 < N && ex) s = fma(-e[i + 1], x[i + 2], s);
+                    for (int i = N - 1; i >= 0; --i) {
+                        double s = x[i];
+                        if (i + 1 < N) {
+                            const bool ex = (sw >> i) & 1u;
+                            s = fma(-(ex ? d[i + 1] - lam : f1[K * i]), x[i + 1], s);
+                            if (i + 2 < N && ex) s = fma(-e[i + 1], x[i + 2], s);
+                        }
+                        x[i] = s * f0[K * i];
                     }
-                    x[i] = s * f0[K * i];
-                }
-                double big = 0;
+                    double big = 0;
 #pragma unroll
-                for (int i = 0; i < N; ++i) big = fmax(big, fabs(x[i]));
-                const double sc = 1.0 / big;
-                double q = 0;
-#pragma unroll
-                for (int i = 0; i < N; ++i) {
-                    x[i] *= sc;
-                    q = fma(x[i], x[i], q);
-                }
-                const double r = rsqrt(q);
-#pragma unroll
-                for (int i = 0; i < N; ++i) x[i] *= r;
-            }
-            double res = 0;
-#pragma unroll
-            for (int i = 0; i < N; ++i) {
-                double t = (d[i] - lam) * x[i];
-                if (i > 0) t = fma(e[i - 1], x[i - 1], t);
-                if (i + 1 < N) t = fma(e[i], x[i + 1], t);
-                res = fmax(res, fabs(t));
-                if (!(fabs(t) <= 1e-12 * nrm)) res = INFINITY;
-            }
-            bad = !(res <= 1e-12 * nrm);
-        } else {
-#pragma unroll
-            for (int i = 0; i < N; ++i) x[i] = 0.0;
-        }
-        // Modified Gram-Schmidt over the lanes, twice.
-#pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass)
-#pragma unroll 1
-            for (int m = 0; m < k; ++m) {
-                if (lane == m) {
+                    for (int i = 0; i < N; ++i) big = fmax(big, fabs(x[i]));
+                    const double sc = 1.0 / big;
                     double q = 0;
 #pragma unroll
-                    for (int i = 0; i < N; ++i) q = fma(x[i], x[i], q);
-                    if (!(q > 1e-12)) bad = true;
+                    for (int i = 0; i < N; ++i) {
+                        x[i] *= sc;
+                        q = fma(x[i], x[i], q);
+                    }
                     const double r = rsqrt(q);
 #pragma unroll
-                    for (int i = 0; i < N; ++i) {
-                        x[i] *= r;
-                        Z[N * m + i] = x[i];
-                    }
+                    for (int i = 0; i < N; ++i) x[i] *= r;
                 }
-                __syncwarp();
-                if (vec && lane > m) {
-                    double q0 = 0, q1 = 0;
-#pragma unroll
-                    for (int i = 0; i < N; i += 2) {
-                        q0 = fma(Z[N * m + i], x[i], q0);
-                        if (i + 1 < N) q1 = fma(Z[N * m + i + 1], x[i + 1], q1);
-                    }
-                    const double q = q0 + q1;
-#pragma unroll
-                    for (int i = 0; i < N; ++i) x[i] = fma(-q, Z[N * m + i], x[i]);
-                }
-                __syncwarp();
             }
-        if (__any_sync(0xffffffffu, bad)) return -1;
+            // Modified Gram-Schmidt over the lanes, twice.
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass)
+#pragma unroll 1
+                for (int m = 0; m < k; ++m) {
+                    if (lane == m) {
+                        double q = 0;
+#pragma unroll
+                        for (int i = 0; i < N; ++i) q = fma(x[i], x[i], q);
+                        const double r = rsqrt(q);
+#pragma unroll
+                        for (int i = 0; i < N; ++i) {
+                            x[i] *= r;
+                            Z[N * m + i] = x[i];
+                        }
+                    }
+                    __syncwarp();
+                    if (vec && lane > m) {
+                        double q0 = 0, q1 = 0;
+#pragma unroll
+                        for (int i = 0; i < N; i += 2) {
+                            q0 = fma(Z[N * m + i], x[i], q0);
+                            if (i + 1 < N) q1 = fma(Z[N * m + i + 1], x[i + 1], q1);
+                        }
+                        const double q = q0 + q1;
+#pragma unroll
+                        for (int i = 0; i < N; ++i) x[i] = fma(-q, Z[N * m + i], x[i]);
+                    }
+                    __syncwarp();
+                }
+            // The residuals of what Gram-Schmidt left.
+            bool off = false;
+            if (vec) {
+#pragma unroll
+                for (int i = 0; i < N; ++i) {
+                    double t = (d[i] - lam) * x[i];
+                    if (i > 0) t = fma(e[i - 1], x[i - 1], t);
+                    if (i + 1 < N) t = fma(e[i], x[i + 1], t);
+                    off = off || !(fabs(t) <= kEigResidual * nrm);
+                }
+            }
+            bad = __any_sync(0xffffffffu, off);
+        }
+        if (bad) return -1;
         // Eigenvectors of the matrix: the reflectors from the last to the first, then scaled by
         // sqrt |lambda| (the update's terms are then products of two equal factors: bitwise symmetric).
         if (vec) {
@@ -333,6 +340,8 @@ struct BlockEig {
     static constexpr int kPacked = N * (N + 1) / 2;
     static constexpr int kStride = N + 1; // of an eigenvector in shared memory: K rows fill the triangle
     static constexpr size_t kScratch = 3 * static_cast<size_t>(N) * K;
+    static_assert(N * N <= static_cast<int>(kScratch), "Jacobi's eigenvectors fit the scratch");
+    static_assert(3 * K <= kWarps * N, "Jacobi's rotations fit the partial sums");
     static_assert(K * kStride <= kPacked, "the eigenvectors fit the matrix");
     double A[kPacked];       // lower triangle: row r at r (r + 1) / 2; then reflectors; then eigenvectors
     double part[kWarps * N]; // partial sums
@@ -340,7 +349,7 @@ struct BlockEig {
     double d[N], e[N], e2[N], beta[N], lam[K];
     double red[kWarps];
     unsigned sw[kT][K];
-    int bad, nneg, npos;
+    int nneg, npos;
 
     static __device__ __forceinline__ int at(int r, int c) { return r * (r + 1) / 2 + c; } // r >= c
 
@@ -445,10 +454,9 @@ struct BlockEig {
         __syncthreads();
     }
 
-    // Inverse iteration for eigenvector c < k by thread c; its vector (not normalised) goes to X[K i + c].
-    // Returns its 2-norm's inverse, or 0 where the residual is not at round-off.
-    __device__ double inverse_iteration(int c, int attempt, double nrm, double* f0, double* f1, double* X) {
-        const double lm = lam[c] + 4 * kEigEps * nrm * attempt, tiny = kEigEps * nrm;
+    // LU of T - lambda_c I for eigenvector c < k by thread c.
+    __device__ void factor(int c, double nrm, double* f0, double* f1) {
+        const double lm = lam[c], tiny = kEigEps * nrm;
         double a = d[0] - lm, b = e[0];
         unsigned bits = 0;
 #pragma unroll 4
@@ -480,9 +488,16 @@ struct BlockEig {
         if (fabs(a) < tiny) a = copysign(tiny, a);
         f0[K * (N - 1) + c] = 1.0 / a;
         f1[K * (N - 1) + c] = 0;
-        double scale = 1.0, res = 0;
+    }
+
+    // Inverse iteration for eigenvector c < k by thread c: two solves from a seeded start (the first without
+    // its forward pass), or one from the vector at X[K i + c], which the result replaces. Returns the
+    // inverse of its 2-norm.
+    __device__ double inverse_iteration(int c, bool first, const double* f0, const double* f1, double* X) {
+        const double lm = lam[c];
+        double scale = 1.0;
         constexpr int U = 8; // rows loaded ahead of the chain
-        for (int it = 0; it < 2; ++it) {
+        for (int it = first ? 0 : 1; it < 2; ++it) {
             if (it > 0) {
                 double x = scale * X[c];
                 for (int i0 = 0; i0 < N - 1; i0 += U) {
@@ -510,13 +525,12 @@ struct BlockEig {
                 X[K * (N - 1) + c] = x;
             }
             double x1 = 0, x2 = 0, q = 0;
-            res = 0;
             for (int i0 = N - U; i0 >= 0; i0 -= U) {
                 double g0[U], g1[U], xv[U];
 #pragma unroll
                 for (int j = U - 1; j >= 0; --j) {
                     g0[j] = f0[K * (i0 + j) + c], g1[j] = f1[K * (i0 + j) + c];
-                    xv[j] = it == 0 ? eig_start(i0 + j, c + K * attempt) : X[K * (i0 + j) + c];
+                    xv[j] = it == 0 ? eig_start(i0 + j, c) : X[K * (i0 + j) + c];
                 }
                 const unsigned word = sw[i0 >> 5][c];
 #pragma unroll
@@ -527,21 +541,165 @@ struct BlockEig {
                     double s = fma(-(ex ? dn : g1[j]), x1, xv[j]);
                     if (ex) s = fma(-sn, x2, s);
                     s *= g0[j];
-                    // Residual of row i + 1, whose neighbours are s and x2.
-                    if (i + 1 < N) res = fmax(res, fabs(fma(dn, x1, fma(e[i], s, sn * x2))));
                     q = fma(s, s, q);
                     X[K * i + c] = s;
                     x2 = x1;
                     x1 = s;
                 }
             }
-            res = fmax(res, fabs(fma(d[0] - lm, x1, e[0] * x2)));
             scale = rsqrt(q);
         }
-        return res * scale <= 1e-12 * nrm ? scale : 0.0; // false for NaN
+        return scale;
     }
 
-    // The reflectors applied to the k eigenvectors of T (X, scaled by `scale` of the thread's column), which
+    // Modified Gram-Schmidt, twice, over the k vectors of X times their factors in y, columns dealt to the
+    // warps and kept in registers; the reflectors stay in A. Returns whether a residual is above round-off.
+    __device__ bool orthonormalise(int k, double nrm, double* X) {
+        static_assert(K % kWarps == 0, "columns per warp");
+        constexpr int J = K / kWarps;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        double z[J][kT];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int c = warp + kWarps * j;
+            const double s = c < k ? y[c] : 0.0;
+#pragma unroll
+            for (int t = 0; t < kT; ++t) z[j][t] = c < k ? s * X[K * (32 * t + lane) + c] : 0.0;
+        }
+        int off = 0;
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass)
+#pragma unroll 1
+            for (int m = 0; m < k; ++m) {
+                double* u = v[m & 1]; // two buffers: one barrier per vector
+                const bool mine = warp == (m & (kWarps - 1));
+                if (mine)
+#pragma unroll
+                    for (int j = 0; j < J; ++j)
+                        if (j == m / kWarps) {
+                            double q = 0;
+#pragma unroll
+                            for (int t = 0; t < kT; ++t) q = fma(z[j][t], z[j][t], q);
+#pragma unroll
+                            for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+                            const double r = rsqrt(q);
+#pragma unroll
+                            for (int t = 0; t < kT; ++t) {
+                                z[j][t] *= r;
+                                u[32 * t + lane] = z[j][t];
+                            }
+                        }
+                __syncthreads();
+#pragma unroll
+                for (int j = 0; j < J; ++j) {
+                    const int c = warp + kWarps * j;
+                    if (c <= m || c >= k) continue; // the same for the whole warp
+                    double q = 0;
+#pragma unroll
+                    for (int t = 0; t < kT; ++t) q = fma(u[32 * t + lane], z[j][t], q);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+#pragma unroll
+                    for (int t = 0; t < kT; ++t) z[j][t] = fma(-q, u[32 * t + lane], z[j][t]);
+                }
+                if (pass > 0 && mine) {
+#pragma unroll
+                    for (int t = 0; t < kT; ++t) {
+                        const int i = 32 * t + lane;
+                        double res = (d[i] - lam[m]) * u[i];
+                        if (i > 0) res = fma(e[i - 1], u[i - 1], res);
+                        if (i < N - 1) res = fma(e[i], u[i + 1], res);
+                        if (!(fabs(res) <= kEigResidual * nrm)) off = 1;
+                    }
+                }
+            }
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int c = warp + kWarps * j;
+#pragma unroll
+            for (int t = 0; t < kT; ++t)
+                if (c < k) X[K * (32 * t + lane) + c] = z[j][t];
+        }
+        return __syncthreads_or(off) != 0; // X is written
+    }
+
+    // All eigenpairs of the matrix in A by the cyclic Jacobi method in the round-robin ordering of lpg_psd.h: a
+    // round's rotations act on disjoint 2 x 2 blocks of the packed triangle, one thread each. V is N N values
+    // of scratch. Leaves what project() does and returns k. Tens of milliseconds; for what inverse iteration
+    // does not resolve.
+    __device__ __noinline__ int jacobi(double* V, int& kind) {
+        using J = PsdJacobi<N>;
+        const int tid = threadIdx.x;
+        double* cs = part;                                // cosine and sine of each pair
+        int* pq = reinterpret_cast<int*>(part + 2 * K); // its indices
+        for (int t = tid; t < N * N; t += kThreads) V[t] = t / N == t % N ? 1.0 : 0.0;
+        const auto entry = [&](int r, int c) -> double& { return A[r >= c ? at(r, c) : at(c, r)]; };
+        for (int sweep = 0; sweep < J::kMaxSweeps; ++sweep) {
+            double off = 0, diag = 0;
+            for (int t = tid; t < N * N; t += kThreads) {
+                const int r = t / N, c = t - N * r;
+                if (r > c) off = fma(A[at(r, c)], A[at(r, c)], off);
+                if (r == c) diag = fma(A[at(r, r)], A[at(r, r)], diag);
+            }
+            off = 2 * sum(off);
+            __syncthreads();
+            diag = sum(diag);
+            if (!(off > J::kOffTol2 * (off + diag))) break;
+            for (int round = 0; round < J::kRounds; ++round) {
+                if (tid < K) {
+                    int p, q;
+                    J::pair(round, tid, p, q);
+                    jacobi_rotation(entry(p, p), entry(q, q), entry(p, q), cs[2 * tid], cs[2 * tid + 1]);
+                    pq[2 * tid] = p;
+                    pq[2 * tid + 1] = q;
+                }
+                __syncthreads();
+                for (int t = tid; t < K * K; t += kThreads) {
+                    const int i = t / K, j = t - K * i;
+                    if (j < i) continue;
+                    const int p = pq[2 * i], q = pq[2 * i + 1], pp = pq[2 * j], qq = pq[2 * j + 1];
+                    const double c = cs[2 * i], s = cs[2 * i + 1], c2 = cs[2 * j], s2 = cs[2 * j + 1];
+                    const double b00 = entry(p, pp), b01 = entry(p, qq), b10 = entry(q, pp), b11 = entry(q, qq);
+                    const double x0 = c2 * b00 - s2 * b01, x1 = s2 * b00 + c2 * b01; // the columns' rotation
+                    const double y0 = c2 * b10 - s2 * b11, y1 = s2 * b10 + c2 * b11;
+                    entry(p, pp) = c * x0 - s * y0;
+                    entry(q, qq) = s * x1 + c * y1;
+                    entry(q, pp) = i == j ? 0.0 : s * x0 + c * y0;
+                    if (i != j) entry(p, qq) = c * x1 - s * y1;
+                }
+                for (int t = tid; t < N * K; t += kThreads) {
+                    const int i = t / K, j = t - K * i;
+                    double &a = V[N * i + pq[2 * j]], &b = V[N * i + pq[2 * j + 1]];
+                    const double va = a, vb = b, c = cs[2 * j], s = cs[2 * j + 1];
+                    a = c * va - s * vb;
+                    b = s * va + c * vb;
+                }
+                __syncthreads();
+            }
+        }
+        __syncthreads();
+        if (tid < N) d[tid] = A[at(tid, tid)];
+        __syncthreads();
+        if (tid == 0) {
+            int n = 0, p = 0;
+            for (int m = 0; m < N; ++m) n += d[m] < 0.0, p += d[m] > 0.0;
+            nneg = n, npos = p;
+            for (int m = 0, c = 0; m < N; ++m)
+                if (n <= p ? d[m] < 0.0 : d[m] > 0.0) pq[c++] = m;
+        }
+        __syncthreads();
+        const bool neg = nneg <= npos;
+        const int k = neg ? nneg : npos;
+        kind = k == 0 ? (neg ? 0 : 2) : (neg ? 1 : 2);
+        for (int t = tid; t < k * N; t += kThreads) {
+            const int c = t / N, i = t - N * c, m = pq[c];
+            A[kStride * c + i] = sqrt(fabs(d[m])) * V[N * i + m];
+        }
+        __syncthreads();
+        return k;
+    }
+
+    // The reflectors applied to the k eigenvectors of T (X, times the column's entry of `scales`), which
     // then replace the reflectors in A (vector c at kStride c). Lanes are columns; a column's rows are dealt
     // to P warps (row p, p + P, ...), which add their parts of each product.
     template <int P> __device__ void back_transform(int k, const double* X, const double* scales) {
@@ -594,66 +752,25 @@ struct BlockEig {
         __syncthreads();
     }
 
-    // Modified Gram-Schmidt over the k vectors in A, twice; a vector that vanishes sets `bad`. The
-    // vectors are left multiplied by sqrt |lambda|.
-    __device__ void orthonormalise(int k) {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        auto normalise = [&](int m, double scale) {
-            double* y0 = A + kStride * m + lane;
-            double q = 0, u[kT];
-#pragma unroll
-            for (int t = 0; t < kT; ++t) {
-                u[t] = y0[32 * t];
-                q = fma(u[t], u[t], q);
+    // The matrix of an element's record times `down` into A. Block (a, b), a <= b, entry (i, c) of the record is
+    // H(3 a + i, 3 b + c): the blocks of a are consecutive.
+    __device__ void load(const double* rec, double down) {
+        for (int a = threadIdx.x >> 5; a < N / 3; a += kWarps) {
+            const double* ra = rec + 9 * (a * (N / 3) - a * (a - 1) / 2);
+            for (int t = threadIdx.x & 31; t < 9 * (N / 3 - a); t += 32) {
+                const int b = a + t / 9, ic = t - 9 * (t / 9), r = 3 * a + ic / 3, c = 3 * b + ic % 3;
+                if (c >= r) A[at(c, r)] = down * ra[t];
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-            if (!(q > 1e-12) && lane == 0) bad = 1;
-            const double r = scale * rsqrt(q);
-#pragma unroll
-            for (int t = 0; t < kT; ++t) y0[32 * t] = r * u[t];
-        };
-        for (int pass = 0; pass < 2; ++pass) {
-            if (warp == 0) normalise(0, 1.0);
-            __syncthreads();
-            for (int m = 0; m < k; ++m) {
-                double u[kT];
-#pragma unroll
-                for (int t = 0; t < kT; ++t) u[t] = A[kStride * m + 32 * t + lane];
-                int c = m + 1 + ((warp - (m + 1)) & (kWarps - 1)); // the warp's first column after m
-                for (; c < k; c += kWarps) {
-                    double* yc = A + kStride * c + lane;
-                    double z[kT], q = 0;
-#pragma unroll
-                    for (int t = 0; t < kT; ++t) {
-                        z[t] = yc[32 * t];
-                        q = fma(u[t], z[t], q);
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-#pragma unroll
-                    for (int t = 0; t < kT; ++t) yc[32 * t] = fma(-q, u[t], z[t]);
-                    if (c == m + 1) {
-                        __syncwarp();
-                        normalise(c, 1.0);
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        for (int c = warp; c < k; c += kWarps) {
-            const double r = sqrt(fabs(lam[c]));
-#pragma unroll
-            for (int t = 0; t < kT; ++t) A[kStride * c + 32 * t + lane] *= r;
         }
         __syncthreads();
     }
 
-    // Projection of the matrix in A (scaled to max |entry| < 1). Returns the number k of vectors
+    // Projection of the record's matrix times `down` (max |entry| < 1). Returns the number k of vectors
     // z_c = sqrt |lambda_c| v_c left in A (at kStride c) and the kind: 0 the matrix is its own projection,
-    // 1 H+ = H + sum z z^T, 2 H+ = sum z z^T, -1 not accurate after the retries.
-    __device__ int project(double* scratch, int& kind) {
+    // 1 H+ = H + sum z z^T, 2 H+ = sum z z^T.
+    __device__ int project(const double* rec, double down, double* scratch, int rounds, int& kind) {
         const int tid = threadIdx.x, lane = tid & 31;
+        load(rec, down);
         tridiagonal();
         double nrm = 0;
         for (int i = lane; i < N; i += 32) {
@@ -671,7 +788,6 @@ struct BlockEig {
             else
                 nneg = n;
         }
-        if (tid == 0) bad = 0;
         __syncthreads();
         const bool neg = nneg <= npos;
         const int k = neg ? nneg : npos;
@@ -700,28 +816,25 @@ struct BlockEig {
         }
         __syncthreads();
         double *f0 = scratch, *f1 = scratch + N * K, *X = scratch + 2 * N * K;
-        // A residual above round-off is tried again from other starts and shifts.
-        for (int attempt = 0;; ++attempt) {
-            if (tid < k) {
-                const double r = inverse_iteration(tid, attempt, nrm, f0, f1, X);
-                y[tid] = r;
-                if (r == 0.0) bad = 1;
-            }
+        if (tid < k) factor(tid, nrm, f0, f1);
+        bool bad = true;
+        for (int round = 0; bad && round < rounds; ++round) {
+            if (tid < k) y[tid] = inverse_iteration(tid, round == 0, f0, f1, X);
             __syncthreads();
-            const bool again = bad != 0;
-            __syncthreads();
-            if (!again || attempt == 3) break;
-            if (tid == 0) bad = 0;
-            __syncthreads();
+            bad = orthonormalise(k, nrm, X);
         }
+        if (bad) {
+            load(rec, down);
+            return jacobi(scratch, kind);
+        }
+        if (tid < k) y[tid] = sqrt(fabs(lam[tid]));
+        __syncthreads();
         if (k <= 32)
             back_transform<16>(k, X, y);
         else if (k <= 64)
             back_transform<8>(k, X, y);
         else
             back_transform<5>(k, X, y);
-        orthonormalise(k);
-        if (bad) kind = -1;
         return k;
     }
 };

@@ -322,6 +322,12 @@ size_t hermite_scratch_doubles(const DevMesh& m);
 // Bytes of the block records launch_hex_eval needs: FP64 records, plus FP32 ones for a
 // projected mixed-precision Hessian (the projection runs in FP64).
 size_t hex_blocks_bytes(const DevMesh& m, int precision, bool projected);
+// Passes of inverse iteration with orthogonalisation before a projection takes the Jacobi method.
+constexpr int kProjectionRounds = 6;
+// The projections alone, of `count` FP64 element Hessians of 8 or 64 nodes (records as in the passes above).
+void launch_projection(int nodes, int count, const double* in, double* out, double* scratch, int rounds,
+                       unsigned* status, cudaStream_t s);
+size_t projection_scratch_doubles(int nodes, int count);
 // Largest step along du keeping det F > 0 at every quadrature point of every hex (x 0.9 as the
 // reference), minimum over the mesh into *alpha (device).
 void launch_hex_feasible(const DevMesh& m, const double* u, const double* du, double* block_min, int nblocks,

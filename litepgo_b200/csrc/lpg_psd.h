@@ -29,6 +29,19 @@ LPG_HD double inv_sqrt(double x) {
 #endif
 }
 
+// The rotation zeroing A(p, q): A' = J^T A J with J_pp = J_qq = c, J_pq = s, J_qp = -s,
+// t = tan phi the smaller root of t^2 + 2 t theta - 1 = 0, theta = (A_qq - A_pp) / (2 A_pq).
+LPG_HD void jacobi_rotation(double app, double aqq, double apq, double& c, double& s) {
+    c = 1.0, s = 0.0;
+    if (apq != 0.0) {
+        const double th = (aqq - app) / (2.0 * apq);
+        const double at = fabs(th);
+        const double t = at > 1e150 ? 0.5 / th : copysign(1.0, th) / (at + sqrt(th * th + 1.0));
+        c = inv_sqrt(t * t + 1.0);
+        s = t * c;
+    }
+}
+
 template <int N>
 struct PsdJacobi {
     static_assert(N % 2 == 0 && N >= 2, "the round-robin ordering pairs an even number of indices");
@@ -55,22 +68,11 @@ struct PsdJacobi {
         q = x < y ? y : x;
     }
 
-    // The rotation zeroing A(p, q): A' = J^T A J with J_pp = J_qq = c, J_pq = s, J_qp = -s,
-    // t = tan phi the smaller root of t^2 + 2 t theta - 1 = 0, theta = (A_qq - A_pp) / (2 A_pq).
+    // The rotation of pair k of round r.
     LPG_HD static void rotation(const double* A, int r, int k, double* cs, int* pq) {
         int p, q;
         pair(r, k, p, q);
-        const double apq = A[p * S + q];
-        double c = 1.0, s = 0.0;
-        if (apq != 0.0) {
-            const double th = (A[q * S + q] - A[p * S + p]) / (2.0 * apq);
-            const double at = fabs(th);
-            const double t = at > 1e150 ? 0.5 / th : copysign(1.0, th) / (at + sqrt(th * th + 1.0));
-            c = inv_sqrt(t * t + 1.0);
-            s = t * c;
-        }
-        cs[2 * k] = c;
-        cs[2 * k + 1] = s;
+        jacobi_rotation(A[p * S + p], A[q * S + q], A[p * S + q], cs[2 * k], cs[2 * k + 1]);
         pq[2 * k] = p;
         pq[2 * k + 1] = q;
     }
