@@ -290,7 +290,7 @@ void lpg_fem::eval_async(const double* du, double* dgrad, int hessian, int preci
         void* blocks = a.hess ? d_proj.ensure(hermite_blocks_bytes(dm, precision, projected)) : nullptr;
         double* scratch = projected && a.hess && T > 0 ? d_herm_q.as<double>(hermite_scratch_doubles(dm)) : nullptr;
         launch_hermite_eval(dm, precision, projected, du, elemE, d_vjp.as<double>(std::max<size_t>(192 * T, 1)), blocks,
-                            scratch, a, stream);
+                            scratch, projected ? d_plist.as<int>(std::max<size_t>(T, 1)) : nullptr, a, stream);
         return;
     }
     if (dm.K == 8) {
@@ -300,7 +300,7 @@ void lpg_fem::eval_async(const double* du, double* dgrad, int hessian, int preci
         void* blocks = a.hess ? d_proj.ensure(hex_blocks_bytes(dm, precision, projected)) : nullptr;
         a.cluster_energy = d_cluster_energy.as<double>(static_cast<size_t>(std::max(dm.ncl, dm.tc_ncl)) + 256);
         launch_hex_eval(dm, precision, projected, du, elemE, d_vjp.as<double>(std::max<size_t>(24 * T, 1)), blocks,
-                        a, stream);
+                        projected ? d_plist.as<int>(std::max<size_t>(T, 1)) : nullptr, a, stream);
         return;
     }
     if (a.hess && hessian == LPG_HESSIAN_PROJECTED) {
@@ -810,7 +810,8 @@ int lpg_fem_eval_material(lpg_fem_t h, const double* W, const double* P, const d
             const bool projected = hessian == LPG_HESSIAN_PROJECTED;
             void* blocks = a.hess ? h->d_proj.ensure(hex_blocks_bytes(h->dm, precision, projected)) : nullptr;
             launch_hex_material_eval(h->dm, precision, hessian, dW, dP, dA, h->d_mat[3].as<double>(nel),
-                                     h->d_vjp.as<double>(24 * nel), blocks, a, s);
+                                     h->d_vjp.as<double>(24 * nel), blocks,
+                                     projected ? h->d_plist.as<int>(nel) : nullptr, a, s);
         } else {
             void* proj = a.hess ? h->d_proj.ensure(project_bytes(h->dm, precision)) : nullptr;
             launch_material_eval(h->dm, precision, hessian, dW, dP, dA, h->d_mat[3].as<double>(nel),

@@ -2212,7 +2212,11 @@ __global__ void __launch_bounds__(256) material_pieces_kernel(const DevMesh m, c
 // elements at a time); then one thread per (element, vertex pair a <= b) accumulates
 // H_ab += w [mu (grad N_a . grad N_b) I + lambda h_a h_b^T - p h_b h_a^T], the pairs (a, a) also
 // g_a = sum w P grad N_a and the pair (0, 0) the energy. FP64 throughout; the blocks are stored in the
-// precision's type. FP64-bound: each of an element's 36 threads used to form the point's kinematics itself.
+// precision's type. With FLAGS (of a projected Hessian), flags[e] says whether some point's tangent may be
+// indefinite: a sum of w B^T A B with semi-definite A is its own projection. The test runs after the points' barrier,
+// beside the other warps' pairs: 110,592 hexes at rest, all of them tridiagonalised before, 1,980 -> 781 us for the
+// whole evaluation; random states, all indefinite, 4,515 -> 4,537.
+// FP64-bound: each of an element's 36 threads used to form the point's kinematics itself.
 // 7,480 hexes at 8 points: 105 -> 33 us (two 256-thread blocks per SM; eight elements in 288 threads left
 // one block per SM and took 44 us).
 // ---------------------------------------------------------------------------
@@ -2261,8 +2265,9 @@ constexpr int kHexThreads = 256;             // one thread per (element, pair), 
 static_assert(36 * kHexEl <= kHexThreads, "one thread per (element, pair)");
 constexpr int kHexChunk = 8;                 // points kept at a time
 
-// One quadrature point of a hex into rec (kHexPoint values); a point with a bad F contributes zeros.
-__device__ __forceinline__ unsigned hex_point(const DevMesh& m, int e, int q, const double* __restrict__ u, double* rec) {
+// One quadrature point of a hex into rec (kHexPoint values) and F^-T; a point with a bad F contributes zeros.
+__device__ __forceinline__ unsigned hex_point(const DevMesh& m, int e, int q, const double* __restrict__ u, double* rec,
+                                              double (&FiT)[9]) {
     unsigned st = 0;
     const int32_t* cell = m.hex_cells + 8 * static_cast<size_t>(e);
     const double lam = m.hex_theta[2 * static_cast<size_t>(e)], mu = m.hex_theta[2 * static_cast<size_t>(e) + 1];
@@ -2308,7 +2313,7 @@ __device__ __forceinline__ unsigned hex_point(const DevMesh& m, int e, int q, co
         return st;
     }
     const double L = log(detF), p = lam * L - mu, iF = 1.0 / detF;
-    double FiT[9], ff = 0;
+    double ff = 0;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         FiT[k] = C[k] * iF;
@@ -2333,13 +2338,16 @@ __device__ __forceinline__ unsigned hex_point(const DevMesh& m, int e, int q, co
     return st;
 }
 
-template <typename R>
+template <typename R, bool FLAGS>
 __global__ void __launch_bounds__(kHexThreads, 2) hex_element_kernel(const DevMesh m, const double* __restrict__ u,
                                                                   double* __restrict__ elemE,
                                                                   double* __restrict__ per_elem,
-                                                                  R* __restrict__ blocks, unsigned* status) {
+                                                                  R* __restrict__ blocks, int* __restrict__ flags,
+                                                                  unsigned* status) {
     __shared__ double sp[kHexEl * kHexChunk * kHexPoint];
+    __shared__ int s_indefinite[kHexEl];
     const int tid = threadIdx.x, el = tid / 36, pr = tid - 36 * el;
+    if (FLAGS && tid < kHexEl) s_indefinite[tid] = 0;
     const int e0 = blockIdx.x * kHexEl, e = e0 + el;
     unsigned st = 0;
     const bool on = el < kHexEl && e < m.T;
@@ -2349,11 +2357,18 @@ __global__ void __launch_bounds__(kHexThreads, 2) hex_element_kernel(const DevMe
     for (int q0 = 0; q0 < m.nq; q0 += kHexChunk) {
         const int nq = min(kHexChunk, m.nq - q0);
         __syncthreads(); // the previous points are read
-        for (int t = tid; t < kHexEl * nq; t += kHexThreads) {
-            const int te = e0 + t / nq, tq = t - nq * (t / nq);
-            if (te < m.T) st |= hex_point(m, te, q0 + tq, u, sp + kHexPoint * ((t / nq) * kHexChunk + tq));
-        }
+        static_assert(kHexEl * kHexChunk <= kHexThreads, "one thread per point");
+        const int pe = tid / kHexChunk, pq = tid % kHexChunk; // this thread's point and its record
+        double* point = sp + kHexPoint * tid;
+        const bool has = pe < kHexEl && e0 + pe < m.T && pq < nq;
+        double FiT[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        if (has) st |= hex_point(m, e0 + pe, q0 + pq, u, point, FiT);
         __syncthreads();
+        // After the barrier, where the other warps have work: a semi-definite tangent at every point?
+        if (FLAGS && has && *static_cast<volatile int*>(s_indefinite + pe) == 0) {
+            const double iw = 1.0 / point[kHexMu];
+            if (!nh_semidefinite(FiT, iw * point[kHexPp], iw * point[kHexL])) s_indefinite[pe] = 1;
+        }
         if (!on) continue;
         for (int q = 0; q < nq; ++q) {
             const double* rec = sp + kHexPoint * (el * kHexChunk + q);
@@ -2409,6 +2424,10 @@ __global__ void __launch_bounds__(kHexThreads, 2) hex_element_kernel(const DevMe
             if (!isfinite(E)) st |= ST_NONFINITE_OUT;
             elemE[e] = E;
         }
+    }
+    if (FLAGS) {
+        __syncthreads();
+        if (tid < kHexEl && e0 + tid < m.T) flags[e0 + tid] = s_indefinite[tid];
     }
     st = __reduce_or_sync(0xffffffffu, st);
     if ((tid & 31) == 0 && st) atomicOr(status, st);
@@ -2610,12 +2629,28 @@ __global__ void __launch_bounds__(128) hex_material_kernel(const DevMesh m, cons
     if ((threadIdx.x & 31) == 0 && st) atomicOr(status, st);
 }
 
+// The same test on a material's own tangents, symmetrised: one thread per point marks its element in flags
+// (zeroed before), with the LDL^T of the tet pass in registers. Bound by its chain of nine divisions. An evaluation
+// of 8,000 hexes at 8 points, definite tangents 255 -> 183 us, indefinite ones 393 -> 418.
+__global__ void __launch_bounds__(128) hex_material_test_kernel(const DevMesh m, const double* __restrict__ A,
+                                                                int* __restrict__ flags) {
+    const size_t t = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= static_cast<size_t>(m.T) * m.nq) return;
+    const double* Aq = A + 81 * t;
+    double M[45];
+#pragma unroll
+    for (int r = 0; r < 9; ++r)
+#pragma unroll
+        for (int c = r; c < 9; ++c) M[sym9(r, c)] = 0.5 * (__ldg(Aq + 9 * r + c) + __ldg(Aq + 9 * c + r));
+    if (!semidefinite9<double>(M)) flags[t / m.nq] = 1;
+}
+
 // Projected Hessian of hex meshes (HessianKind::Projected, mesh_energy.cpp:16-27): one warp per element
 // loads its record of 36 FP64 blocks (hex_element_kernel) as the 24 x 24 element Hessian, projects it
 // (WarpEig) and writes the result as 36 blocks in the precision's type: in place for FP64 (a lane writes
 // the entries it read), into a separate FP32 record array for mixed precision. Each entry is formed from
-// its upper-triangle position, so the diagonal blocks stay bitwise symmetric. An element without an
-// eigenvalue below -8 eps |H| is kept as it is.
+// its upper-triangle position, so the diagonal blocks stay bitwise symmetric. An element whose flag is zero
+// (a sum of semi-definite tangents) or without an eigenvalue below -8 eps |H| is kept as it is.
 // Bound by the FP64 pipe (about 8,500 warp instructions per element) and by the latency of its chains at 16
 // warps per SM.
 // 7,480 hexes, every one indefinite: 214 us (a cyclic Jacobi iteration in shared memory took 1,664 us, and a
@@ -2637,7 +2672,8 @@ using HexEig = WarpEig<24>;
 
 template <typename R>
 __global__ void __launch_bounds__(32 * kHexPsdWarps, 4) hex_psd_kernel(int T, const double* in, R* out,
-                                                                      int rounds, unsigned* status) {
+                                                                      const int* __restrict__ flags, int rounds,
+                                                                      unsigned* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned short s_at[kHexRecord]; // record entry -> row << 8 | column of its upper entry
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2653,6 +2689,11 @@ __global__ void __launch_bounds__(32 * kHexPsdWarps, 4) hex_psd_kernel(int T, co
     if (e >= T) return;
     const double* rec = in + kHexRecord * static_cast<size_t>(e);
     R* o = out + kHexRecord * static_cast<size_t>(e);
+    if (flags != nullptr && flags[e] == 0) {
+        if (static_cast<const void*>(rec) != static_cast<const void*>(o))
+            for (int t = lane; t < kHexRecord; t += 32) o[t] = static_cast<R>(rec[t]);
+        return;
+    }
     constexpr int S = HexEig::S;
     constexpr int kPer = (kHexRecord + 31) / 32;
     double h[kPer], amax = 0;
@@ -2719,14 +2760,16 @@ __global__ void __launch_bounds__(32 * kHexPsdWarps, 4) hex_psd_kernel(int T, co
     st = __reduce_or_sync(0xffffffffu, st);
     if (lane == 0 && st) atomicOr(status, st);
 }
-// Each element's FP64 record projected into out's records (which may be the same memory).
+// Each element's FP64 record projected into out's records (which may be the same memory); with flags, those of
+// the elements marked in them.
 template <typename R>
-void launch_hex_psd(const DevMesh& m, const double* in, R* out, unsigned* status, cudaStream_t s,
+void launch_hex_psd(const DevMesh& m, const double* in, R* out, const int* flags, unsigned* status, cudaStream_t s,
                     int rounds = kProjectionRounds) {
     const size_t sm = kHexPsdWarps * sizeof(HexEig);
     thread_local LaunchCache cache;
     resident_grid(hex_psd_kernel<R>, 32 * kHexPsdWarps, sm, cache);
-    hex_psd_kernel<R><<<(m.T + kHexPsdWarps - 1) / kHexPsdWarps, 32 * kHexPsdWarps, sm, s>>>(m.T, in, out, rounds, status);
+    hex_psd_kernel<R><<<(m.T + kHexPsdWarps - 1) / kHexPsdWarps, 32 * kHexPsdWarps, sm, s>>>(m.T, in, out, flags, rounds,
+                                                                                                status);
 }
 
 // Feasible step of a hex mesh: at every quadrature point F and dF (the increment's gradient),
@@ -2824,7 +2867,8 @@ __device__ __forceinline__ void hermite_G(const double* tq, int b, const double 
 // each point's w lambda, w p, w mu, F^-T and w P in shared memory (four threads per point); then, eight
 // points at a time, every node's G and h = F^-T G, and one thread per pair of node pairs (2 x 2 blocks
 // H_ab, a <= b, in registers) accumulates them; diagonal blocks are mirrored so the matrix is bitwise
-// symmetric. The first block also writes the energy (points in order) and the gradient. FP64-bound
+// symmetric. The first block also writes the energy (points in order), the gradient and the element's flag as
+// hex_element_kernel does. FP64-bound
 // (28 operations per block and point; a thread's four nodes serve four blocks).
 // 80 elements at 64 points: 1,056 us (one 128-thread block per element, the nodes' gradients and
 // kinematics formed per block pair) -> 114 us.
@@ -2851,7 +2895,8 @@ template <typename R>
 __global__ void __launch_bounds__(kHermThreads, 2) hermite_element_kernel(const DevMesh m, const double* __restrict__ u,
                                                                           double* __restrict__ elemE,
                                                                           double* __restrict__ per_elem,
-                                                                          R* __restrict__ blocks, unsigned* status) {
+                                                                          R* __restrict__ blocks, int* __restrict__ flags,
+                                                                          unsigned* status) {
     __shared__ double sD[192];
     __shared__ double sK[64 * kHermPoint];
     __shared__ double sN[kHermChunk * 64 * 6]; // G, h per node
@@ -2948,6 +2993,14 @@ __global__ void __launch_bounds__(kHermThreads, 2) hermite_element_kernel(const 
             }
         }
     }
+    if (flags && third == 0) { // by the last 64 threads, beside the energy and the gradient
+        const int q = tid - (kHermThreads - 64);
+        const double* k = sK + kHermPoint * max(q, 0);
+        const double iw = 1.0 / k[2];
+        const bool indefinite = q >= 0 && q < m.nq && !nh_semidefinite(k + 4, iw * k[1], iw * k[0]);
+        const int any = __syncthreads_or(indefinite);
+        if (tid == 0) flags[e] = any;
+    }
     if (blocks) {
         const int tile = third * kHermThreads + tid;
         int tr = 0, tc = 0;
@@ -3042,11 +3095,14 @@ __global__ void __launch_bounds__(kHermThreads, 2) hermite_element_kernel(const 
 // record in `in` (FP64) is replaced by, or written in the precision's type to, `out`.
 // Bound by the chains of the tridiagonalisation (190 steps of five barriers), of the Sturm counts and of
 // the inverse iterations: one element per SM. 80 elements at
-// 64 points: 23.7 ms (tridiagonalisation and a QL iteration whose rotations one thread generated) -> 1.28 ms.
+// 64 points: 23.7 ms (tridiagonalisation and a QL iteration whose rotations one thread generated) -> 1.25 ms. Elements
+// whose points' tangents are all semi-definite are kept: 1,728 at rest, evaluation 12.9 (7.1 with the QL iteration
+// behind a test per point) -> 2.15 ms.
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(BlockEig::kThreads) hermite_psd_kernel(int T, const double* in, R* out,
-                                                                        double* __restrict__ scratch, int rounds,
+                                                                        double* __restrict__ scratch,
+                                                                        const int* __restrict__ flags, int rounds,
                                                                         unsigned* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BlockEig& B = *reinterpret_cast<BlockEig*>(smem_raw);
@@ -3057,6 +3113,11 @@ __global__ void __launch_bounds__(BlockEig::kThreads) hermite_psd_kernel(int T, 
     for (int e = blockIdx.x; e < T; e += gridDim.x) {
         const double* rec = in + kHermiteRecord * static_cast<size_t>(e);
         R* o = out + kHermiteRecord * static_cast<size_t>(e);
+        if (flags != nullptr && flags[e] == 0) { // a sum of semi-definite tangents
+            if (static_cast<const void*>(o) != static_cast<const void*>(rec))
+                for (int t = tid; t < kHermiteRecord; t += BlockEig::kThreads) o[t] = static_cast<R>(rec[t]);
+            continue;
+        }
         double amax = 0; // infinite where an entry is not finite
         for (int t = tid; t < kHermiteRecord; t += BlockEig::kThreads) {
             const double v = fabs(rec[t]);
@@ -3484,7 +3545,7 @@ void launch_hex_deformation_gradients(const DevMesh& m, const double* u, double*
 }
 
 void launch_hex_material_eval(const DevMesh& m, int precision, int hessian, const double* W, const double* P,
-                              const double* A, double* elemE, double* per_elem, void* blocks,
+                              const double* A, double* elemE, double* per_elem, void* blocks, int* flags,
                               const EvalArgs& a, cudaStream_t s) {
     const bool projected = hessian == LPG_HESSIAN_PROJECTED;
     if (m.T > 0) {
@@ -3493,12 +3554,15 @@ void launch_hex_material_eval(const DevMesh& m, int precision, int hessian, cons
         double* per_grad = a.grad ? per_elem : nullptr;
         if (a.hess && projected) {
             double* records = static_cast<double*>(blocks);
+            LPG_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * static_cast<size_t>(m.T), s));
+            const size_t points = static_cast<size_t>(m.T) * m.nq;
+            hex_material_test_kernel<<<static_cast<unsigned>((points + 127) / 128), 128, 0, s>>>(m, A, flags);
             hex_material_kernel<double><<<grid, 128, 0, s>>>(m, W, P, A, elemE, per_grad, records, a.status);
             if (precision == LPG_PRECISION_F64) {
-                launch_hex_psd<double>(m, records, records, a.status, s);
+                launch_hex_psd<double>(m, records, records, flags, a.status, s);
             } else {
                 float* out = reinterpret_cast<float*>(records + kHexRecord * static_cast<size_t>(m.T));
-                launch_hex_psd<float>(m, records, out, a.status, s);
+                launch_hex_psd<float>(m, records, out, flags, a.status, s);
                 blocks = out;
             }
         } else if (precision == LPG_PRECISION_F64 || !a.hess) {
@@ -3538,19 +3602,20 @@ int hermite_psd_grid(const DevMesh& m) {
     return std::max(1, std::min(m.T, sms));
 }
 template <typename R>
-void launch_hermite_psd(const DevMesh& m, const double* in, R* out, double* scratch, unsigned* status, cudaStream_t s,
-                        int rounds = kProjectionRounds) {
+void launch_hermite_psd(const DevMesh& m, const double* in, R* out, double* scratch, const int* flags, unsigned* status,
+                        cudaStream_t s, int rounds = kProjectionRounds) {
     thread_local LaunchCache cache;
     resident_grid(hermite_psd_kernel<R>, BlockEig::kThreads, sizeof(BlockEig), cache);
-    hermite_psd_kernel<R><<<hermite_psd_grid(m), BlockEig::kThreads, sizeof(BlockEig), s>>>(m.T, in, out, scratch, rounds,
-                                                                                     status);
+    hermite_psd_kernel<R><<<hermite_psd_grid(m), BlockEig::kThreads, sizeof(BlockEig), s>>>(m.T, in, out, scratch, flags,
+                                                                                     rounds, status);
 }
 } // namespace
 
 size_t hermite_scratch_doubles(const DevMesh& m) { return BlockEig::kScratch * static_cast<size_t>(hermite_psd_grid(m)); }
 
 void launch_hermite_eval(const DevMesh& m, int precision, bool projected, const double* u, double* elemE,
-                         double* per_elem, void* blocks, double* scratch, const EvalArgs& a, cudaStream_t s) {
+                         double* per_elem, void* blocks, double* scratch, int* flags, const EvalArgs& a,
+                         cudaStream_t s) {
     if (m.T > 0) {
         if (a.ev_begin) LPG_CUDA(cudaEventRecord(a.ev_begin, s));
         double* per_grad = a.grad ? per_elem : nullptr;
@@ -3558,21 +3623,21 @@ void launch_hermite_eval(const DevMesh& m, int precision, bool projected, const 
             // FP64 element Hessians, projected into the precision's records.
             double* records = static_cast<double*>(blocks);
             hermite_element_kernel<double><<<kHermParts * m.T, kHermThreads, 0, s>>>(m, u, elemE, per_grad, records,
-                                                                                     a.status);
+                                                                                     flags, a.status);
             if (precision == LPG_PRECISION_F64) {
-                launch_hermite_psd<double>(m, records, records, scratch, a.status, s);
+                launch_hermite_psd<double>(m, records, records, scratch, flags, a.status, s);
             } else {
                 float* out = reinterpret_cast<float*>(records + kHermiteRecord * static_cast<size_t>(m.T));
-                launch_hermite_psd<float>(m, records, out, scratch, a.status, s);
+                launch_hermite_psd<float>(m, records, out, scratch, flags, a.status, s);
                 blocks = out;
             }
         } else if (precision == LPG_PRECISION_F64 || !a.hess) {
             double* records = a.hess ? static_cast<double*>(blocks) : nullptr;
             hermite_element_kernel<double><<<herm_parts(records) * m.T, kHermThreads, 0, s>>>(m, u, elemE, per_grad, records,
-                                                                                              a.status);
+                                                                                              nullptr, a.status);
         } else {
-            hermite_element_kernel<float><<<kHermParts * m.T, kHermThreads, 0, s>>>(m, u, elemE, per_grad,
-                                                                                    static_cast<float*>(blocks), a.status);
+            hermite_element_kernel<float><<<kHermParts * m.T, kHermThreads, 0, s>>>(
+                m, u, elemE, per_grad, static_cast<float*>(blocks), nullptr, a.status);
         }
         if (a.grad) vertex_gather_kernel<64><<<std::min(m.ncl, 148 * 8), 128, 0, s>>>(m, per_elem, 1.0, a.grad);
         if (a.hess) {
@@ -3598,7 +3663,7 @@ size_t hex_blocks_bytes(const DevMesh& m, int precision, bool projected) {
 }
 
 void launch_hex_eval(const DevMesh& m, int precision, bool projected, const double* u, double* elemE,
-                     double* per_elem, void* blocks, const EvalArgs& a, cudaStream_t s) {
+                     double* per_elem, void* blocks, int* flags, const EvalArgs& a, cudaStream_t s) {
     if (m.T > 0) {
         const int grid = (m.T + kHexEl - 1) / kHexEl;
         if (a.ev_begin) LPG_CUDA(cudaEventRecord(a.ev_begin, s));
@@ -3606,20 +3671,20 @@ void launch_hex_eval(const DevMesh& m, int precision, bool projected, const doub
         if (a.hess && projected) {
             // FP64 element Hessians, projected into the precision's records.
             double* records = static_cast<double*>(blocks);
-            hex_element_kernel<double><<<grid, kHexThreads, 0, s>>>(m, u, elemE, per_grad, records, a.status);
+            hex_element_kernel<double, true><<<grid, kHexThreads, 0, s>>>(m, u, elemE, per_grad, records, flags, a.status);
             if (precision == LPG_PRECISION_F64) {
-                launch_hex_psd<double>(m, records, records, a.status, s);
+                launch_hex_psd<double>(m, records, records, flags, a.status, s);
             } else {
                 float* out = reinterpret_cast<float*>(records + kHexRecord * static_cast<size_t>(m.T));
-                launch_hex_psd<float>(m, records, out, a.status, s);
+                launch_hex_psd<float>(m, records, out, flags, a.status, s);
                 blocks = out;
             }
         } else if (precision == LPG_PRECISION_F64) {
-            hex_element_kernel<double><<<grid, kHexThreads, 0, s>>>(m, u, elemE, per_grad,
-                                                           a.hess ? static_cast<double*>(blocks) : nullptr, a.status);
+            hex_element_kernel<double, false><<<grid, kHexThreads, 0, s>>>(
+                m, u, elemE, per_grad, a.hess ? static_cast<double*>(blocks) : nullptr, nullptr, a.status);
         } else {
-            hex_element_kernel<float><<<grid, kHexThreads, 0, s>>>(m, u, elemE, per_grad,
-                                                          a.hess ? static_cast<float*>(blocks) : nullptr, a.status);
+            hex_element_kernel<float, false><<<grid, kHexThreads, 0, s>>>(
+                m, u, elemE, per_grad, a.hess ? static_cast<float*>(blocks) : nullptr, nullptr, a.status);
         }
         if (a.grad) vertex_gather_kernel<8><<<std::min(m.ncl, 148 * 8), 128, 0, s>>>(m, per_elem, 1.0, a.grad);
         if (a.hess) {
@@ -3649,9 +3714,9 @@ void launch_projection(int nodes, int count, const double* in, double* out, doub
     DevMesh m;
     m.T = count;
     if (nodes == 8)
-        launch_hex_psd<double>(m, in, out, status, s, rounds);
+        launch_hex_psd<double>(m, in, out, nullptr, status, s, rounds);
     else
-        launch_hermite_psd<double>(m, in, out, scratch, status, s, rounds);
+        launch_hermite_psd<double>(m, in, out, scratch, nullptr, status, s, rounds);
     LPG_CUDA(cudaGetLastError());
 }
 

@@ -300,23 +300,25 @@ void launch_sum_pairs(const double* per_elem, int T, double* partial, int nblock
 // Hex Q1 element pass (K = 8): energy per element into elemE (T), gradient pieces (24 per element)
 // into per_elem when a.grad is set, the 36 blocks per element (precision's type) into blocks when
 // a.hess is set, then the gradient gather, the energy sum and the block gather. With projected,
-// every element's 24x24 Hessian is first projected to PSD; blocks then holds hex_blocks_bytes().
+// every element's 24x24 Hessian is first projected to PSD (flags: T ints of scratch, which mark the elements that
+// may need it); blocks then holds hex_blocks_bytes().
 void launch_hex_eval(const DevMesh& m, int precision, bool projected, const double* u, double* elemE,
-                     double* per_elem, void* blocks, const EvalArgs& a, cudaStream_t s);
+                     double* per_elem, void* blocks, int* flags, const EvalArgs& a, cudaStream_t s);
 // Python/Torch materials on hex meshes: F at every quadrature point (9 per point, T * nq rows,
 // element-major), and the caller's W (T nq), P (9 T nq) and A (81 T nq, or null without a
-// Hessian) integrated per hex and assembled (blocks as for launch_hex_eval).
+// Hessian) integrated per hex and assembled (blocks and flags as for launch_hex_eval).
 void launch_hex_deformation_gradients(const DevMesh& m, const double* u, double* F, unsigned* status, cudaStream_t s);
 void launch_hex_material_eval(const DevMesh& m, int precision, int hessian, const double* W, const double* P,
-                              const double* A, double* elemE, double* per_elem, void* blocks,
+                              const double* A, double* elemE, double* per_elem, void* blocks, int* flags,
                               const EvalArgs& a, cudaStream_t s);
 // Tricubic Hermite hex element pass (Exact Hessian): energy per element into elemE, gradient
 // pieces (192 per element) into per_elem when a.grad is set, the 2080 blocks per element
 // (precision's type, kHermiteRecord values) into blocks when a.hess is set, then the gathers.
 // With projected, each element's 192 x 192 Hessian is first projected to PSD (scratch:
-// hermite_scratch_doubles()); blocks then holds hermite_blocks_bytes().
+// hermite_scratch_doubles(), flags as for launch_hex_eval); blocks then holds hermite_blocks_bytes().
 void launch_hermite_eval(const DevMesh& m, int precision, bool projected, const double* u, double* elemE,
-                         double* per_elem, void* blocks, double* scratch, const EvalArgs& a, cudaStream_t s);
+                         double* per_elem, void* blocks, double* scratch, int* flags, const EvalArgs& a,
+                         cudaStream_t s);
 size_t hermite_blocks_bytes(const DevMesh& m, int precision, bool projected);
 size_t hermite_scratch_doubles(const DevMesh& m);
 // Bytes of the block records launch_hex_eval needs: FP64 records, plus FP32 ones for a

@@ -217,6 +217,48 @@ LPG_HD bool semidefinite_ldlt(R* V, R tol) {
     return pd;
 }
 
+// Whether the neo-Hookean tangent d2W/dF2 is positive semi-definite, up to the round-off allowance of the test above,
+// 64 eps of its largest diagonal entry, from G = F^-T, a = (lambda log J - mu) / mu and l = lambda / mu. In the frame
+// of the singular values g_i of G (det F > 0) the tangent over mu falls apart into
+// - a 2 x 2 block [[1, -a g_i g_j], [., 1]] for each i < j: semi-definite where I - a^2 K^T K is, K the cofactors of
+//   G (by its LDL^T);
+// - the 3 x 3 block diag(1 - a g_i^2) + l g g^T: definite where a <= 0, else where its three elementary symmetric
+//   polynomials are positive, which the invariants of G^T G give. They cancel near a singular block, so this asks
+//   for a margin.
+// False says nothing: the caller then looks at the Hessian itself.
+LPG_HD bool nh_semidefinite(const double* G, double a, double l) {
+    double gmax = 0, e1 = 0;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int t = 0; t < 9; ++t) {
+        gmax = fmax(gmax, G[t] * G[t]);
+        e1 += G[t] * G[t];
+    }
+    const double tol = 64 * 2.220446049250313e-16 * (1.0 + fabs(l - a) * gmax);
+    if (!(tol < 1e-3)) return false; // F nearly singular
+    const double K0 = G[4] * G[8] - G[5] * G[7], K1 = G[5] * G[6] - G[3] * G[8], K2 = G[3] * G[7] - G[4] * G[6];
+    const double K3 = G[2] * G[7] - G[1] * G[8], K4 = G[0] * G[8] - G[2] * G[6], K5 = G[1] * G[6] - G[0] * G[7];
+    const double K6 = G[1] * G[5] - G[2] * G[4], K7 = G[2] * G[3] - G[0] * G[5], K8 = G[0] * G[4] - G[1] * G[3];
+    const double a2 = a * a, s = (1.0 + tol) * (1.0 + tol);
+    const double c0 = K0 * K0 + K3 * K3 + K6 * K6, c1 = K1 * K1 + K4 * K4 + K7 * K7, c2 = K2 * K2 + K5 * K5 + K8 * K8;
+    const double d0 = s - a2 * c0, s1 = s - a2 * c1, s2 = s - a2 * c2;
+    if (!(d0 > 0 && s1 > 0 && s2 > 0)) return false;
+    // The elimination's rows times d0: no division.
+    const double t01 = a2 * (K0 * K1 + K3 * K4 + K6 * K7), t02 = a2 * (K0 * K2 + K3 * K5 + K6 * K8);
+    const double t12 = a2 * (K1 * K2 + K4 * K5 + K7 * K8);
+    const double d1 = d0 * s1 - t01 * t01, d2 = d0 * s2 - t02 * t02, e12 = d0 * t12 + t01 * t02;
+    if (!(d1 > 0 && d2 * d1 - e12 * e12 > 0)) return false;
+    if (a <= 0) return true;
+    const double det = G[0] * K0 + G[1] * K1 + G[2] * K2, e2 = c0 + c1 + c2, e3 = det * det;
+    const double ae1 = a * e1, ae2 = a2 * e2, ae3 = a2 * a * e3, le1 = l * e1, lae2 = l * a * e2, lae3 = l * a2 * e3;
+    const double margin = 1e-8;
+    return 3.0 - ae1 + le1 > margin * (3.0 + ae1 + le1) &&
+           3.0 - 2 * ae1 + ae2 + 2 * le1 - 2 * lae2 > margin * (3.0 + 2 * ae1 + ae2 + 2 * le1 + 2 * lae2) &&
+           1.0 - ae1 + ae2 - ae3 + le1 - 2 * lae2 + 3 * lae3 >
+               margin * (1.0 + ae1 + ae2 + ae3 + le1 + 2 * lae2 + 3 * lae3);
+}
+
 // A team of one: the host form of the loops above.
 struct SerialTeam {
     LPG_HD int lane() const { return 0; }

@@ -894,7 +894,7 @@ void eval_elastic_async(lpg_fem& h, const lpg_newton_terms* t, const double* x, 
         const bool projected = hk == LPG_HESSIAN_PROJECTED;
         void* blocks = a.hess ? h.d_proj.ensure(hex_blocks_bytes(m, prec, projected)) : nullptr;
         launch_hex_material_eval(m, prec, hk, W, g ? P : nullptr, A, h.d_mat[3].as<double>(nel), h.d_vjp.as<double>(24 * nel),
-                                 blocks, a, s);
+                                 blocks, projected ? h.d_plist.as<int>(nel) : nullptr, a, s);
     } else {
         void* proj = a.hess ? h.d_proj.ensure(project_bytes(m, prec)) : nullptr;
         launch_material_eval(m, prec, hk, W, g ? P : nullptr, A, h.d_mat[3].as<double>(nel), h.d_vjp.as<double>(12 * nel),

@@ -60,7 +60,7 @@ struct lpg_fem {
     lpg::DeviceBuffer b_sell[6]; // sliced-ELL pattern of the solvers
     lpg::DeviceBuffer bt_int[8], bt_dbl[4], bt_skip[2]; // batched Newton (bt_skip: per-cluster skip flags)
     // Scratch of the evaluation entry points.
-    lpg::DeviceBuffer d_plist, d_pcount; // elements listed for the projection's eigenvalue clamp
+    lpg::DeviceBuffer d_plist, d_pcount; // elements listed, or flags of those that may need, the projection's eigenvalue clamp
     lpg::DeviceBuffer d_mat[6];          // material outputs (W, P, A), per-element energies, F and G
     lpg::DeviceBuffer d_result, d_cluster_energy, d_block, d_alpha, d_u, d_u2, d_grad, d_hess, d_proj, d_vjp;
     // Solver state (Newton / PCG / adjoint).
