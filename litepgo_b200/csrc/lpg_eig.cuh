@@ -552,19 +552,20 @@ struct BlockEig {
         return scale;
     }
 
-    // Modified Gram-Schmidt, twice, over the k vectors of X times their factors in y, columns dealt to the
-    // warps and kept in registers; the reflectors stay in A. Returns whether a residual is above round-off.
+    // Modified Gram-Schmidt, twice, over the k vectors of X times their factors in y, a column per half warp and
+    // in registers (three columns a lane: half the shuffles and global sectors of a column per warp); the
+    // reflectors stay in A. Returns whether a residual is above round-off.
     __device__ bool orthonormalise(int k, double nrm, double* X) {
-        static_assert(K % kWarps == 0, "columns per warp");
-        constexpr int J = K / kWarps;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        double z[J][kT];
+        static_assert(K % (2 * kWarps) == 0, "columns per half warp");
+        constexpr int J = K / (2 * kWarps), kH = N / 16;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, l = lane & 15;
+        double z[J][kH];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-            const int c = warp + kWarps * j;
+            const int c = 2 * (warp + kWarps * j) + half;
             const double s = c < k ? y[c] : 0.0;
 #pragma unroll
-            for (int t = 0; t < kT; ++t) z[j][t] = c < k ? s * X[K * (32 * t + lane) + c] : 0.0;
+            for (int t = 0; t < kH; ++t) z[j][t] = c < k ? s * X[K * (16 * t + l) + c] : 0.0;
         }
         int off = 0;
 #pragma unroll 1
@@ -572,35 +573,37 @@ struct BlockEig {
 #pragma unroll 1
             for (int m = 0; m < k; ++m) {
                 double* u = v[m & 1]; // two buffers: one barrier per vector
-                const bool mine = warp == (m & (kWarps - 1));
+                const bool mine = warp == ((m >> 1) & (kWarps - 1));
                 if (mine)
 #pragma unroll
                     for (int j = 0; j < J; ++j)
-                        if (j == m / kWarps) {
+                        if (j == m / (2 * kWarps)) {
                             double q = 0;
 #pragma unroll
-                            for (int t = 0; t < kT; ++t) q = fma(z[j][t], z[j][t], q);
+                            for (int t = 0; t < kH; ++t) q = fma(z[j][t], z[j][t], q);
 #pragma unroll
-                            for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+                            for (int o = 8; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
                             const double r = rsqrt(q);
+                            if (half == (m & 1))
 #pragma unroll
-                            for (int t = 0; t < kT; ++t) {
-                                z[j][t] *= r;
-                                u[32 * t + lane] = z[j][t];
-                            }
+                                for (int t = 0; t < kH; ++t) {
+                                    z[j][t] *= r;
+                                    u[16 * t + l] = z[j][t];
+                                }
                         }
                 __syncthreads();
 #pragma unroll
                 for (int j = 0; j < J; ++j) {
-                    const int c = warp + kWarps * j;
-                    if (c <= m || c >= k) continue; // the same for the whole warp
+                    const int c0 = 2 * (warp + kWarps * j), c = c0 + half;
+                    if (c0 + 1 <= m || c0 >= k) continue; // the same for the whole warp
                     double q = 0;
 #pragma unroll
-                    for (int t = 0; t < kT; ++t) q = fma(u[32 * t + lane], z[j][t], q);
+                    for (int t = 0; t < kH; ++t) q = fma(u[16 * t + l], z[j][t], q);
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+                    for (int o = 8; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+                    if (c > m)
 #pragma unroll
-                    for (int t = 0; t < kT; ++t) z[j][t] = fma(-q, u[32 * t + lane], z[j][t]);
+                        for (int t = 0; t < kH; ++t) z[j][t] = fma(-q, u[16 * t + l], z[j][t]);
                 }
                 if (pass > 0 && mine) {
 #pragma unroll
@@ -615,10 +618,10 @@ struct BlockEig {
             }
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-            const int c = warp + kWarps * j;
+            const int c = 2 * (warp + kWarps * j) + half;
 #pragma unroll
-            for (int t = 0; t < kT; ++t)
-                if (c < k) X[K * (32 * t + lane) + c] = z[j][t];
+            for (int t = 0; t < kH; ++t)
+                if (c < k) X[K * (16 * t + l) + c] = z[j][t];
         }
         return __syncthreads_or(off) != 0; // X is written
     }
