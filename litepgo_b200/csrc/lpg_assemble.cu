@@ -1697,7 +1697,6 @@ __global__ void __launch_bounds__(kTcThreads, MINB) tet_cluster_kernel(const Dev
 // pass and a cluster takes two block barriers instead of four. Item pass: one lane per row, component
 // and part of the row's contributors, the parts split and added as in tet_cluster_kernel (the gradient is
 // bitwise that of the Hessian pass).
-constexpr int kTgEnts = 4 * kTcElems; // at most four contributors of diagonal items per element
 template <typename R> constexpr int tg_minb() { return sizeof(R) == 8 ? 3 : 4; }
 template <typename R> constexpr size_t tg_smem_bytes() {
     return (32 + 3 * kTcVerts) * sizeof(double) + 12 * static_cast<size_t>(kTcStride) * sizeof(R) +

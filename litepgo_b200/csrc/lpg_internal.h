@@ -137,6 +137,8 @@ constexpr int kTcVals = LPG_TC_VALS; // output staging values of a cluster (its 
 constexpr int kTcItems = kTcVals / 9;
 constexpr int kTcEnts = LPG_TC_ENTS;
 static_assert(kTcEnts % 8 == 0, "contributor lists are staged in 16-byte chunks");
+// Contributor words that the gradient pass stages: its diagonal items', at most four per element.
+constexpr int kTgEnts = 4 * kTcElems;
 static_assert(kTcElems <= 256 && kTcRows <= 256, "tet cluster indices are 8-bit");
 // Clusters of 64-node cells (Hermite hexes: 8 slot rows per vertex, ~216 blocks per row) hold at
 // most one vertex's rows, so a cluster's slot and contributor tables fit in shared memory.

@@ -686,6 +686,7 @@ void check_tet_clusters(const HostPlan& p, const int32_t* tets) {
     const int V = p.V, T = p.T;
     auto vert = [&](int e, int a) { return tets[4 * static_cast<size_t>(e) + a]; };
     const int ncl = static_cast<int>(p.tc_row_ptr.size()) - 1;
+    if (static_cast<int>(p.tc_dent.size()) != ncl) bad("contributors of diagonal items per cluster");
     std::vector<int> owner(static_cast<size_t>(V), -1), energy_count(static_cast<size_t>(T), 0);
     for (int c = 0; c < ncl; ++c)
         for (int k = p.tc_row_ptr[c]; k < p.tc_row_ptr[c + 1]; ++k) {
@@ -741,6 +742,15 @@ void check_tet_clusters(const HostPlan& p, const int32_t* tets) {
         const int i0 = p.tc_item_ptr[c], ni = p.tc_item_ptr[c + 1] - i0;
         const int nd = p.tc_ndiag[c];
         if (nd != nr) bad("one diagonal item per row");
+        size_t dent = 0; // the diagonal items' lists come first, one after the other
+        for (int it = 0; it < nd; ++it) {
+            const uint32_t lists = p.tc_items[4 * static_cast<size_t>(i0 + it) + 2];
+            if ((lists & 0xfffffu) != dent) bad("diagonal contributor lists not in order");
+            dent += lists >> 20;
+        }
+        if (p.tc_dent[c] != static_cast<int>((dent + 7) & ~size_t(7)) || p.tc_dent[c] > kTgEnts ||
+            p.tc_dent[c] > p.tc_ent_ptr[c + 1] - p.tc_ent_ptr[c])
+            bad("staged contributors of diagonal items");
         size_t prev = ~size_t(0);
         for (int it = 0; it < ni; ++it) {
             const uint32_t* w = p.tc_items.data() + 4 * static_cast<size_t>(i0 + it);
