@@ -186,6 +186,13 @@ template <typename R> constexpr size_t pcg_p_bytes(int rows, int halo, bool stag
     return (static_cast<size_t>(rows + halo) * pcg_stride<R>() * sizeof(R) + halo * sizeof(int32_t) + 15) / 16 * 16 +
            pcg_stage_bytes<R>(staged ? halo : 0);
 }
+// Slots of a warp in registers: KR of the kernel, which has two builds. Large systems, whose blocks read values from
+// L2, gain more from one more slot on the chip (and in FP32 from three words of the halo in flight) than its
+// spills cost; the others run better without. Newton, small build then large: 8^3 cubes mixed 11.4 and 12.4 ms,
+// 24^3 FP64 45.6 and 43.6, 36^3 FP64 150 and 134.
+template <typename R> constexpr int pcg_register_slots(bool large) { return (sizeof(R) == 4 ? 2 : 1) + (large ? 1 : 0); }
+// Warps that share a chunk in a block of nc chunks.
+__host__ __device__ constexpr int pcg_sub(int nc) { return 4 * nc <= kPcgWarps ? 4 : 2 * nc <= kPcgWarps ? 2 : 1; }
 // Shared memory of one slot of a chunk (32 blocks).
 template <typename R> constexpr size_t pcg_slot_bytes() { return 32 * 9 * sizeof(R); }
 constexpr size_t kPcgFixed = (2 * kPcgWarps + 22) * sizeof(double); // sums and scalars
@@ -251,10 +258,10 @@ __device__ __forceinline__ double shfl_xor_add(double keep, double send, int o) 
     return keep + __shfl_xor_sync(0xffffffffu, send, o);
 }
 
-template <typename R>
+template <typename R, int KR>
 __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh m, const PcgPlan plan, const PcgArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int PS = pcg_stride<R>(), KR = sizeof(R) == 4 ? 3 : 1, G = sizeof(R) == 4 ? 3 : 1;
+    constexpr int PS = pcg_stride<R>(), G = KR == 3 ? 3 : 1;
     constexpr int MS = 16; // most slots of a warp in shared memory (their column indices are in registers)
     double* red = reinterpret_cast<double*>(smem_raw); // [2 values][warps]
     double* total = red + 2 * kPcgWarps; // [warp]: the sums of 32 blocks
@@ -283,8 +290,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_solve_kernel(const DevMesh
     const size_t vectors = kPcgFixed + pcg_p_bytes<R>(own_rows, L, staged);
     unsigned char* rest = smem_raw + vectors;
     // `sub` warps share a chunk (its slots dealt round robin); the first of them owns the rows.
-    int sub = 1;
-    while (2 * sub * nc <= kPcgWarps && sub < 4) sub *= 2;
+    const int sub = pcg_sub(nc);
     const int ch = warp / sub, part = warp - sub * ch;
     const bool on = ch < nc;
     const int c = c0 + (on ? ch : 0);

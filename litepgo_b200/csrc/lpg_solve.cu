@@ -615,13 +615,27 @@ void clear_words(lpg_fem& h, PcgPlanStore& P) {
     LPG_CUDA(cudaMemsetAsync(P.z.ptr, 0, 4 * sizeof(double) * static_cast<size_t>(h.dm.V), h.stream));
 }
 
-// Plan of the one-launch PCG of `groups` (chunk and vertex ranges). It is not used (state -1, or 1 for FP64)
+// Chunks per block of a group of `chunks`, at least. An exchange waits for every block of the group, so that
+// many blocks of few chunks lose to fewer blocks whose 16 warps are all at work (four warps a chunk up to 4, two up
+// to 8); FP64 keeps to what its values leave room for in shared memory. us per PCG iteration of a Newton solve, all
+// its other work included, as few chunks a block as there are SMs for, then this: 14^3 cubes FP64 7.6 and 6.3, mixed
+// 7.9 and 6.2; 16^3 10.3 and 7.5, 9.3 and 6.7; 20^3 7.7 and 7.1, 8.7 and 6.7; 24^3 8.6 and 8.9, 7.5 and 7.5; 28^3
+// 9.9 and 10.1, 8.0 and 8.3. They vary by a tenth with the SMs that a launch gets.
+template <typename R> int pcg_chunks(int chunks) {
+    if (chunks <= (sizeof(R) == 8 ? 32 : 16)) return 1;
+    if (chunks <= 56) return 2;
+    if (chunks <= 296 || sizeof(R) == 8) return 4;
+    return chunks <= 1184 ? 8 : 16;
+}
+
+// Plan of the one-launch PCG in precision R of `groups` (chunk and vertex ranges). It is not used (state -1)
 // where a group's chunks exceed one per warp of one block per SM (a row's state then no longer fits a lane),
 // where a block's z exceeds its shared memory, or where it would take more than `most_launches`. Below that
 // line it is the faster one at every size measured: whole Newton solves, launches per step then one launch,
-// 4^3 cubes FP64 32 and 15 ms, 30^3 FP64 200 and 105, 36^3 FP64 (50,653 vertices, most values read from L2
-// each iteration) 261 and 171, 40x40x36 mixed 167 and 93.
-void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, int most_launches) {
+// 4^3 cubes FP64 32 and 8.5 ms, 36^3 FP64 (50,653 vertices, most values read from L2 each iteration) 261 and 131,
+// 40x40x36 mixed 167 and 76.
+template <typename R>
+void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, int most_launches, bool few_blocks = true) {
     const DevMesh& m = h.dm;
     cudaStream_t s = h.stream;
     P.state = -1;
@@ -631,24 +645,32 @@ void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, i
     LPG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h.device));
     sms = std::min(sms, kPcgMaxBlocks);
     if (!coop || m.n_sell <= 0) return;
-    // The fewest chunks per block with which all groups run at once, else full blocks and several launches.
-    // A group whose values fit one block's shared memory in FP64 takes one: it then exchanges nothing. Newton
-    // of 3^3 and 4^3 cubes, a block per chunk then one block: 9.0 and 8.1 ms, 9.6 and 8.8.
+    // The fewest chunks per block, from pcg_chunks() on, with which all groups run at once, else full blocks and
+    // several launches. A group whose values fit one block's registers and shared memory takes one: it then
+    // exchanges nothing. Newton of 3^3 and 4^3 cubes, a block per chunk then one block: 9.0 and 8.1 ms, 9.6 and 8.8;
+    // of 6^3 in FP32, which fits too: 8.7 and 8.3.
+    const HostPlan& p = h.plan;
+    const auto slots_of = [&](int c) { return (p.sell_ptr[c + 1] - p.sell_ptr[c] + p.sell_bptr[c + 1] - p.sell_bptr[c]) / 32; };
     const auto resident = [&](const PcgGroup& g) {
-        if (g.c1 - g.c0 > kPcgWarps) return false;
-        const HostPlan& p = h.plan;
-        const size_t slots = (p.sell_ptr[g.c1] - p.sell_ptr[g.c0] + p.sell_bptr[g.c1] - p.sell_bptr[g.c0]) / 32;
-        return kPcgFixed + pcg_p_bytes<double>(32 * (g.c1 - g.c0), 0, true) + slots * pcg_slot_bytes<double>() <=
-               static_cast<size_t>(optin);
+        const int nc = g.c1 - g.c0;
+        if (nc > kPcgWarps) return false;
+        size_t slots = 0;
+        for (int c = g.c0; c < g.c1; ++c) slots += std::max(slots_of(c) - pcg_register_slots<R>(false) * pcg_sub(nc), 0);
+        return kPcgFixed + pcg_p_bytes<R>(32 * nc, 0, true) + slots * pcg_slot_bytes<R>() <= static_cast<size_t>(optin);
     };
     const auto blocks_of = [&](const PcgGroup& g, int per) { return resident(g) ? 1 : (g.c1 - g.c0 + per - 1) / per; };
-    int per = 0;
+    int per = 0, preferred = 1;
+    if (few_blocks)
+        for (const PcgGroup& g : groups) preferred = std::max(preferred, pcg_chunks<R>(g.c1 - g.c0));
+    per = preferred - 1;
     int64_t all = 0;
     do {
         ++per;
         all = 0;
         for (const PcgGroup& g : groups) all += blocks_of(g, per);
     } while (all > sms && per < kPcgWarps);
+    P.large = false; // the line between the builds: 296 chunks, 9,472 vertices
+    for (const PcgGroup& g : groups) P.large = P.large || g.c1 - g.c0 > 296 || (per > 8 && !resident(g));
     P.first.assign(1, 0);
     P.blocks = 0;
     int words = 0;
@@ -682,7 +704,10 @@ void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, i
     int rows = 0; // of the largest block
     for (const PcgGroup& g : groups)
         for (int b = 0; b < g.blocks; ++b) rows = std::max(rows, 32 * (pcg_first_chunk(g, b + 1) - pcg_first_chunk(g, b)));
-    if (rows + P.stride >= 65536 || !fits(pcg_p_bytes<float>(rows, P.stride, false))) return;
+    if (rows + P.stride >= 65536 || !fits(pcg_p_bytes<R>(rows, P.stride, false))) {
+        if (preferred > 1) build_pcg_plan<R>(h, P, groups, most_launches, false); // smaller blocks have smaller halos
+        return;
+    }
     pcg_plan_kernel<<<P.blocks, kPcgThreads, bits, s>>>(
         m, dg, dof, pos, P.halo.as<int32_t>(static_cast<size_t>(P.blocks) * P.stride), P.stride, count,
         P.own.as<uint16_t>(std::max<size_t>(h.plan.sell_col.size(), 1)),
@@ -693,7 +718,7 @@ void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, i
     P.words.ensure(3 * sizeof(uint4) * P.blocks + sizeof(unsigned) * P.groups);
     P.z.ensure(4 * sizeof(double) * static_cast<size_t>(m.V));
     clear_words(h, P);
-    P.state = fits(pcg_p_bytes<double>(rows, P.stride, false)) ? 2 : 1;
+    P.state = 1;
 }
 
 // The solve of every group of plan P, one cooperative launch for as many as run at once: x4 from b4, the
@@ -701,7 +726,8 @@ void build_pcg_plan(lpg_fem& h, PcgPlanStore& P, std::vector<PcgGroup> groups, i
 template <typename R> void launch_pcg(lpg_fem& h, PcgPlanStore& P, PcgArgs<R> a) {
     int optin = 0;
     LPG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h.device));
-    LPG_CUDA(cudaFuncSetAttribute(pcg_solve_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    auto* kernel = P.large ? pcg_solve_kernel<R, pcg_register_slots<R>(true)> : pcg_solve_kernel<R, pcg_register_slots<R>(false)>;
+    LPG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     a.z4 = static_cast<R*>(P.z.ptr);
     a.words = static_cast<uint4*>(P.words.ptr);
     a.number = reinterpret_cast<unsigned*>(a.words + 3 * static_cast<size_t>(P.blocks));
@@ -721,7 +747,7 @@ template <typename R> void launch_pcg(lpg_fem& h, PcgPlanStore& P, PcgArgs<R> a)
     void* args[] = {&dm, &plan, &a};
     for (size_t k = 0; k + 1 < P.first.size(); ++k) {
         a.first_block = P.first[k];
-        LPG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(pcg_solve_kernel<R>),
+        LPG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel),
                                              dim3(P.first[k + 1] - P.first[k]), dim3(kPcgThreads), args, a.smem, h.stream));
     }
 }
@@ -1041,8 +1067,9 @@ struct Solver {
     }
 
     template <typename R> bool one_launch() {
-        if (h.pcg_plan.state == 0) build_pcg_plan(h, h.pcg_plan, {PcgGroup{0, h.dm.n_sell, 0, V, 0, 0}}, 1);
-        return h.pcg_plan.state >= (sizeof(R) == 8 ? 2 : 1);
+        PcgPlanStore& P = h.pcg_plan[sizeof(R) == 8];
+        if (P.state == 0) build_pcg_plan<R>(h, P, {PcgGroup{0, h.dm.n_sell, 0, V, 0, 0}}, 1);
+        return P.state > 0;
     }
 
     // Solves mask K x = mask b (FP64 b of norm bnorm, x): inner PCG in precision R on Kin (values of type R),
@@ -1123,12 +1150,12 @@ struct Solver {
                 a.tol = inner_tol;
                 a.max_iters = max_iters - static_cast<int>(out.iters);
                 a.first_direction = true;
-                launch_pcg<R>(h, h.pcg_plan, a);
+                launch_pcg<R>(h, h.pcg_plan[sizeof(R) == 8], a);
                 copy_state();
                 update();
                 read_state();
                 if (hs.lost) {
-                    clear_words(h, h.pcg_plan); // the blocks' numbers may differ now
+                    clear_words(h, h.pcg_plan[sizeof(R) == 8]); // the blocks' numbers may differ now
                     fail(LPG_ECUDA, "PCG: the solve's blocks lost one another");
                 }
             } else {
@@ -2098,7 +2125,7 @@ struct BatchSolver {
         bool same = h.batch_graph != nullptr;
         for (int i = 0; i < 12 && same; ++i) same = h.batch_graph_key[i] == key[i];
         cudaStream_t gs = h.own_stream;
-        const bool one = h.batch_plan.state >= (sizeof(R) == 8 ? 2 : 1);
+        const bool one = h.batch_plan.state > 0;
         if (!one && !same) {
             if (h.batch_graph) {
                 cudaGraphExecDestroy(h.batch_graph);
@@ -2279,8 +2306,12 @@ void batch_newton_solve(lpg_fem& h, int M, const int32_t* voff_h, const int32_t*
         g.c1 = i / 32 + 1;
     }
     // Each further launch adds its slowest mesh's iterations, where the launches per step all advance
-    // together: 1500 boxes of 3 to 4 cubes a side (11 launches) 126 ms per step, 109 so; 3000 (21) 196 and 194.
-    build_pcg_plan(h, h.batch_plan, groups, 20);
+    // together: 1500 boxes of 3 to 4 cubes a side (11 launches) 126 ms per step, 109 so; 3000 (21) 196 and 194;
+    // 256 boxes of 4 to 24, with a long tail of a few buckling ones, mixed 3.12 s and 1.74.
+    if (o.precision == LPG_PRECISION_F64)
+        build_pcg_plan<double>(h, h.batch_plan, groups, 20);
+    else
+        build_pcg_plan<float>(h, h.batch_plan, groups, 20);
     BatchSolver B(h, d);
     B.up(d.voff, std::vector<int>(voff_h, voff_h + M + 1));
     B.up(d.eoff, std::vector<int>(eoff_h, eoff_h + M + 1));

@@ -34,8 +34,9 @@ struct ScopedEvent {
 };
 
 struct PcgPlanStore {
-    int state = 0; // 0 not built, 1 usable in FP32 only, 2 in both precisions, -1 not usable
+    int state = 0; // 0 not built, 1 usable, -1 not usable
     int groups = 0, blocks = 0, stride = 0;
+    bool large = false; // the build of the kernel (pcg_register_slots)
     std::vector<int> first; // first block of each launch, then the number of blocks
     DeviceBuffer group, of_block, pos, halo, count, own, bor, words, z;
 };
@@ -72,9 +73,9 @@ struct lpg_fem {
     // CUDA graph of a chunk of PCG iterations, reused while its pointers stay the same.
     cudaGraphExec_t pcg_graph = nullptr;
     const void* pcg_graph_key[12] = {};
-    // Plans of the one-launch PCG (lpg_pcg.cuh): of the whole mesh, built at the first solve, and of the
-    // meshes of a batched solve, built by each call.
-    lpg::PcgPlanStore pcg_plan, batch_plan;
+    // Plans of the one-launch PCG (lpg_pcg.cuh): of the whole mesh in FP32 and FP64, built at the first solve, and
+    // of the meshes of a batched solve, built by each call.
+    lpg::PcgPlanStore pcg_plan[2], batch_plan;
     unsigned pcg_polls = 1u << 22; // polls of one word before a block of it gives up (seconds)
     cudaGraphExec_t batch_graph = nullptr; // the batched (per-mesh) PCG iterations
     const void* batch_graph_key[12] = {};
