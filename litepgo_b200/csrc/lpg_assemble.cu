@@ -1001,7 +1001,7 @@ __global__ void __launch_bounds__(kProjThreads) project_kernel(const DevMesh m, 
 // One warp a block: a thread's scratch rows, not its registers, then bound the resident warps in FP64 (11).
 constexpr int kClampThreads = 32;
 // Register-budget variants of the clamp (autotuner), as resident blocks per SM: FP32 at 16 (128 registers) or
-// 12 (168, no spill); FP64 has one, at what its shared memory allows.
+// 12 (168, 48 bytes spilled); FP64 has one, at what its shared memory allows.
 template <typename R> constexpr int clamp_minb(int v) {
     return sizeof(R) == 8 ? 11 : (v == 0 ? 16 : 12);
 }

@@ -40,8 +40,8 @@ __device__ __forceinline__ double eig_start(int i, int c) {
 
 // Eigenvalues of the n x n tridiagonal matrix (d, off-diagonals squared e2) below x, by the signs of the
 // leading principal minors p_i = (d_i - x) p_{i-1} - e2_{i-1} p_{i-2}: no division in the chain, one
-// dependent FMA per row. |d|, |e| <= 1 (the matrix is scaled), and both terms of the pair are rescaled by
-// a power of two every 8 rows.
+// dependent FMA per row. The matrix's entries are below 1, so |d| and |e| below N, and both terms of the
+// pair are rescaled by a power of two every 8 rows.
 template <int N> __device__ __forceinline__ int sturm_count(const double* d, const double* e2, double x) {
     double p2 = 1.0, p1 = d[0] - x;
     if (p1 == 0.0) p1 = -1e-30;

@@ -19,19 +19,20 @@
 // the products and FP64 latency.
 //
 // The recurrences are those of the launches per step. The form with one reduction (Chronopoulos and Gear,
-// 1989), which takes p.Ap from z.Az and the sums before and A p from a recurrence, is no faster here, since p
-// of the halo costs no exchange, and not stable enough in FP32: on blocks with a Poisson ratio of 0.4999 it
-// took 60 % more iterations, from 0.499975 on it lost the sign of p.Ap, and so it did on columns of 60 cubes.
+// 1989), which takes p.Ap from z.Az and the sums before and A p from a recurrence, saves the second exchange of
+// sums (nothing to speak of where a system is on few blocks: pcg_chunks) and is not stable enough in FP32: on
+// blocks with a Poisson ratio of 0.4999 it took 60 % more iterations, from 0.499975 on it lost the sign of p.Ap,
+// and so it did on columns of 60 cubes.
 //
 // A batch of meshes is one launch too: every mesh has blocks of its own (one block exchanges nothing), its
 // own sums, tolerance and end, where the launches per step run all meshes in lockstep to the slowest.
 //
 // Measured per iteration, B200 (launch-per-step, then this kernel): 648 vertices FP64 14.2 and 4.0 us; 4,896
 // FP64 16.4 and 5.4; 62,197 FP32 15.6 and 7.5, where the products (18 slots a lane) and the wait for the
-// slowest block are half; 48 boxes of 4 to 16 cubes, 64,000 vertices, 24 in lockstep and 9.4 side by side. Three
-// slots of a lane are in registers in FP32 (KR), which spills 56 bytes: with two the slowest block waits for
-// one more slot from L2 (a Newton solve of 62,197 vertices 90 ms instead of 82), with four the spills cost more
-// (86). Beside 227 KB of shared memory there is hardly any L1 to hold them, hence G and one word per lane.
+// slowest block are half; 48 boxes of 4 to 16 cubes, 64,000 vertices, 24 in lockstep and 9.4 side by side. Large
+// systems keep three slots of a lane in registers in FP32 (KR), which spills 56 bytes: with two the slowest block
+// waits for one more slot from L2 (a Newton solve of 62,197 vertices 90 ms instead of 82), with four the spills cost
+// more (86). Beside 227 KB of shared memory there is hardly any L1 to hold them, hence G and one word per lane.
 #pragma once
 
 namespace lpg {
