@@ -39,7 +39,7 @@ namespace lpg {
 namespace {
 
 constexpr int kPcgThreads = 512, kPcgWarps = kPcgThreads / 32;
-constexpr int kPcgMaxBlocks = 160;     // five slots per polling lane
+constexpr int kPcgMaxBlocks = 160; // two sums of five groups of 32 blocks: a polling warp each
 
 // One linear system of a launch: a mesh's chunks and vertices (a chunk at a mesh's ends may hold rows of its
 // neighbours, which are passed over) and the blocks that work on it. Groups know nothing of one another.
